@@ -5,6 +5,7 @@
 #include <string>
 #include <vector>
 
+#include "f64_dmma.cuh"
 #include "reduce.cuh"
 #include "sp2b_tune.h"
 
@@ -309,12 +310,6 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
-__device__ __forceinline__ void dmma884(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
-}
-
 template <int BT, int WM, int WN>
 struct F64Cfg {
   static constexpr int BK = 16;
@@ -340,9 +335,6 @@ __global__ void __launch_bounds__(WM* WN * 32, 1) k_sym_gemm_f64(const StepArgs 
     if (br < 0) return;
     if (br == BR_X2) { alpha = 1.0; beta = 0.0; }
     else { alpha = -1.0; beta = 2.0; }
-    // response products after step k: P1 = a X Delta + b Delta (control 2, the step's
-    // own a, b), then Delta' = a Delta X + P1 (control 3)
-    if (p.control == 3) beta = 1.0;
   }
   int bi, bj, nloc = p.np, core = p.core;
   size_t row0 = 0;
@@ -597,8 +589,8 @@ cudaError_t launch_f64_multistep(const MultiStepArgs& a, cudaStream_t st) {
   return e;
 }
 
-// Tile edge of the dense FP64 step for np: the measured choice when one was made for this
-// device and size (tune_f64_tile), else 128 once its tiles fill the SMs twice, else 64.
+// Tile edge of a single dense FP64 product of padded size np: the solve's measured choice
+// for this device and size (tune_f64_solve) when one was made, else 128 once its tiles fill the SMs twice, else 64.
 int f64_tile(int np) {
   int c = 0;
   if (tune_lookup(f64_tune_key(np), &c) && (c == 64 || c == 128)) return c;
@@ -646,45 +638,6 @@ cudaError_t launch_sym_gemm_f64(const StepArgs& a0, cudaStream_t st) {
   const int t = a.np / bt;
   a.ntiles = t * (t + 1) / 2;   // the partial sums the last CTA reduces: one per launched tile
   return launch_f64_bt(a, bt, a.ntiles, st);
-}
-
-// Measures the dense step's tile edges 128 and 64 at np (one plain product each on
-// x_in -> x_out, the same k order per element in both) and records the faster one for
-// f64_tile.  partials must hold 4 doubles per 64-edge tile.
-int tune_f64_tile(int np, const double* x_in, double* x_out, double* partials, unsigned* counter,
-                  double* sums_out, cudaStream_t st) {
-  int c = 0;
-  const std::string key = f64_tune_key(np);
-  if (!tune_enabled() || tune_lookup(key, &c)) return 0;
-  const int edges[2] = {128, 64};
-  StepArgs q;
-  memset(&q, 0, sizeof(q));
-  q.np = np;
-  q.ld = np;
-  q.A = q.B = q.E = x_in;
-  q.out = x_out;
-  q.alpha = 1.0;
-  q.beta = 0.0;
-  q.partials = partials;
-  q.counter = counter;
-  q.sums_out = sums_out;
-  // timed on zeros (the buffer may not hold data yet; DMMA time does not depend on values)
-  if (cudaMemsetAsync(const_cast<double*>(x_in), 0, (size_t)np * np * sizeof(double), st) !=
-      cudaSuccess)
-    return 3;   // SP2B_CUDA_ERROR
-  std::vector<float> ms;
-  int best = 0;
-  const int rc = tune_measure(2, 2, st, [&](int cand) -> int {
-    const int t = np / edges[cand];
-    q.ntiles = t * (t + 1) / 2;
-    if (cudaMemsetAsync(counter, 0, 4 * sizeof(unsigned), st) != cudaSuccess ||
-        launch_f64_bt(q, edges[cand], q.ntiles, st) != cudaSuccess)
-      return 3;   // SP2B_CUDA_ERROR
-    return 0;
-  }, &ms, &best);
-  if (rc != 0) return rc;
-  tune_store(key, edges[best], ms);
-  return 0;
 }
 
 cudaError_t launch_sym_gemm_f64_batched(const StepArgs& a, int bt, cudaStream_t st) {

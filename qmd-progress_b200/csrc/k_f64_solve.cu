@@ -1,0 +1,552 @@
+// The dense FP64 SP2 recursion as one persistent cooperative launch: every step's
+// symmetric product, the branch update, the sums and the branch decision, and for the
+// forward-mode response the anticommutator {X, Delta} beside X^2.
+#include <algorithm>
+#include <cstring>
+#include <string>
+#include <vector>
+
+#include "f64_tile.cuh"
+#include "reduce.cuh"
+#include "sp2b_tune.h"
+
+namespace sp2b {
+
+namespace {
+
+// The work of one step in units of one 16-row k-block of one tile, tile after tile: first
+// the ntiles products X^2 (kb units each), then, with a response, the ntiles
+// anticommutator tiles X Delta + Delta X (2 kb units each, K concatenated).  CTA c takes
+// the units [bound(c), bound(c + 1)): equal shares, so no partial last wave of tiles leaves
+// SMs idle.  A tile cut by a bound is summed by the CTA that holds its last units; the
+// others leave their accumulators in a workspace slot.  A bound closer than `snap` units to
+// a tile edge moves to that edge.
+struct F64Split {
+  int kb, ntiles, snap, G;
+  long long total;
+
+  __device__ __forceinline__ int len(int job) const { return job < ntiles ? kb : 2 * kb; }
+  __device__ __forceinline__ void locate(long long u, int& job, int& off) const {
+    const long long first = (long long)ntiles * kb;
+    if (u < first) {
+      job = (int)(u / kb);
+      off = (int)(u - (long long)job * kb);
+    } else {
+      const long long v = u - first;
+      const int q = (int)(v / (2 * kb));
+      job = ntiles + q;
+      off = (int)(v - (long long)q * 2 * kb);
+    }
+  }
+  __device__ __forceinline__ long long bound(int c) const {
+    const long long u = total * c / G;
+    int job, off;
+    locate(u, job, off);
+    if (off == 0) return u;
+    if (off < snap) return u - off;
+    const int rest = len(job) - off;
+    return rest < snap ? u + rest : u;
+  }
+};
+
+// Waits (bounded) until *word >= target; false when the wait ran out or another CTA gave up.
+__device__ __forceinline__ bool spin_until(const unsigned* word, unsigned target, const int* err) {
+  for (uint32_t it = 0; it < kSpinLimit; ++it) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
+    if (v >= target) return true;
+    if ((it & 63) == 63 && *(volatile const int*)err) return false;
+  }
+  return false;
+}
+
+constexpr int kMaxPieces = 64;   // pieces of one tile other CTAs hold (see f64_plan)
+constexpr int kSums = 5;   // ||X'||^2, Tr X', ||X - X^2||^2 (core rows), Tr X^2, Tr Delta'
+
+// Barrier of the consumer warps.
+template <int NT>
+__device__ __forceinline__ void consumer_sync() {
+  asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
+}
+
+struct F64SolveMaps {
+  CUtensorMap x[2], d[2];
+};
+
+}  // namespace
+
+// Bound by the DMMA pipe (37 TFLOP/s measured with registers only).  The per-step launches
+// this replaces spent ~10 us of each step on launch, record reads, mirrored stores and the
+// last CTA's sums, computed whole padded 128-blocks, left SMs idle in the last wave of
+// tiles and, for the response, formed {X, Delta} as two products with a stored middle.  Here
+// a step costs its k-blocks (92 % of the DMMA rate at n = 3500), ~4 us per tile epilogue and
+// ~3 us of barrier and decision.  Per solve on B200, before -> now: n = 100 365 -> 169 us,
+// n = 1000 985 -> 640 us, n = 2000 (14 steps) 4.0 ms, n = 3500 23.0 -> 19.3 ms, response
+// n = 777 2.40 -> 0.91 ms.
+//
+// One CTA walks its share of each step's units (F64Split), then all CTAs meet at a grid
+// barrier (a counter, bounded wait) and every CTA sums the partials in CTA order and takes
+// the same branch decision, so no launch, no host poll and no last-CTA pass lies between
+// steps.  A CTA's segments run: the open head of its last tile first (its workspace slot is
+// then long full when the owner asks for it), its whole tiles, and last the tile whose head
+// other CTAs hold.  The last warp loads (its pipeline runs across segments), the others multiply.
+template <int BT>
+__global__ void __launch_bounds__(F64Tile<BT>::NT + 32, 1)
+    k_f64_solve(const __grid_constant__ F64SolveMaps maps, const __grid_constant__ F64SolveArgs p) {
+  using C = F64Tile<BT>;
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t bar_full[C::ST], bar_empty[C::ST];
+  __shared__ double s_red[kSums][C::NW + 1], s_tot[kSums];
+  __shared__ SP2Decision s_dec;
+  __shared__ double s_fro2;          // ||X_k||_F^2
+  __shared__ int s_run;              // 0: the loop has ended
+  __shared__ int s_piece[kMaxPieces], s_npiece;
+  __shared__ volatile int s_abort;
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const int G = (int)gridDim.x, cta = (int)blockIdx.x;
+  const bool resp = p.d[0] != nullptr;
+  F64Split sp;
+  sp.kb = p.kb;
+  sp.ntiles = p.ntiles;
+  sp.snap = p.snap;
+  sp.G = G;
+  sp.total = (long long)p.ntiles * p.kb * (resp ? 3 : 1);
+  const long long u0 = sp.bound(cta), u1 = sp.bound(cta + 1);
+  int ja, oa, jb, ob;
+  sp.locate(u0, ja, oa);
+  sp.locate(u1, jb, ob);
+  const bool open = u1 > u0 && ob > 0;                     // the range ends inside tile jb
+  const int nseg = u1 > u0 ? (open ? 1 : 0) + (jb - ja) : 0;
+  // segment i: job and its unit range
+  auto segment = [&](int i, int& job, int& k0, int& k1) {
+    if (open && i == 0) {
+      job = jb;
+      k0 = ja == jb ? oa : 0;
+      k1 = ob;
+      return;
+    }
+    const int q = i - (open ? 1 : 0);   // 0 .. jb - ja - 1: ja + 1, ..., jb - 1, then ja
+    job = q + 1 < jb - ja ? ja + 1 + q : ja;
+    k0 = job == ja ? oa : 0;
+    k1 = sp.len(job);
+  };
+  const int ld = p.ld;
+
+  if (tid == 0) {
+    s_abort = 0;
+    for (int s = 0; s < C::ST; ++s) {
+      mbar_init(smem_u32(&bar_full[s]), 1);
+      mbar_init(smem_u32(&bar_empty[s]), C::NW);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    // the CTAs that hold the head of this CTA's first tile, nearest first
+    s_npiece = 0;
+    if (nseg > (open ? 1 : 0) && oa > 0)
+      for (int c = cta - 1; c >= 0 && s_npiece < kMaxPieces; --c) {
+        const long long hi = sp.bound(c + 1);
+        if (hi <= u0 - oa) break;
+        if (sp.bound(c) < hi) s_piece[s_npiece++] = c;
+      }
+    const SP2Rec r = p.rec[p.k0];
+    s_run = 1;
+    if (p.k0 > 0 && *(volatile const int*)&p.sout->done) {
+      s_run = 0;   // an earlier launch of this solve ended the loop
+    } else if (r.done) {
+      // reached at k = 0 when normalisation flagged the input
+      s_run = 0;
+      if (cta == 0) {
+        p.rec[p.k0 + 1] = r;
+        p.sout->nupd = p.k0;
+        p.sout->iter = r.iter;
+        p.sout->status = r.status;
+        p.sout->done = 1;
+      }
+    } else {
+      s_dec = sp2_decide(p.ctl, r, p.k0, p.pp_in);
+      s_fro2 = r.fro2;
+    }
+  }
+  __syncthreads();
+  typename C::Frag frag;
+  frag.init(lane);
+  uint32_t g = 0;   // units loaded (loader) or consumed so far, over all steps
+  for (int k = p.k0; k < p.k1; ++k) {
+    if (!s_run) return;
+    if (s_dec.branch == BR_STOP) {
+      if (cta == 0 && tid == 0) {
+        SP2Rec nx = s_dec.next;
+        nx.done = 1;
+        nx.last_branch = BR_STOP;
+        p.rec[k + 1] = nx;
+        p.sout->nupd = k;
+        p.sout->iter = nx.iter;
+        p.sout->status = nx.status;
+        p.sout->done = 1;
+      }
+      return;
+    }
+    const bool sq = s_dec.branch == BR_X2;
+    const double alpha = sq ? 1.0 : -1.0, beta = sq ? 0.0 : 2.0;
+    double s[kSums] = {0.0, 0.0, 0.0, 0.0, 0.0};
+
+    if (warp == C::NW) {
+      // ---------------- producer ----------------
+      if (lane == 0) {
+        fence_proxy_async_global();   // the other CTAs' X_k, then the TMA reads
+        const CUtensorMap* mx = &maps.x[k & 1];
+        const CUtensorMap* md = &maps.d[k & 1];
+        for (int seg = 0; seg < nseg; ++seg) {
+          int job, k0, k1, bi, bj;
+          segment(seg, job, k0, k1);
+          const bool isx = job < p.ntiles;
+          upper_tile(isx ? job : job - p.ntiles, bi, bj);
+          const bool one = isx && bi == bj;   // a diagonal tile of X^2: A and B are the same
+          for (int kk = k0; kk < k1; ++kk, ++g) {
+            const int st = g % C::ST;
+            if (g >= (uint32_t)C::ST)
+              mbar_wait(smem_u32(&bar_empty[st]), (g / C::ST - 1) & 1, &s_abort);
+            const uint32_t fb = smem_u32(&bar_full[st]), dst = sbase + st * C::STAGE;
+            const bool second = kk >= p.kb;   // Delta X after X Delta
+            const int row = (second ? kk - p.kb : kk) * C::BK;
+            mbar_expect_tx(fb, one ? C::OPERAND : C::STAGE);
+            tma_load_3d(dst, second ? md : mx, fb, 0, row, bi * (BT / 16));
+            if (!one)
+              tma_load_3d(dst + C::OPERAND, isx || second ? mx : md, fb, 0, row, bj * (BT / 16));
+          }
+        }
+      }
+      __syncwarp();
+    } else {
+      // ---------------- consumers ----------------
+      double2* stash = reinterpret_cast<double2*>(smem_raw + (sbase - smem_u32(smem_raw)) +
+                                                  C::ST * C::STAGE) + tid;   // this thread's
+      const int am8 = warp / C::WN * C::MI, bn8 = warp % C::WN * C::NI;
+      for (int seg = 0; seg < nseg; ++seg) {
+        int job, k0, k1, bi, bj;
+        segment(seg, job, k0, k1);
+        const bool isx = job < p.ntiles;
+        upper_tile(isx ? job : job - p.ntiles, bi, bj);
+        const bool diag = bi == bj;
+        const uint32_t boff = isx && diag ? 0 : C::OPERAND;
+        double acc[C::MI][C::NI][2];
+#pragma unroll
+        for (int mi = 0; mi < C::MI; ++mi)
+#pragma unroll
+          for (int ni = 0; ni < C::NI; ++ni) acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
+        // X Delta and Delta X are summed apart (one chain of 2 n terms has more rounding
+        // error than two of n): the first waits in shared memory
+        const bool both = !isx && k0 < p.kb && k1 > p.kb;
+        for (int kk = k0; kk < k1; ++kk, ++g) {
+          const int st = g % C::ST;
+          if (both && kk == p.kb) {
+#pragma unroll
+            for (int mi = 0; mi < C::MI; ++mi)
+#pragma unroll
+              for (int ni = 0; ni < C::NI; ++ni) {
+                stash[(mi * C::NI + ni) * C::NT] = make_double2(acc[mi][ni][0], acc[mi][ni][1]);
+                acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
+              }
+          }
+          mbar_wait(smem_u32(&bar_full[st]), (g / C::ST) & 1, &s_abort);
+          const uint32_t a = sbase + st * C::STAGE;
+          C::mma(a, a + boff, am8, bn8, frag, acc);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&bar_empty[st]));
+        }
+        if (both) {
+#pragma unroll
+          for (int mi = 0; mi < C::MI; ++mi)
+#pragma unroll
+            for (int ni = 0; ni < C::NI; ++ni) {
+              const double2 v = stash[(mi * C::NI + ni) * C::NT];
+              acc[mi][ni][0] += v.x;
+              acc[mi][ni][1] += v.y;
+            }
+        }
+        if (open && seg == 0) {
+          // the head (or a middle piece) of a tile another CTA finishes
+          double2* w = reinterpret_cast<double2*>(p.ws) + (size_t)cta * (BT * BT / 2) + tid;
+#pragma unroll
+          for (int mi = 0; mi < C::MI; ++mi)
+#pragma unroll
+            for (int ni = 0; ni < C::NI; ++ni)
+              w[(mi * C::NI + ni) * C::NT] = make_double2(acc[mi][ni][0], acc[mi][ni][1]);
+          __threadfence();
+          consumer_sync<C::NT>();
+          if (tid == 0)
+            asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p.flags + cta),
+                         "r"((unsigned)(k + 1 - p.k0))
+                         : "memory");
+          continue;
+        }
+        if (k0 > 0) {
+          // add the pieces other CTAs hold
+          for (int q = 0; q < s_npiece; ++q) {
+            const int c = s_piece[q];
+            if (tid == 0 && !s_abort &&
+                !spin_until(p.flags + c, (unsigned)(k + 1 - p.k0), p.err))
+              s_abort = 1;
+            consumer_sync<C::NT>();
+            const double2* w = reinterpret_cast<const double2*>(p.ws) + (size_t)c * (BT * BT / 2) + tid;
+#pragma unroll
+            for (int mi = 0; mi < C::MI; ++mi)
+#pragma unroll
+              for (int ni = 0; ni < C::NI; ++ni) {
+                const double2 v = __ldcg(w + (mi * C::NI + ni) * C::NT);
+                acc[mi][ni][0] += v.x;
+                acc[mi][ni][1] += v.y;
+              }
+          }
+        }
+        // out = alpha acc + beta E, mirrored store, FP64 sums (of X, and Tr Delta')
+        const double* E = isx ? p.x[k & 1] : p.d[k & 1];
+        double* out = isx ? p.x[(k + 1) & 1] : p.d[(k + 1) & 1];
+#pragma unroll
+        for (int mi = 0; mi < C::MI; ++mi) {
+#pragma unroll
+          for (int ni = 0; ni < C::NI; ++ni) {
+            const int r = bi * BT + C::row(mi), c = bj * BT + C::col(ni);
+            const double2 e = __ldcg(reinterpret_cast<const double2*>(E + (size_t)r * ld + c));
+            const double a0 = acc[mi][ni][0], a1 = acc[mi][ni][1];
+            const double v0 = alpha * a0 + beta * e.x;
+            const double v1 = alpha * a1 + beta * e.y;
+            if (isx) {
+              const double d0 = e.x - a0, d1 = e.y - a1;
+              if (!diag && p.core <= 0) {
+                s[0] += 2.0 * (v0 * v0 + v1 * v1);
+                s[2] += 2.0 * (d0 * d0 + d1 * d1);
+              } else {
+                const int w0 = sym_weight(diag, r, c), w1 = sym_weight(diag, r, c + 1);
+                s[0] += w0 * v0 * v0 + w1 * v1 * v1;
+                s[2] += core_weight(w0, r, c, p.core) * d0 * d0 +
+                        core_weight(w1, r, c + 1, p.core) * d1 * d1;
+                if (r == c) { s[1] += v0; s[3] += a0; }
+                if (r == c + 1) { s[1] += v1; s[3] += a1; }
+              }
+            } else {
+              if (r == c) s[4] += v0;
+              if (r == c + 1) s[4] += v1;
+            }
+            if (!diag) {
+              *reinterpret_cast<double2*>(out + (size_t)r * ld + c) = make_double2(v0, v1);
+              out[(size_t)c * ld + r] = v0;
+              out[(size_t)(c + 1) * ld + r] = v1;
+            } else {
+              if (r <= c) { out[(size_t)r * ld + c] = v0; out[(size_t)c * ld + r] = v0; }
+              if (r <= c + 1) { out[(size_t)r * ld + c + 1] = v1; out[(size_t)(c + 1) * ld + r] = v1; }
+            }
+          }
+        }
+      }
+      fence_proxy_async_global();   // these stores, then the other CTAs' TMA reads
+      __threadfence();
+    }
+
+    // ---- grid barrier, the step's sums and the next decision ----
+#pragma unroll
+    for (int q = 0; q < kSums; ++q) s[q] = warp_sum(s[q]);
+    if (lane == 0)
+      for (int q = 0; q < kSums; ++q) s_red[q][warp] = s[q];
+    __syncthreads();
+    double* part = p.partials + (size_t)(k & 1) * G * kSums;
+    if (warp == 0) {
+#pragma unroll
+      for (int q = 0; q < kSums; ++q) s[q] = warp_sum(lane < C::NW ? s_red[q][lane] : 0.0);
+    }
+    if (tid == 0) {
+      for (int q = 0; q < kSums; ++q) part[(size_t)q * G + cta] = s[q];
+      __threadfence();
+      atomicAdd(p.bar, 1u);
+      if (!s_abort && !spin_until(p.bar, (unsigned)G * (unsigned)(k + 1 - p.k0), p.err)) s_abort = 1;
+      if (s_abort) {
+        // the call reports SP2B_TIMEOUT; the other CTAs leave at their next wait
+        atomicExch(p.err, 1);
+        p.sout->status = SP2B_TIMEOUT;
+        __threadfence();
+        p.sout->done = 1;
+      }
+      __threadfence();
+    }
+    __syncthreads();
+    if (s_abort) {
+      // leave no copy of this CTA in flight: wait (bounded) for the last ones issued
+      if (warp == C::NW && lane == 0)
+        for (uint32_t u = g > (uint32_t)C::ST ? g - C::ST : 0; u < g; ++u)
+          for (uint32_t i = 0; i < kSpinLimit; ++i)
+            if (mbar_try(smem_u32(&bar_full[u % C::ST]), (u / C::ST) & 1)) break;
+      return;
+    }
+    // warp q sums total q over the CTAs, in CTA order per lane
+    if (warp < kSums) {
+      double v = 0.0;
+      for (int j = lane; j < G; j += 32) v += __ldcg(part + (size_t)warp * G + j);
+      v = warp_sum(v);
+      if (lane == 0) s_tot[warp] = v;
+    }
+    __syncthreads();
+    if (tid == 0) {
+      const double* t = s_tot;
+      SP2Rec nx = s_dec.next;
+      nx.fro2 = t[0];
+      nx.trx_data = t[1];
+      nx.trp = t[3];
+      nx.pbias = s_fro2 - t[3];
+      nx.last_branch = s_dec.branch;
+      if (!(t[0] == t[0]) || !(t[1] == t[1]) || !(t[2] == t[2]) || t[0] > 1e300) {
+        nx.status = SP2B_BAD_INPUT;
+        nx.done = 1;
+      }
+      if (cta == 0) {
+        if (p.pp_out) p.pp_out[k] = s_dec.branch;
+        if (p.vv_out) {
+          if (p.vv_accumulate) p.vv_out[k] += t[2];
+          else p.vv_out[k] = sqrt(t[2]);
+        }
+        if (p.trd_out) *p.trd_out = t[4];
+        p.rec[k + 1] = nx;
+        p.sout->nupd = k + 1;
+        p.sout->iter = nx.iter;
+        p.sout->status = nx.status;
+        if (nx.done) p.sout->done = 1;
+      }
+      if (nx.done) {
+        s_run = 0;
+      } else {
+        s_dec = sp2_decide(p.ctl, nx, k + 1, p.pp_in);
+        s_fro2 = nx.fro2;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+namespace {
+
+struct F64Plan {
+  int bt, tiles, grid, snap;
+};
+
+// Grid of an order-n solve: one CTA per SM, but at least kMinUnits k-blocks each (a cut tile
+// costs its owner and the others ~2 us of workspace traffic, four to eight k-blocks of a
+// 64-edge tile; cutting 32-edge tiles, 0.13 us a k-block, pays only for longer pieces).
+F64Plan f64_plan(int n, int bt, bool resp) {
+  F64Plan pl;
+  pl.bt = bt;
+  pl.tiles = (n + bt - 1) / bt;
+  const int kb = (n + 15) / 16, min_units = bt == 32 ? 24 : 8;
+  const long long tiles = (long long)pl.tiles * (pl.tiles + 1) / 2;
+  const long long units = tiles * kb * (resp ? 3 : 1), jobs = tiles * (resp ? 2 : 1);
+  pl.snap = 4;
+  pl.grid = (int)std::min<long long>(device_sms(), std::max(jobs, units / min_units));
+  return pl;
+}
+
+template <int BT>
+cudaError_t launch_solve(const F64SolveArgs& a, int grid, cudaStream_t st) {
+  using C = F64Tile<BT>;
+  F64SolveMaps m;
+  for (int i = 0; i < 2; ++i)
+    if (!make_tmap_f64(&m.x[i], a.x[i], a.ld, a.ld, BT) ||
+        !make_tmap_f64(&m.d[i], a.d[i] ? a.d[i] : a.x[i], a.ld, a.ld, BT))
+      return cudaErrorInvalidValue;
+  // the response keeps one tile of sums beside the stages
+  const size_t smem = C::SMEM + (a.d[0] ? BT * BT * sizeof(double) : 0);
+  const cudaError_t e = cudaFuncSetAttribute(k_f64_solve<BT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)smem);
+  if (e != cudaSuccess) return e;
+  void* args[] = {(void*)&m, (void*)&a};
+  return cudaLaunchCooperativeKernel((const void*)k_f64_solve<BT>, dim3(grid), dim3(C::NT + 32), args,
+                                     smem, st);
+}
+
+}  // namespace
+
+// Tile edge of an order-n solve: 32 up to kSmallN, where 64-edge tiles are too few for the
+// SMs (n = 300: 235 us a solve with 32, 270 us with 64; n = 500: 296 and 284); above it the
+// measured choice for this device and padded size (tune_f64_solve), else 64.
+constexpr int kSmallN = 416;
+int f64_solve_tile(int n, int np, bool resp) {
+  if (n <= kSmallN) return 32;
+  int c = 0;
+  if (resp) return 64;   // a 128-edge tile of sums does not fit beside the stages
+  return tune_lookup(f64_tune_key(np), &c) && (c == 64 || c == 128) ? c : 64;
+}
+
+// Steps per launch: a launch stays below a tenth of a second (30 TFLOP/s of symmetric
+// products), so that a long solve leaves the GPU to others in between.
+int f64_solve_chunk(int n, bool resp) {
+  const double flops = (double)n * n * n * (resp ? 3.0 : 1.0);
+  return (int)std::max(1.0, std::min(1e6, 2e12 / flops));
+}
+
+static size_t solve_work(const F64Plan& pl) {
+  return (size_t)pl.grid * pl.bt * pl.bt + 2 * (size_t)pl.grid * kSums + pl.grid / 2 + 2;
+}
+
+// Workspace of an order-n solve, for either tile edge the tuner may try.
+size_t f64_solve_ws_doubles(int n, bool resp) {
+  if (n <= kSmallN) return solve_work(f64_plan(n, 32, resp));
+  if (resp) return solve_work(f64_plan(n, 64, resp));
+  return std::max(solve_work(f64_plan(n, 64, resp)), solve_work(f64_plan(n, 128, resp)));
+}
+
+static cudaError_t launch_f64_solve_bt(const F64SolveArgs& a0, int n, int np, int bt, double* work,
+                                       cudaStream_t st) {
+  F64SolveArgs a = a0;
+  const F64Plan pl = f64_plan(n, bt, a.d[0] != nullptr);
+  a.ld = np;
+  a.kb = (n + 15) / 16;
+  a.ntiles = pl.tiles * (pl.tiles + 1) / 2;
+  a.snap = pl.snap;
+  a.ws = work;
+  a.partials = work + (size_t)pl.grid * pl.bt * pl.bt;
+  a.flags = reinterpret_cast<unsigned*>(a.partials + 2 * (size_t)pl.grid * kSums);
+  a.bar = a.flags + pl.grid;
+  cudaError_t e = cudaMemsetAsync(a.flags, 0, (pl.grid + 1) * sizeof(unsigned), st);
+  if (e != cudaSuccess) return e;
+  if (pl.bt == 32) e = launch_solve<32>(a, pl.grid, st);
+  else if (pl.bt == 64) e = launch_solve<64>(a, pl.grid, st);
+  else e = launch_solve<128>(a, pl.grid, st);
+  note_launch();
+  return e == cudaSuccess ? cudaGetLastError() : e;
+}
+
+cudaError_t launch_f64_solve(const F64SolveArgs& a, int n, int np, double* work, cudaStream_t st) {
+  return launch_f64_solve_bt(a, n, np, f64_solve_tile(n, np, a.d[0] != nullptr), work, st);
+}
+
+// Measures the tile edges 128 and 64 at np (one SP2 step each) and records the faster one
+// for f64_solve_tile.  `a` as for a solve; its records, sums and iterates are overwritten.
+int tune_f64_solve(int n, int np, const F64SolveArgs& a0, double* work, cudaStream_t st) {
+  int c = 0;
+  const std::string key = f64_tune_key(np);
+  if (n <= kSmallN || a0.d[0] || !tune_enabled() || tune_lookup(key, &c)) return SP2B_OK;
+  F64SolveArgs a = a0;
+  a.k0 = 0;
+  a.k1 = 1;
+  a.ctl.algo = ALGO_SEQ;
+  a.ctl.icount = 1;
+  a.pp_out = nullptr;
+  a.vv_out = nullptr;
+  a.trd_out = nullptr;
+  // timed on zeros (the buffers may not hold data yet; DMMA time does not depend on values)
+  const size_t bytes = (size_t)np * np * sizeof(double);
+  if (cudaMemsetAsync(a.x[0], 0, bytes, st) != cudaSuccess ||
+      cudaMemsetAsync(const_cast<int*>(a.pp_in), 0, sizeof(int), st) != cudaSuccess ||
+      cudaMemsetAsync(a.rec, 0, sizeof(SP2Rec), st) != cudaSuccess ||
+      cudaMemsetAsync(a.err, 0, sizeof(int), st) != cudaSuccess)
+    return SP2B_CUDA_ERROR;
+  const int edges[2] = {128, 64};
+  std::vector<float> ms;
+  int best = 0;
+  const int rc = tune_measure(2, 2, st, [&](int cand) -> int {
+    return launch_f64_solve_bt(a, n, np, edges[cand], work, st) == cudaSuccess ? SP2B_OK
+                                                                             : SP2B_CUDA_ERROR;
+  }, &ms, &best);
+  if (rc == SP2B_OK) tune_store(key, edges[best], ms);
+  return rc;
+}
+
+}  // namespace sp2b

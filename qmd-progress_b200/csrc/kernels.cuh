@@ -60,10 +60,8 @@ struct StepArgs {
 };
 
 // FP64 path ---------------------------------------------------------------------------
-int f64_tile(int np);  // tile edge chosen for this size (64 or 128)
+int f64_tile(int np);  // tile edge of a single product of this size (64 or 128)
 std::string f64_tune_key(int np);
-int tune_f64_tile(int np, const double* x_in, double* x_out, double* partials, unsigned* counter,
-                  double* sums_out, cudaStream_t st);
 int device_sms();       // SM count of the current device
 int f64_ntiles(int np);
 cudaError_t launch_gersh(const double* h, int n, int ld, double* rowsum, int nsplit,
@@ -74,6 +72,36 @@ cudaError_t launch_normalize_f64(const double* h, int n, int ld, int np, const d
                                  double* norm_out, cudaStream_t st);
 cudaError_t launch_sym_gemm_f64(const StepArgs& a, cudaStream_t st);
 cudaError_t launch_sym_gemm_f64_batched(const StepArgs& a, int bt, cudaStream_t st);
+
+// SP2 steps [k0, k1) of a dense solve in one cooperative launch (k_f64_solve.cu); fewer
+// when the loop ends first.  With d[0] != nullptr each step also forms the response
+// Delta' = a {X, Delta} + b Delta, (a, b) the step's branch.
+struct F64SolveArgs {
+  double* x[2];         // ping-pong iterates, np x np; x[k0 & 1] holds X_k0
+  double* d[2];         // ping-pong Delta, or null
+  int k0, k1;
+  int core;             // > 0: residual sums over the first `core` rows only
+  SP2Ctl ctl;
+  SP2Rec* rec;
+  const int* pp_in;
+  int* pp_out;
+  double* vv_out;
+  int vv_accumulate;
+  double* trd_out;      // Tr Delta' of the last step taken (may be null)
+  SolveOut* sout;
+  int* err;
+  // set by launch_f64_solve
+  int ld, kb, ntiles, snap;
+  double* ws;           // one BT x BT piece per CTA
+  double* partials;
+  unsigned* flags;      // per CTA: its piece of step k is complete (k + 1 - k0)
+  unsigned* bar;        // grid barrier counter
+};
+int f64_solve_tile(int n, int np, bool resp);
+int tune_f64_solve(int n, int np, const F64SolveArgs& a, double* work, cudaStream_t st);
+size_t f64_solve_ws_doubles(int n, bool resp);
+int f64_solve_chunk(int n, bool resp);
+cudaError_t launch_f64_solve(const F64SolveArgs& a, int n, int np, double* work, cudaStream_t st);
 
 // All maxiter SP2 steps of a small batch of parts (the FP64 re-solve of flagged parts)
 // in one cooperative launch: one CTA per 32 x 32 upper tile; the tiles of a part meet

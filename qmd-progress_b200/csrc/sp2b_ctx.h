@@ -14,10 +14,12 @@ struct Ctx {
   cudaStream_t stream = nullptr;
   std::mutex mu;
   // FP64 square buffers (np x np): ping-pong iterates [0, 1]; the FP64-DMMA McWeeny
-  // product [2]; the forward-mode response's Delta ping-pong [2, 3] and its first
-  // product / host staging [4]
+  // product [2]; the forward-mode response's Delta ping-pong [2, 3] and host staging [4]
   double* x64[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   size_t x64_cap[5] = {0, 0, 0, 0, 0};
+  // FP64 solve: pieces of cut tiles, partial sums, flags
+  double* f64w = nullptr;
+  size_t f64w_cap = 0;
   // split-precision iterates (hi/lo ping-pong)
   __half* hi[2] = {nullptr, nullptr};
   __half* lo[2] = {nullptr, nullptr};
@@ -56,6 +58,7 @@ struct Ctx {
   std::vector<cudaEvent_t> ev_ref;  // INT8 refinement phase boundaries
 
   cudaError_t ensure_f64(int np, int nbuf);
+  cudaError_t ensure_f64_solve(int n, bool resp);
   cudaError_t ensure_split(int np);
   cudaError_t ensure_common(size_t nin, int np, int maxlaunch, int n);
   cudaError_t ensure_oz(int np, cudaStream_t st);

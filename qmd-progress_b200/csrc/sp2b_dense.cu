@@ -87,6 +87,10 @@ cudaError_t Ctx::ensure_f64(int np, int nbuf) {
   return cudaSuccess;
 }
 
+cudaError_t Ctx::ensure_f64_solve(int n, bool resp) {
+  return grow(f64w, f64w_cap, f64_solve_ws_doubles(n, resp));
+}
+
 cudaError_t Ctx::ensure_split(int np) {
   for (int i = 0; i < 2; ++i) {
     cudaError_t e = grow(hi[i], hi_cap[i], (size_t)np * np);
@@ -236,12 +240,25 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
                         np <= 65536;
   const size_t nn = (size_t)n * n;
   SP2B_CUDA_TRY(c->ensure_common(j.dev_ptrs ? 0 : nn, np, maxlaunch, n));
-  SP2B_CUDA_TRY(c->ensure_f64(np, split ? (oz ? 1 : 3) : (resp ? 5 : 2)));
+  SP2B_CUDA_TRY(c->ensure_f64(np, split ? (oz ? 1 : 3) : (resp ? (j.dev_ptrs ? 4 : 5) : 2)));
   if (split) SP2B_CUDA_TRY(c->ensure_split(np));
-  // FP64 steps: the measured tile edge for this size (first solve at np on this device)
-  if (!split && !exact) {
-    const int trc = tune_f64_tile(np, c->x64[0], c->x64[1], c->partials, c->counter,
-                                  c->small + 16, st);
+  const bool fp64 = !split && !exact;
+  F64SolveArgs fa;
+  memset(&fa, 0, sizeof(fa));
+  if (fp64) {
+    for (int i = 0; i < 2; ++i) {
+      fa.x[i] = c->x64[i];
+      fa.d[i] = resp ? c->x64[2 + i] : nullptr;
+    }
+    fa.core = j.core;
+    fa.ctl = j.ctl;
+    fa.rec = c->rec;
+    fa.pp_in = c->pp_dev;
+    fa.sout = c->sout;
+    fa.err = c->err;
+    SP2B_CUDA_TRY(c->ensure_f64_solve(n, resp));
+    // the measured tile edge for this size (first solve at np on this device)
+    const int trc = tune_f64_solve(n, np, fa, c->f64w, st);
     if (trc != SP2B_OK) {
       set_last_error("FP64 tile tuning failed");
       return trc;
@@ -303,7 +320,8 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
   }
   int* pp_out_dev = (j.ctl.algo == ALGO_SEQ) ? nullptr : c->pp_dev;
 
-  // ---- SP2 steps: one launch each, chunked host polling of the device "done" word ----
+  // ---- SP2 steps: FP64 many per launch, else one launch each; the host polls the device
+  // "done" word between chunks ----
   StepArgs a;
   memset(&a, 0, sizeof(a));
   a.np = np;
@@ -328,8 +346,11 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
   a.partials = c->partials;
   a.counter = c->counter;
   a.err = c->err;
+  fa.pp_out = pp_out_dev;
+  fa.vv_out = c->vv_dev;
+  fa.vv_accumulate = j.vv_accumulate;
   int k = 0;
-  int chunk = 4;
+  int chunk = fp64 ? f64_solve_chunk(n, resp) : 4;
   bool done = (maxlaunch == 0);
   const bool timing = g_step_timing.load() != 0;
   while (!done && k < maxlaunch) {
@@ -341,11 +362,20 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
     if (fallback) kend = std::min(kend, std::max(j.exact_switch, k + 1));
     const int k0 = k;
     if (timing) {
-      while ((int)c->ev.size() < 2 * chunk) {
+      while ((int)c->ev.size() < (fp64 ? 2 : 2 * chunk)) {
         cudaEvent_t e;
         SP2B_CUDA_TRY(cudaEventCreate(&e));
         c->ev.push_back(e);
       }
+    }
+    if (fp64) {
+      // every step up to kend in one launch, the branch decisions inside it
+      fa.k0 = k;
+      fa.k1 = kend;
+      if (timing) SP2B_CUDA_TRY(cudaEventRecord(c->ev[0], st));
+      SP2B_CUDA_TRY(launch_f64_solve(fa, n, np, c->f64w, st));
+      if (timing) SP2B_CUDA_TRY(cudaEventRecord(c->ev[1], st));
+      k = kend;
     }
     for (; k < kend; ++k) {
       a.k = k;
@@ -366,45 +396,26 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
         a.E = c->x64[bin];
         a.out = c->x64[bout];
         SP2B_CUDA_TRY(launch_oz_crt_step(c->oz_q, c->oz_scale, a, st));
-      } else if (split) {
+      } else {
         a.A = a.B = a.E = c->hi[bin];
         a.A_lo = a.B_lo = a.E_lo = c->lo[bin];
         a.out = c->hi[bout];
         a.out_lo = c->lo[bout];
         a.ntiles = tc_ntiles(np);
         SP2B_CUDA_TRY(launch_sym_gemm_tc(a, bf16, st));
-      } else {
-        a.A = a.B = a.E = c->x64[bin];
-        a.out = c->x64[bout];
-        a.ntiles = f64_ntiles(np);
-        SP2B_CUDA_TRY(launch_sym_gemm_f64(a, st));
       }
       if (timing) SP2B_CUDA_TRY(cudaEventRecord(c->ev[2 * (k - k0) + 1], st));
-      if (resp) {
-        // {X_k, Delta_k} on the upper tiles from two products that follow step k's branch
-        // (a, b) = (1, 0) or (-1, 2): P1 = a X Delta + b Delta, Delta' = a Delta X + P1
-        // (src/prg_response_mod.F90:725-746); both exactly symmetric by construction
-        StepArgs q = a;
-        q.pp_out = nullptr;
-        q.vv_out = nullptr;
-        q.sums_out = c->small + 24;
-        q.control = 2;
-        q.A = c->x64[bin];
-        q.B = q.E = c->x64[2 + bin];
-        q.out = c->x64[4];
-        SP2B_CUDA_TRY(launch_sym_gemm_f64(q, st));
-        q.control = 3;
-        q.A = c->x64[2 + bin];
-        q.B = c->x64[bin];
-        q.E = c->x64[4];
-        q.out = c->x64[2 + bout];
-        SP2B_CUDA_TRY(launch_sym_gemm_f64(q, st));
-      }
     }
     SP2B_CUDA_TRY(cudaMemcpyAsync(c->h_sout, c->sout, sizeof(SolveOut), cudaMemcpyDeviceToHost, st));
     SP2B_CUDA_TRY(cudaStreamSynchronize(st));
     done = c->h_sout->done != 0;
-    if (timing) {
+    if (timing && fp64) {
+      float ms = 0.f;
+      SP2B_CUDA_TRY(cudaEventElapsedTime(&ms, c->ev[0], c->ev[1]));
+      std::lock_guard<std::mutex> lk2(g_timing_mu);
+      g_step_ms += ms;
+      g_step_timed += (done ? c->h_sout->nupd : kend) - k0;   // steps
+    } else if (timing) {
       // only launches that did work (k < the launch that finished the loop, + itself)
       double ms = 0.0;
       long long cnt = 0;
@@ -419,7 +430,7 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
       g_step_ms += ms;
       g_step_timed += cnt;
     }
-    chunk = std::min(chunk * 2, 16);
+    if (!fp64) chunk = std::min(chunk * 2, 16);
   }
   c->last_launches = k;
   SolveOut so = *c->h_sout;

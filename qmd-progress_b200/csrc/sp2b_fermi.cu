@@ -3,9 +3,9 @@
 // number of SP2 steps (the sequence generated on the device in the first pass of the
 // init, replayed after), and the host takes one Newton step on mu from the traces the
 // last step published.  prg_sp2_fermi_init also carries X1 = dX/dmu through the same
-// recursion, as the forward-mode response does (two FP64 products per step following
-// the step's branch); prg_sp2_fermi ends with X + lambda DX, DX = -beta X (I - X), as one
+// recursion, as the forward-mode response does ({X, X1} with the step's branch); prg_sp2_fermi ends with X + lambda DX, DX = -beta X (I - X), as one
 // more product: (1 - lambda beta) X + lambda beta X^2.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -38,14 +38,18 @@ int fermi_pass(Ctx* c, const double* hdev, int n, int nsteps, double nocc, doubl
   SP2B_CUDA_TRY(cudaMemsetAsync(c->counter, 0, 4 * sizeof(unsigned), st));
   SP2B_CUDA_TRY(cudaMemsetAsync(c->err, 0, sizeof(int), st));
   SP2B_CUDA_TRY(cudaMemsetAsync(c->sout, 0, sizeof(SolveOut), st));
-  SP2B_CUDA_TRY(cudaMemsetAsync(c->small + 24, 0, 4 * sizeof(double), st));
+  SP2B_CUDA_TRY(cudaMemsetAsync(c->small + 24, 0, sizeof(double), st));
   SP2B_CUDA_TRY(launch_normalize_f64(hdev, n, n, np, bounds, c->x64[0], c->partials, c->counter,
                                      c->rec, norm_out, st));
   if (deriv) SP2B_CUDA_TRY(launch_resp_init(nullptr, n, n, np, bounds, c->x64[2], st));
-  StepArgs a;
+  // X <- X^2 or 2X - X^2, and X1 <- {X, X1} or 2 X1 - {X, X1} with X = X_k
+  // (src/prg_sp2_fermi_mod.F90:113-120)
+  F64SolveArgs a;
   memset(&a, 0, sizeof(a));
-  a.np = np;
-  a.control = 1;
+  for (int i = 0; i < 2; ++i) {
+    a.x[i] = c->x64[i];
+    a.d[i] = deriv ? c->x64[2 + i] : nullptr;
+  }
   a.ctl.algo = gen ? ALGO_FERMI_GEN : ALGO_SEQ;
   a.ctl.icount = nsteps;
   a.ctl.maxit = nsteps + 1;
@@ -54,40 +58,19 @@ int fermi_pass(Ctx* c, const double* hdev, int n, int nsteps, double nocc, doubl
   a.rec = c->rec;
   a.pp_in = c->pp_dev;
   a.pp_out = gen ? c->pp_dev : nullptr;
+  a.trd_out = c->small + 24;
   a.sout = c->sout;
-  a.partials = c->partials;
-  a.counter = c->counter;
   a.err = c->err;
-  a.ntiles = f64_ntiles(np);
-  for (int k = 0; k < nsteps; ++k) {
-    a.k = k;
-    const int bin = k & 1, bout = (k + 1) & 1;
-    a.A = a.B = a.E = c->x64[bin];
-    a.out = c->x64[bout];
-    SP2B_CUDA_TRY(launch_sym_gemm_f64(a, st));
-    if (deriv) {
-      // X1 <- {X, X1} or 2 X1 - {X, X1} with X = X_k (src/prg_sp2_fermi_mod.F90:113-120):
-      // P1 = a X X1 + b X1, X1' = a X1 X + P1, (a, b) the step's (1, 0) or (-1, 2)
-      StepArgs q = a;
-      q.pp_out = nullptr;
-      q.sums_out = c->small + 24;
-      q.control = 2;
-      q.A = c->x64[bin];
-      q.B = q.E = c->x64[2 + bin];
-      q.out = c->x64[4];
-      SP2B_CUDA_TRY(launch_sym_gemm_f64(q, st));
-      q.control = 3;
-      q.A = c->x64[2 + bin];
-      q.B = c->x64[bin];
-      q.E = c->x64[4];
-      q.out = c->x64[2 + bout];
-      SP2B_CUDA_TRY(launch_sym_gemm_f64(q, st));
-    }
+  const int chunk = f64_solve_chunk(n, deriv);
+  for (int k = 0; k < nsteps; k += chunk) {
+    a.k0 = k;
+    a.k1 = std::min(nsteps, k + chunk);
+    SP2B_CUDA_TRY(launch_f64_solve(a, n, np, c->f64w, st));
   }
   SP2Rec r;
   SP2B_CUDA_TRY(cudaMemcpyAsync(c->h_sout, c->sout, sizeof(SolveOut), cudaMemcpyDeviceToHost, st));
   SP2B_CUDA_TRY(cudaMemcpyAsync(&r, c->rec + nsteps, sizeof(SP2Rec), cudaMemcpyDeviceToHost, st));
-  SP2B_CUDA_TRY(cudaMemcpyAsync(c->h_small + 24, c->small + 24, 4 * sizeof(double),
+  SP2B_CUDA_TRY(cudaMemcpyAsync(c->h_small + 24, c->small + 24, sizeof(double),
                                 cudaMemcpyDeviceToHost, st));
   SP2B_CUDA_TRY(cudaMemcpyAsync(c->h_small + 8, norm_out, 4 * sizeof(double), cudaMemcpyDeviceToHost, st));
   SP2B_CUDA_TRY(cudaStreamSynchronize(st));
@@ -107,8 +90,7 @@ int fermi_pass(Ctx* c, const double* hdev, int n, int nsteps, double nocc, doubl
   }
   out->trx = r.trx_data;
   out->fro2 = r.fro2;
-  // Tr X1: the last control-3 product publishes the trace of its output, X1_nsteps
-  out->trx1 = nsteps > 0 ? c->h_small[24 + 1] : -(double)n / (hN - h1);
+  out->trx1 = nsteps > 0 ? c->h_small[24] : -(double)n / (hN - h1);
   if (!(out->trx == out->trx) || !(out->fro2 == out->fro2) || !(out->trx1 == out->trx1)) {
     set_last_error("non-finite values during SP2-Fermi");
     return SP2B_BAD_INPUT;
@@ -143,7 +125,8 @@ int fermi_setup(const double* h, int n, int nsteps, bool deriv, const sp2b_opts*
   const int np = padded(n);
   const size_t nn = (size_t)n * n;
   SP2B_CUDA_TRY(c->ensure_common(s->dev ? 0 : nn, np, nsteps + 2, n));
-  SP2B_CUDA_TRY(c->ensure_f64(np, deriv ? 5 : 2));
+  SP2B_CUDA_TRY(c->ensure_f64(np, deriv ? 4 : 2));
+  SP2B_CUDA_TRY(c->ensure_f64_solve(n, deriv));
   s->hdev = h;
   if (!s->dev) {
     SP2B_CUDA_TRY(cudaMemcpyAsync(c->hin, h, nn * sizeof(double), cudaMemcpyHostToDevice, s->st));
