@@ -3,7 +3,6 @@
 #include <algorithm>
 #include <cstring>
 #include <string>
-#include <vector>
 
 #include "f64_dmma.cuh"
 #include "reduce.cuh"
@@ -336,26 +335,15 @@ __global__ void __launch_bounds__(WM* WN * 32, 1) k_sym_gemm_f64(const StepArgs 
     if (br == BR_X2) { alpha = 1.0; beta = 0.0; }
     else { alpha = -1.0; beta = 2.0; }
   }
-  int bi, bj, nloc = p.np, core = p.core;
-  size_t row0 = 0;
-  if (p.tiles) {
-    const int4 t = p.tiles[blockIdx.x];
-    row0 = (size_t)t.x;
-    bi = t.y >> 16;
-    bj = t.y & 0xffff;
-    nloc = t.z;
-    core = t.w;
-  } else {
-    upper_tile(blockIdx.x, bi, bj);
-  }
+  int bi, bj;
+  upper_tile(blockIdx.x, bi, bj);
   const int i0 = bi * BT, j0 = bj * BT;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t4 = lane & 3;
   const int wm = warp / WN, wn = warp % WN;
   const int ld = p.ld;
-  // the part's square block starts at row row0 of the packed buffers
-  const double* __restrict__ A = (const double*)p.A + row0 * ld;
-  const double* __restrict__ B = (const double*)p.B + row0 * ld;
+  const double* __restrict__ A = (const double*)p.A;
+  const double* __restrict__ B = (const double*)p.B;
 
   double acc[C::MI][C::NI][2];
 #pragma unroll
@@ -363,9 +351,7 @@ __global__ void __launch_bounds__(WM* WN * 32, 1) k_sym_gemm_f64(const StepArgs 
 #pragma unroll
     for (int ni = 0; ni < C::NI; ++ni) acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
 
-  // every valid tile starts inside its part; anything else contributes nothing
-  const bool tile_ok = !p.tiles || (i0 < nloc && j0 < nloc);
-  const int KB = tile_ok ? nloc / C::BK : 0;
+  const int KB = p.np / C::BK;
   auto load = [&](int stage, int kb) {
     double* As = sm + stage * 2 * C::BK * C::LDS;
     double* Bs = As + C::BK * C::LDS;
@@ -408,11 +394,11 @@ __global__ void __launch_bounds__(WM* WN * 32, 1) k_sym_gemm_f64(const StepArgs 
 
   // ---- epilogue: out = alpha*acc + beta*E, mirrored store, FP64 sums ----
   const bool diag = (bi == bj);
-  const double* __restrict__ E = (const double*)p.E + row0 * ld;
-  double* __restrict__ out = p.out ? (double*)p.out + row0 * ld : nullptr;
+  const double* __restrict__ E = (const double*)p.E;
+  double* __restrict__ out = (double*)p.out;
   double s[4] = {0.0, 0.0, 0.0, 0.0};  // ||out||^2, Tr out, ||E-acc||^2 (core rows), Tr acc
 #pragma unroll
-  for (int mi = 0; mi < (tile_ok ? C::MI : 0); ++mi) {
+  for (int mi = 0; mi < C::MI; ++mi) {
 #pragma unroll
     for (int ni = 0; ni < C::NI; ++ni) {
       const int r = i0 + wm * C::TM + mi * 8 + g;
@@ -424,7 +410,7 @@ __global__ void __launch_bounds__(WM* WN * 32, 1) k_sym_gemm_f64(const StepArgs 
       const int w0 = sym_weight(diag, r, c), w1 = sym_weight(diag, r, c + 1);
       const double d0 = e.x - a0, d1 = e.y - a1;
       s[0] += w0 * v0 * v0 + w1 * v1 * v1;
-      s[2] += core_weight(w0, r, c, core) * d0 * d0 + core_weight(w1, r, c + 1, core) * d1 * d1;
+      s[2] += core_weight(w0, r, c, p.core) * d0 * d0 + core_weight(w1, r, c + 1, p.core) * d1 * d1;
       if (r == c) { s[1] += v0; s[3] += a0; }
       if (r == c + 1) { s[1] += v1; s[3] += a1; }
       if (out) {
@@ -440,153 +426,6 @@ __global__ void __launch_bounds__(WM* WN * 32, 1) k_sym_gemm_f64(const StepArgs 
     }
   }
   publish_and_finalize(p, s, red, &s_flag);
-}
-
-// Tiles of the one-launch form: 32 x 32, 8 warps of 16 x 8, k blocks of 64 in a 3-deep
-// pipeline (the k order of every sum is that of F64Cfg<32, 2, 4>: 4 at a time, ascending);
-// 110 KB of stages, two CTAs per SM.
-struct MsCfg {
-  static constexpr int BK = 64, NT = 256, LDS = 36, ST = 3;
-  static constexpr int TM = 16, TN = 8, MI = 2, NI = 1;
-  static constexpr size_t SMEM = (size_t)ST * 2 * BK * LDS * sizeof(double);
-};
-
-// All SP2 steps of a batch of parts in one cooperative launch (see MultiStepArgs).
-// Tile math and the order of every sum are those of k_sym_gemm_f64<32, 2, 4>, so each
-// part's result equals that of the per-step launches bit for bit; the per-step sums
-// (traces, vv) are not formed.  Between steps every CTA of a part adds one to the part's
-// counter and waits, with a bounded spin, until the part's tiles have all finished the
-// step; operands are read through L2 (cp.async.cg, ld.global.cg), never a stale L1 line.
-__global__ void __launch_bounds__(256, 1) k_f64_multistep(const MultiStepArgs a) {
-  using C = MsCfg;
-  extern __shared__ __align__(16) double sm[];
-  const int4 t = a.tiles[blockIdx.x];
-  const size_t row0 = (size_t)t.x;
-  const int bi = t.y >> 16, bj = t.y & 0xffff, nloc = t.z, part = t.w;
-  const unsigned per = (unsigned)a.part_tiles[part];
-  const int i0 = bi * 32, j0 = bj * 32;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int g = lane >> 2, t4 = lane & 3;
-  const int wm = warp / 4, wn = warp % 4;   // WM = 2, WN = 4
-  const int ld = a.ld;
-  const bool tile_ok = i0 < nloc && j0 < nloc;
-  const int KB = tile_ok ? nloc / C::BK : 0;
-  const bool diag = bi == bj;
-  __shared__ int s_bad;
-  if (tid == 0) s_bad = 0;
-  __syncthreads();
-  for (int k = 0; k < a.maxiter; ++k) {
-    const double* __restrict__ X = a.x[k & 1] + row0 * ld;
-    double* __restrict__ out = a.x[(k + 1) & 1] + row0 * ld;
-    const bool sq = a.pp[k] != 0;
-    const double alpha = sq ? 1.0 : -1.0, beta = sq ? 0.0 : 2.0;
-    double acc[C::MI][C::NI][2];
-#pragma unroll
-    for (int mi = 0; mi < C::MI; ++mi)
-#pragma unroll
-      for (int ni = 0; ni < C::NI; ++ni) acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
-    auto load = [&](int stage, int kb) {
-      double* As = sm + stage * 2 * C::BK * C::LDS;
-      double* Bs = As + C::BK * C::LDS;
-      const int k0 = kb * C::BK;
-      for (int c = tid; c < C::BK * 32 / 2; c += C::NT) {
-        const int row = c / 16, col = (c % 16) * 2;   // BT / 2 = 16 pieces per row
-        cp_async16(As + row * C::LDS + col, X + (size_t)(k0 + row) * ld + i0 + col);
-        cp_async16(Bs + row * C::LDS + col, X + (size_t)(k0 + row) * ld + j0 + col);
-      }
-    };
-#pragma unroll
-    for (int s = 0; s < C::ST - 1; ++s) {
-      if (s < KB) load(s, s);
-      cp_async_commit();
-    }
-    for (int kb = 0; kb < KB; ++kb) {
-      cp_async_wait<C::ST - 2>();
-      __syncthreads();
-      {
-        const int nk = kb + C::ST - 1;
-        if (nk < KB) load(nk % C::ST, nk);
-        cp_async_commit();
-      }
-      const double* As = sm + (kb % C::ST) * 2 * C::BK * C::LDS;
-      const double* Bs = As + C::BK * C::LDS;
-#pragma unroll
-      for (int kk = 0; kk < C::BK; kk += 4) {
-        double av[C::MI], bv[C::NI];
-#pragma unroll
-        for (int mi = 0; mi < C::MI; ++mi) av[mi] = As[(kk + t4) * C::LDS + wm * C::TM + mi * 8 + g];
-#pragma unroll
-        for (int ni = 0; ni < C::NI; ++ni) bv[ni] = Bs[(kk + t4) * C::LDS + wn * C::TN + ni * 8 + g];
-#pragma unroll
-        for (int mi = 0; mi < C::MI; ++mi)
-#pragma unroll
-          for (int ni = 0; ni < C::NI; ++ni) dmma884(acc[mi][ni], av[mi], bv[ni]);
-      }
-    }
-    cp_async_wait<0>();
-    __syncthreads();   // every warp is done with the stages before the next step reuses them
-#pragma unroll
-    for (int mi = 0; mi < (tile_ok ? C::MI : 0); ++mi) {
-#pragma unroll
-      for (int ni = 0; ni < C::NI; ++ni) {
-        const int r = i0 + wm * C::TM + mi * 8 + g;
-        const int c = j0 + wn * C::TN + ni * 8 + 2 * t4;
-        const double ex = __ldcg(X + (size_t)r * ld + c), ey = __ldcg(X + (size_t)r * ld + c + 1);
-        const double v0 = alpha * acc[mi][ni][0] + beta * ex;
-        const double v1 = alpha * acc[mi][ni][1] + beta * ey;
-        if (!diag) {
-          *reinterpret_cast<double2*>(out + (size_t)r * ld + c) = make_double2(v0, v1);
-          out[(size_t)c * ld + r] = v0;
-          out[(size_t)(c + 1) * ld + r] = v1;
-        } else {
-          if (r <= c) { out[(size_t)r * ld + c] = v0; out[(size_t)c * ld + r] = v0; }
-          if (r <= c + 1) { out[(size_t)r * ld + c + 1] = v1; out[(size_t)(c + 1) * ld + r] = v1; }
-        }
-      }
-    }
-    // per-part barrier before X_{k+1} is read
-    __syncthreads();
-    if (tid == 0) {
-      __threadfence();
-      atomicAdd(a.bar + part, 1u);
-      const unsigned target = per * (unsigned)(k + 1);
-      bool ok = false;
-      for (uint32_t it = 0; it < kSpinLimit; ++it) {
-        unsigned v;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar + part) : "memory");
-        if (v >= target) { ok = true; break; }
-        if (*(volatile int*)a.err) break;
-        __nanosleep(64);
-      }
-      if (!ok) {
-        atomicExch(a.err, 1);
-        s_bad = 1;
-      }
-      __threadfence();
-    }
-    __syncthreads();
-    if (s_bad) return;
-  }
-}
-
-cudaError_t launch_f64_multistep(const MultiStepArgs& a, cudaStream_t st) {
-  using C = MsCfg;
-  static int max_blocks = -1;
-  if (max_blocks < 0) {
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaFuncSetAttribute(k_f64_multistep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_f64_multistep, C::NT, C::SMEM);
-    max_blocks = sms * per_sm;
-  }
-  if (a.ntiles <= 0) return cudaSuccess;
-  if (a.ntiles > max_blocks) return cudaErrorCooperativeLaunchTooLarge;
-  void* args[] = {(void*)&a};
-  const cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_f64_multistep, dim3(a.ntiles),
-                                                    dim3(C::NT), args, C::SMEM, st);
-  note_launch();
-  return e;
 }
 
 // Tile edge of a single dense FP64 product of padded size np: the solve's measured choice
@@ -613,16 +452,9 @@ static cudaError_t launch_f64_bt(const StepArgs& a, int bt, int ntiles, cudaStre
     auto kern = k_sym_gemm_f64<128, 2, 4>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
     kern<<<ntiles, C::NT, C::SMEM, st>>>(a);
-  } else if (bt == 64) {
+  } else {
     using C = F64Cfg<64, 2, 2>;
     auto kern = k_sym_gemm_f64<64, 2, 2>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
-    kern<<<ntiles, C::NT, C::SMEM, st>>>(a);
-  } else {
-    // 32-edge tiles for small batches: 8 warps of 16 x 8 so that a tile's k loop is
-    // spread over all four schedulers (each element still sums k in the same order)
-    using C = F64Cfg<32, 2, 4>;
-    auto kern = k_sym_gemm_f64<32, 2, 4>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
     kern<<<ntiles, C::NT, C::SMEM, st>>>(a);
   }
@@ -632,16 +464,10 @@ static cudaError_t launch_f64_bt(const StepArgs& a, int bt, int ntiles, cudaStre
 
 cudaError_t launch_sym_gemm_f64(const StepArgs& a0, cudaStream_t st) {
   StepArgs a = a0;
-  a.tiles = nullptr;
   if (a.ld == 0) a.ld = a.np;
   const int bt = f64_tile(a.np);
   const int t = a.np / bt;
   a.ntiles = t * (t + 1) / 2;   // the partial sums the last CTA reduces: one per launched tile
-  return launch_f64_bt(a, bt, a.ntiles, st);
-}
-
-cudaError_t launch_sym_gemm_f64_batched(const StepArgs& a, int bt, cudaStream_t st) {
-  if (!a.tiles || a.ntiles <= 0 || (bt != 32 && bt != 64 && bt != 128)) return cudaErrorInvalidValue;
   return launch_f64_bt(a, bt, a.ntiles, st);
 }
 

@@ -44,6 +44,24 @@ cudaError_t launch_place_core(const long long* hptr, const int* halo, const int*
                               const long long* off, int nparts, const double* src, double* rho,
                               long long n, cudaStream_t st);
 
+// The FP64 batch in one persistent launch (k_f64_parts.cu): tiles {row0, bi << 16 | bj,
+// K extent (a multiple of 16), core} of edge bt over each part's upper blocks.
+struct F64PartsArgs {
+  double* x[2];         // packed ping-pong buffers; x[0] holds X_0
+  const int4* tiles;
+  const int* tpart;     // part of each tile
+  const int* pnt;       // tiles of each part
+  const int* pp;        // branch of each step: 0 = 2X - X^2, else X^2
+  unsigned* done;       // per part, finished tiles over all steps (zero at launch)
+  unsigned* ticket;     // next item (zero at launch)
+  double* partials;     // residual sums, f64_parts_partials() doubles (null: not formed)
+  int* err;
+  int ntiles, nsteps, ld;
+};
+size_t f64_parts_partials(int ntiles, int nsteps, int bt);
+cudaError_t launch_f64_parts(const F64PartsArgs& a, int bt, long long rows, double* vv,
+                             cudaStream_t st);
+
 // Batched INT8 digit-split form (exact INT8 precision of the sub-graph loop): the
 // iterate as four signed 8-bit planes of M = rint(2^31 (X - I/2)) in each packed buffer
 // (plane s at base + s rows ld).  Tiles {row0, bi << 16 | bj64, K extent, core} of

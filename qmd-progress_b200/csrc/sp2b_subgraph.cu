@@ -2,10 +2,11 @@
 // (src/prg_subgraphloop_mod.F90:36-126) as one batched GPU solve.
 //
 // All parts share the branch sequence pp(1:maxIter) and the global bounds
-// (src/prg_subgraphloop_mod.F90:104-106), so every part advances in lock step: one
-// launch per SP2 iteration covers the upper tiles of every part (a ragged batch,
-// largest parts first), and the whole sequence normalise -> maxIter steps -> scatter
-// is captured once into a CUDA graph and replayed as one graph launch.
+// (src/prg_subgraphloop_mod.F90:104-106).  The FP64 and INT8 forms run every step of every
+// part in one persistent launch; the split form launches one kernel per SP2 iteration over
+// the upper tiles of every part (a ragged batch, largest parts first).  The whole sequence
+// normalise -> maxIter steps -> scatter is captured once into a CUDA graph and replayed as
+// one graph launch.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -71,7 +72,7 @@ struct SubBufs {
   __half* hi[2] = {};            size_t hi_cap[2] = {};
   __half* lo[2] = {};            size_t lo_cap[2] = {};
   int8_t* dig[2] = {};           size_t dig_cap[2] = {};   // INT8 digit planes (4 per buffer)
-  int* tpart = nullptr;          size_t tpart_cap = 0;     // INT8: part of each tile
+  int* tpart = nullptr;          size_t tpart_cap = 0;     // FP64, INT8: part of each tile
   double* i8part = nullptr;      size_t i8part_cap = 0;    // INT8: per-step sums
   PartDesc* parts = nullptr;     size_t parts_cap = 0;
   int4* tiles = nullptr;         size_t tiles_cap = 0;
@@ -89,12 +90,10 @@ struct SubBufs {
   int* pp = nullptr;             size_t pp_cap = 0;
   double* vv = nullptr;          size_t vv_cap = 0;
   double* idem = nullptr;        size_t idem_cap = 0;   // per-part core idempotency sums
-  // 32-edge FP64 layouts: the tile list of the one-launch multi-step solve (the INT8
-  // solve uses ms_part_tiles and ms_bar too: tiles per part, finished-tile counters)
-  int4* ms_tiles = nullptr;      size_t ms_tiles_cap = 0;
-  int* ms_part_tiles = nullptr;  size_t ms_part_tiles_cap = 0;
-  unsigned* ms_bar = nullptr;    size_t ms_bar_cap = 0;
-  int ms_ntiles = 0;
+  // persistent solves (FP64, INT8): tiles per part, finished-tile counters (and the FP64
+  // solve's item counter behind them)
+  int* pnt = nullptr;            size_t pnt_cap = 0;
+  unsigned* done = nullptr;      size_t done_cap = 0;
   double* hback = nullptr;       size_t hback_cap = 0;  // pinned: vv, part sums, status
   int* dflag = nullptr;          size_t dflag_cap = 0;  // device: part-list comparison
   // layout of the last call (reused when the part lists are unchanged)
@@ -158,7 +157,7 @@ struct SubJob {
   double* dense;         // device, n x n, or null
   bool clear_dense;      // zero `dense` before the scatter
   bool part_idem;        // split and INT8 only: per-part idempotency sums into b.idem
-  bool multistep;        // FP64 only: all steps in one cooperative launch when it fits
+  bool resolve;        // FP64 only: the re-solve (no per-step sums, no graph)
   // measured launch configuration (-1: the built-in rule).  FP64: the tile edge (32 or 64);
   // split: the order of the tile list (0 largest parts first, 1 balanced over the CTAs)
   int variant = -1;
@@ -186,16 +185,16 @@ static int batched_solve(Ctx* c, SubBufs& b, const SubJob& j, cudaStream_t st,
   // tile edge of the step kernel: 128 split; FP64 64, or 32 when the 64-tiles of all
   // parts would not fill the SMs once (a handful of parts, e.g. the re-solve of flagged
   // ones).  The FP64 sums run in the same k order for every edge, so the results agree
-  // bit for bit.
+  // bit for bit.  FP64 tiles cover the part size rounded up to the edge.
   int bt = 128;
   if (!split && !dig) {
     long long t64 = 0;
     for (int p = 0; p < nparts; ++p) {
-      const long long t = padded((int)(hp[p + 1] - hp[p])) / 64;
+      const long long t = (hp[p + 1] - hp[p] + 63) / 64;
       t64 += t * (t + 1) / 2;
     }
-    bt = (t64 < 148 || j.multistep) ? 32 : 64;
-    if (!j.multistep && (j.variant == 32 || j.variant == 64)) bt = j.variant;
+    bt = t64 < 148 ? 32 : 64;
+    if (j.variant == 32 || j.variant == 64) bt = j.variant;
   }
   const int tile_order = (split && j.variant == 1) ? 1 : 0;
   // (the caller may pass the cached lists themselves, which then need no comparison)
@@ -271,6 +270,13 @@ static int batched_solve(Ctx* c, SubBufs& b, const SubJob& j, cudaStream_t st,
             tiles.push_back(make_int4((int)P[p].row0, (bi << 16) | bj, n64, P[p].ncore));
         continue;
       }
+      if (!split) {
+        const int T = (P[p].n + bt - 1) / bt, kext = (P[p].n + 15) / 16 * 16;
+        for (int bj = 0; bj < T; ++bj)
+          for (int bi = 0; bi <= bj; ++bi)
+            tiles.push_back(make_int4((int)P[p].row0, (bi << 16) | bj, kext, P[p].ncore));
+        continue;
+      }
       const int T = P[p].np / bt;
       for (int bj = 0; bj < T; ++bj)
         for (int bi = 0; bi <= bj; ++bi)
@@ -292,34 +298,18 @@ static int batched_solve(Ctx* c, SubBufs& b, const SubJob& j, cudaStream_t st,
       for (int w0 = G; w0 < ntiles; w0 += 2 * G)
         std::reverse(tiles.begin() + w0, tiles.begin() + std::min(ntiles, w0 + G));
     }
-    if (bt == 32) {
-      // the multi-step launch: one CTA per tile, the part index in place of the core count
-      std::vector<int4> ms;
-      std::vector<int> per(nparts, 0);
-      for (const int4& t : tiles) {
-        const int p = row_part[t.x];
-        ms.push_back(make_int4(t.x, t.y, t.z, p));
-        ++per[p];
-      }
-      SP2B_CUDA_TRY(grow_buf(b.ms_tiles, b.ms_tiles_cap, ms.size()));
-      SP2B_CUDA_TRY(grow_buf(b.ms_part_tiles, b.ms_part_tiles_cap, (size_t)nparts));
-      SP2B_CUDA_TRY(grow_buf(b.ms_bar, b.ms_bar_cap, (size_t)nparts));
-      SP2B_CUDA_TRY(cudaMemcpyAsync(b.ms_tiles, ms.data(), ms.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
-      SP2B_CUDA_TRY(cudaMemcpyAsync(b.ms_part_tiles, per.data(), nparts * sizeof(int), cudaMemcpyHostToDevice, st));
-      b.ms_ntiles = (int)ms.size();
-    }
-    if (dig) {
-      // the persistent INT8 solve orders a part's steps by counting its finished tiles
+    if (!split) {
+      // the persistent solves order a part's steps by counting its finished tiles
       std::vector<int> tp(ntiles), per(nparts, 0);
       for (int t = 0; t < ntiles; ++t) {
         tp[t] = row_part[tiles[t].x];
         ++per[tp[t]];
       }
       SP2B_CUDA_TRY(grow_buf(b.tpart, b.tpart_cap, (size_t)ntiles));
-      SP2B_CUDA_TRY(grow_buf(b.ms_part_tiles, b.ms_part_tiles_cap, (size_t)nparts));
-      SP2B_CUDA_TRY(grow_buf(b.ms_bar, b.ms_bar_cap, (size_t)nparts));
+      SP2B_CUDA_TRY(grow_buf(b.pnt, b.pnt_cap, (size_t)nparts));
+      SP2B_CUDA_TRY(grow_buf(b.done, b.done_cap, (size_t)nparts + 1));
       SP2B_CUDA_TRY(cudaMemcpyAsync(b.tpart, tp.data(), ntiles * sizeof(int), cudaMemcpyHostToDevice, st));
-      SP2B_CUDA_TRY(cudaMemcpyAsync(b.ms_part_tiles, per.data(), nparts * sizeof(int), cudaMemcpyHostToDevice, st));
+      SP2B_CUDA_TRY(cudaMemcpyAsync(b.pnt, per.data(), nparts * sizeof(int), cudaMemcpyHostToDevice, st));
       SP2B_CUDA_TRY(cudaStreamSynchronize(st));
     }
     SP2B_CUDA_TRY(grow_buf(b.parts, b.parts_cap, nparts));
@@ -370,7 +360,27 @@ static int batched_solve(Ctx* c, SubBufs& b, const SubJob& j, cudaStream_t st,
   }
   const bool idem = (split || dig) && j.part_idem;
   if (idem) SP2B_CUDA_TRY(grow_buf(b.idem, b.idem_cap, (size_t)nparts * kPartIdemGroups));
-  SP2B_CUDA_TRY(grow_buf(b.partials, b.partials_cap, 4 * (size_t)ntiles));
+  const bool f64 = !split && !dig;
+  // the item counter and the partial sums of the FP64 solve (none for a re-solve)
+  if (split) SP2B_CUDA_TRY(grow_buf(b.partials, b.partials_cap, 4 * (size_t)ntiles));
+  else if (f64 && !j.resolve)
+    SP2B_CUDA_TRY(grow_buf(b.partials, b.partials_cap, f64_parts_partials(ntiles, maxiter, bt)));
+  F64PartsArgs fa;
+  memset(&fa, 0, sizeof(fa));
+  if (f64) {
+    fa.x[0] = b.xs;
+    fa.x[1] = b.x2;
+    fa.tiles = b.tiles;
+    fa.tpart = b.tpart;
+    fa.pnt = b.pnt;
+    fa.done = b.done;
+    fa.ticket = b.done + nparts;
+    fa.partials = j.resolve ? nullptr : b.partials;
+    fa.err = c->err;
+    fa.ntiles = ntiles;
+    fa.nsteps = maxiter;
+    fa.ld = ld;
+  }
   SP2B_CUDA_TRY(grow_buf(b.rec, b.rec_cap, (size_t)maxiter + 2));
   SP2B_CUDA_TRY(grow_buf(b.pp, b.pp_cap, (size_t)maxiter + 1));
   SP2B_CUDA_TRY(grow_buf(b.vv, b.vv_cap, (size_t)maxiter + 1));
@@ -384,10 +394,10 @@ static int batched_solve(Ctx* c, SubBufs& b, const SubJob& j, cudaStream_t st,
   double* core_d = j.core;
   double* dense_d = j.dense;
 
-  // ---- a few FP64 parts: every step in one cooperative launch ----
-  if (j.multistep && !split && !dig && bt == 32 && maxiter > 0) {
+  // ---- the FP64 re-solve of flagged parts (another set each call): no graph ----
+  if (j.resolve && f64 && maxiter > 0) {
     SP2B_CUDA_TRY(cudaMemsetAsync(c->err, 0, sizeof(int), st));
-    SP2B_CUDA_TRY(cudaMemsetAsync(b.ms_bar, 0, nparts * sizeof(unsigned), st));
+    SP2B_CUDA_TRY(cudaMemsetAsync(b.done, 0, (nparts + 1) * sizeof(unsigned), st));
     if (dense_d && j.clear_dense)
       SP2B_CUDA_TRY(cudaMemsetAsync(dense_d, 0, (size_t)n * n * sizeof(double), st));
     if (fused) {
@@ -401,38 +411,25 @@ static int batched_solve(Ctx* c, SubBufs& b, const SubJob& j, cudaStream_t st,
       SP2B_CUDA_TRY(launch_norm_parts(b.xs, b.row_part, b.parts, rows, ld, j.mineval, j.maxeval,
                                       prec, nullptr, nullptr, st));
     }
-    MultiStepArgs ma;
-    ma.x[0] = b.xs;
-    ma.x[1] = b.x2;
-    ma.tiles = b.ms_tiles;
-    ma.ntiles = b.ms_ntiles;
-    ma.part_tiles = b.ms_part_tiles;
-    ma.pp = b.pp;
-    ma.maxiter = maxiter;
-    ma.ld = ld;
-    ma.bar = b.ms_bar;
-    ma.err = c->err;
-    const cudaError_t me = launch_f64_multistep(ma, st);
-    if (me == cudaSuccess) {
-      SP2B_CUDA_TRY(launch_scatter_parts((maxiter & 1) ? b.x2 : b.xs, nullptr, nullptr, prec,
-                                         b.parts, nparts, b.halo, ld, core_d, dense_d, n, st));
-      SP2B_CUDA_TRY(grow_pinned(b.hback, b.hback_cap, 1));
-      SP2B_CUDA_TRY(cudaMemcpyAsync(b.hback, c->err, sizeof(int), cudaMemcpyDeviceToHost, st));
-      SP2B_CUDA_TRY(cudaStreamSynchronize(st));
-      int herr = 0;
-      memcpy(&herr, b.hback, sizeof(int));
-      if (herr) {
-        set_last_error("a device-side wait timed out");
-        return SP2B_TIMEOUT;
-      }
-      vvh.assign(maxiter + 1, 0.0);   // the one-launch form forms no per-step sums
-      return SP2B_OK;
-    }
-    if (me != cudaErrorCooperativeLaunchTooLarge) {
-      set_last_error("multi-step launch failed: %s", cudaGetErrorString(me));
+    fa.pp = b.pp;
+    const cudaError_t me = launch_f64_parts(fa, bt, rows, nullptr, st);
+    if (me != cudaSuccess) {
+      set_last_error("FP64 sub-graph launch failed: %s", cudaGetErrorString(me));
       return SP2B_CUDA_ERROR;
     }
-    (void)cudaGetLastError();   // too many tiles to be resident at once: per-step launches
+    SP2B_CUDA_TRY(launch_scatter_parts((maxiter & 1) ? b.x2 : b.xs, nullptr, nullptr, prec,
+                                       b.parts, nparts, b.halo, ld, core_d, dense_d, n, st));
+    SP2B_CUDA_TRY(grow_pinned(b.hback, b.hback_cap, 1));
+    SP2B_CUDA_TRY(cudaMemcpyAsync(b.hback, c->err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    SP2B_CUDA_TRY(cudaStreamSynchronize(st));
+    int herr = 0;
+    memcpy(&herr, b.hback, sizeof(int));
+    if (herr) {
+      set_last_error("a device-side wait timed out");
+      return SP2B_TIMEOUT;
+    }
+    vvh.assign(maxiter + 1, 0.0);   // the re-solve forms no per-step sums
+    return SP2B_OK;
   }
 
   // ---- the batched solve, captured once into a graph ----
@@ -468,8 +465,8 @@ static int batched_solve(Ctx* c, SubBufs& b, const SubJob& j, cudaStream_t st,
                           dig ? (const void*)b.dig[0] : b.hi[0], dig ? (const void*)b.dig[1] : b.hi[1],
                           b.lo[0], b.lo[1], b.parts, b.tiles, b.row_part, b.halo, b.skey,
                           b.sval, b.partials, b.rec, b.pp, (const void*)cap,
-                          idem ? b.idem : nullptr, dig ? b.tpart : nullptr,
-                          dig ? b.ms_bar : nullptr, dig ? b.i8part : nullptr};
+                          idem ? b.idem : nullptr, b.tpart, b.done,
+                          dig ? (const void*)b.i8part : b.pnt};
   memcpy(key.p, ptrs, sizeof(ptrs));
   const long long qs[10] = {n, nparts, rows, ld, maxiter, prec, ntiles, (long long)(size_t)b.vv,
                             j.clear_dense ? 1 : 0, bt};
@@ -536,7 +533,7 @@ static int batched_solve(Ctx* c, SubBufs& b, const SubJob& j, cudaStream_t st,
       }
       if (dig && maxiter > 0) {
         // every step in one persistent launch
-        if ((e = cudaMemsetAsync(b.ms_bar, 0, nparts * sizeof(unsigned), cap)) != cudaSuccess)
+        if ((e = cudaMemsetAsync(b.done, 0, nparts * sizeof(unsigned), cap)) != cudaSuccess)
           return e;
         if ((e = cudaMemsetAsync(b.i8part, 0, i8_steps_partials(maxiter) * sizeof(double), cap)) !=
             cudaSuccess)
@@ -544,9 +541,9 @@ static int batched_solve(Ctx* c, SubBufs& b, const SubJob& j, cudaStream_t st,
         I8StepsArgs ia;
         ia.tiles = b.tiles;
         ia.tpart = b.tpart;
-        ia.pnt = b.ms_part_tiles;
+        ia.pnt = b.pnt;
         ia.pp = b.pp;
-        ia.done = b.ms_bar;
+        ia.done = b.done;
         ia.partials = b.i8part;
         ia.err = c->err;
         ia.ntiles = ntiles;
@@ -554,22 +551,20 @@ static int batched_solve(Ctx* c, SubBufs& b, const SubJob& j, cudaStream_t st,
         ia.rows = (int)rows;
         if ((e = launch_i8_steps(ia, b.dig[0], b.dig[1], ld, b.vv, cap)) != cudaSuccess) return e;
       }
-      for (int k = 0; k < maxiter && !dig; ++k) {
+      if (f64 && maxiter > 0) {
+        if ((e = cudaMemsetAsync(b.done, 0, (nparts + 1) * sizeof(unsigned), cap)) != cudaSuccess)
+          return e;
+        fa.pp = b.pp;
+        if ((e = launch_f64_parts(fa, bt, rows, b.vv, cap)) != cudaSuccess) return e;
+      }
+      for (int k = 0; k < maxiter && split; ++k) {
         a.k = k;
         const int bin = k & 1, bout = (k + 1) & 1;
-        if (split) {
-          a.A = a.B = a.E = b.hi[bin];
-          a.A_lo = a.B_lo = a.E_lo = b.lo[bin];
-          a.out = b.hi[bout];
-          a.out_lo = b.lo[bout];
-          e = launch_sym_gemm_tc_batched(a, rows, prec == SP2B_PREC_MIXED_BF16, cap);
-        } else {
-          double* xin = bin ? b.x2 : b.xs;
-          double* xout = bout ? b.x2 : b.xs;
-          a.A = a.B = a.E = xin;
-          a.out = xout;
-          e = launch_sym_gemm_f64_batched(a, bt, cap);
-        }
+        a.A = a.B = a.E = b.hi[bin];
+        a.A_lo = a.B_lo = a.E_lo = b.lo[bin];
+        a.out = b.hi[bout];
+        a.out_lo = b.lo[bout];
+        e = launch_sym_gemm_tc_batched(a, rows, prec == SP2B_PREC_MIXED_BF16, cap);
         if (e != cudaSuccess) return e;
       }
       const int fb = maxiter & 1;
@@ -607,8 +602,8 @@ static int batched_solve(Ctx* c, SubBufs& b, const SubJob& j, cudaStream_t st,
     b.exec_key = kbytes;
   }
   cudaError_t le = cudaGraphLaunch(exec, st);
-  // extract, normalise, the steps (INT8: one persistent launch and its sums), scatter
-  note_launch((dig ? (fused ? 1 : 2) + (maxiter > 0 ? 2 : 0) + 1 : maxiter + 3) + (idem ? 1 : 0));
+  // extract, normalise, the steps (FP64, INT8: one persistent launch and its sums), scatter
+  note_launch((split ? maxiter : maxiter > 0 ? 2 : 0) + (fused ? 1 : 2) + 1 + (idem ? 1 : 0));
   if (le != cudaSuccess) {
     set_last_error("graph launch failed: %s", cudaGetErrorString(le));
     return SP2B_CUDA_ERROR;
@@ -644,7 +639,7 @@ static int batched_solve(Ctx* c, SubBufs& b, const SubJob& j, cudaStream_t st,
 // whole solves of this job; sets j.variant.
 static int tune_subgraph(Ctx* c, SubBufs& b, SubJob& j, cudaStream_t st) {
   j.variant = -1;
-  if (!tune_enabled() || j.multistep || j.prec == SP2B_PREC_EXACT_INT8) return SP2B_OK;
+  if (!tune_enabled() || j.resolve || j.prec == SP2B_PREC_EXACT_INT8) return SP2B_OK;
   const bool split = j.prec != SP2B_PREC_FP64;
   const std::vector<long long>& hp = *j.hp;
   std::map<int, int> hist;
