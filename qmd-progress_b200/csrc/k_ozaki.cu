@@ -68,8 +68,9 @@ constexpr int TMEM_COLS = 2 * BN;
 // (as the bits of a non-negative double, for atomicMax) and the chosen exponent S.
 struct OzScale {
   unsigned long long r2max_bits;
+  unsigned long long next_bits;   // running maximum of k_oz_rowmax (zero between launches)
   int S;      // -1: no valid scale (non-finite input)
-  int pad;
+  unsigned counter;               // CTAs of k_oz_rowmax that have arrived
 };
 
 // SP2-step context of the launches that compute one step's X^2 (the exact INT8 mode):
@@ -160,8 +161,7 @@ __global__ void k_oz_rownorm_f64(const double* __restrict__ x, int np, OzScale* 
 
 // S: the largest exponent with (2^S sqrt(r2max) + sqrt(np)/2)^2 < prod/2, which bounds
 // every |(M M)_ij| (row norms of M are at most 2^S ||x_i|| + sqrt(np)/2).
-__global__ void k_oz_scale(OzScale* sc, int np) {
-  const double r2 = __longlong_as_double((long long)sc->r2max_bits);
+__device__ __forceinline__ int oz_choose_scale(double r2, int np) {
   int S = -1;
   if (r2 == r2 && r2 < 1e300) {
     const double lim = sqrt(oz::half_prod()) * (1.0 - 1e-12);
@@ -174,75 +174,92 @@ __global__ void k_oz_scale(OzScale* sc, int np) {
       while (S > -1 && ldexp(r, S) + e >= lim) --S;
     }
   }
-  sc->S = S;
+  return S;
+}
+__global__ void k_oz_scale(OzScale* sc, int np) {
+  sc->S = oz_choose_scale(__longlong_as_double((long long)sc->r2max_bits), np);
 }
 
 // ---------------------------------------------------------------------------------
 // 2. Residue planes: R_t = rint(2^S X) mod m_t in the symmetric range (signed 8-bit).
 //    Plane t is np x np at res + t * np * np.
 // ---------------------------------------------------------------------------------
-// A residue of M = mh 2^21 + ml modulo m, any representative with |r| <= 127 (the
-// products only need r = M mod m and |r| <= 128).  v = mh (2^21 mod m) + ml is an integer
-// below 2^24 in magnitude, exact in FP32; q = rint(v / m) is off the nearest integer by at
-// most one ulp of v/m, so r = v - q m is exact and |r| <= m/2 + 0.005 m.
+// M = rint(x 2^S), |M| < sqrt(prod/2) < 2^36, as the low mantissa bits of x 2^S + 1.5 2^52 (one
+// FMA rounds to nearest even, like rint): no FP64 conversion or floor instruction.  It is
+// split as M = mh 2^21 + ml (0 <= ml < 2^21, |mh| < 2^15), both exact in FP32.
+struct OzInt {
+  float mh, ml;
+  uint32_t low;   // M mod 2^32
+};
+__device__ __forceinline__ OzInt oz_round(double x, double scale) {
+  const double t = fma(x, scale, 0x1.8p52);
+  const uint32_t lo = (uint32_t)__double2loint(t);
+  const int hi = __double2hiint(t) - 0x43380000;
+  const int mh = (int)__funnelshift_l(lo, (uint32_t)hi, 11);
+  OzInt r;
+  r.mh = __int_as_float(0x4b400000 + mh) - 0x1.8p23f;
+  r.ml = __int_as_float(0x4b000000 | (int)(lo & 0x1fffffu)) - 0x1p23f;
+  r.low = lo;
+  return r;
+}
+// A residue of M modulo m, any representative in [-128, 127] (the products only need
+// r = M mod m).  v = mh c + ml, c = 2^21 mod m in the symmetric range, is an integer below
+// 2^23 in magnitude, exact in FP32; q = v / m to the nearest integer (the FMA rounds
+// v inv + 1.5 2^23 once, so q errs only within 0.001 of a tie, where either neighbour's
+// residue is below 128 in magnitude), and r = v - q m is exact.  The result is the low byte
+// of r + 1.5 2^23: five full-rate FP32 instructions and no conversion.
 template <int t>
-__device__ __forceinline__ int8_t oz_residue(float mhf, float mlf, int ml) {
+__device__ __forceinline__ uint32_t oz_residue(const OzInt& M) {
   constexpr int m = oz::mod(t);
   if constexpr (m == 256) {
-    return (int8_t)(uint8_t)(ml & 255);
+    return M.low;
   } else {
-    constexpr float c = (float)oz::pow2_mod(21, m);
-    constexpr float inv = 1.0f / (float)m;
-    const float v = fmaf(mhf, c, mlf);
-    const float q = rintf(v * inv);
-    return (int8_t)__float2int_rn(fmaf(-q, (float)m, v));
+    constexpr int c0 = oz::pow2_mod(21, m);
+    constexpr float c = (float)(c0 > m / 2 ? c0 - m : c0), inv = 1.0f / (float)m;
+    const float v = fmaf(M.mh, c, M.ml);
+    const float q = fmaf(v, inv, 0x1.8p23f) - 0x1.8p23f;
+    return (uint32_t)__float_as_int(fmaf(-q, (float)m, v) + 0x1.8p23f);
   }
 }
+__device__ __forceinline__ uint32_t low_bytes(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  return __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
+}
 
+// Eight consecutive elements of every plane from plane offset off.
 template <int t>
 __device__ __forceinline__ void oz_store_planes(int8_t* res, size_t plane, size_t off,
-                                                const float (&mh)[16], const float (&mlf)[16],
-                                                const int (&ml)[16]) {
+                                                const OzInt (&M)[8]) {
   if constexpr (t < oz::T) {
-    alignas(16) int8_t v[16];
-#pragma unroll
-    for (int q = 0; q < 16; ++q) v[q] = oz_residue<t>(mh[q], mlf[q], ml[q]);
-    *reinterpret_cast<uint4*>(res + (size_t)t * plane + off) = *reinterpret_cast<const uint4*>(v);
-    oz_store_planes<t + 1>(res, plane, off, mh, mlf, ml);
+    uint2 v;
+    v.x = low_bytes(oz_residue<t>(M[0]), oz_residue<t>(M[1]), oz_residue<t>(M[2]), oz_residue<t>(M[3]));
+    v.y = low_bytes(oz_residue<t>(M[4]), oz_residue<t>(M[5]), oz_residue<t>(M[6]), oz_residue<t>(M[7]));
+    *reinterpret_cast<uint2*>(res + (size_t)t * plane + off) = v;
+    oz_store_planes<t + 1>(res, plane, off, M);
   }
 }
 
+// Bound by HBM and FP32 issue (8 moduli x 5.75 instructions an element).
 template <typename T>
 __global__ void k_oz_residues(const T* __restrict__ hi, const T* __restrict__ lo, int np,
                               const OzScale* __restrict__ sc, int8_t* __restrict__ res) {
   using SP = OzSplit<T>;
   const int S = sc->S;
-  const double scale = ldexp(1.0, S < 0 ? 0 : S);
+  const double scale = S < 0 ? 0.0 : ldexp(1.0, S);   // no valid scale: planes of zeros
   const size_t plane = (size_t)np * np;
-  const size_t groups = plane / 16;
+  const size_t groups = plane / 8;
   for (size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x; g < groups;
        g += (size_t)gridDim.x * blockDim.x) {
-    const size_t off = g * 16;
-    alignas(16) T hv[16], lv[16];
-    reinterpret_cast<uint4*>(hv)[0] = reinterpret_cast<const uint4*>(hi + off)[0];
-    reinterpret_cast<uint4*>(hv)[1] = reinterpret_cast<const uint4*>(hi + off)[1];
-    reinterpret_cast<uint4*>(lv)[0] = reinterpret_cast<const uint4*>(lo + off)[0];
-    reinterpret_cast<uint4*>(lv)[1] = reinterpret_cast<const uint4*>(lo + off)[1];
-    float mh[16], mlf[16];
-    int ml[16];
+    const size_t off = g * 8;
+    alignas(16) T hv[8], lv[8];
+    *reinterpret_cast<uint4*>(hv) = *reinterpret_cast<const uint4*>(hi + off);
+    *reinterpret_cast<uint4*>(lv) = *reinterpret_cast<const uint4*>(lo + off);
+    OzInt M[8];
 #pragma unroll
-    for (int q = 0; q < 16; ++q) {
-      // |x| <= sqrt(r2max), so |M| < sqrt(prod/2) < 2^36: exact in FP64, and the split
-      // M = mh 2^21 + ml (0 <= ml < 2^21, |mh| < 2^15) is exact in FP32 and int32.
+    for (int q = 0; q < 8; ++q) {
       const double x = fma(SP::kInv, SP::d(lv[q]), SP::d(hv[q]));
-      const double M = S < 0 ? 0.0 : rint(x * scale);
-      const double h = floor(M * 0x1p-21);
-      const double l = M - h * 0x1p21;
-      mh[q] = (float)h;
-      mlf[q] = (float)l;
-      ml[q] = (int)l;
+      M[q] = oz_round(S < 0 ? 0.0 : x, scale);
     }
-    oz_store_planes<0>(res, plane, off, mh, mlf, ml);
+    oz_store_planes<0>(res, plane, off, M);
   }
 }
 
@@ -251,29 +268,21 @@ __global__ void k_oz_residues_f64(const double* __restrict__ x, int np,
                                   const OzStepCtl c) {
   if (oz_skip(c)) return;
   const int S = sc->S;
-  const double scale = ldexp(1.0, S < 0 ? 0 : S);
+  const double scale = S < 0 ? 0.0 : ldexp(1.0, S);
   const size_t plane = (size_t)np * np;
-  const size_t groups = plane / 16;
+  const size_t groups = plane / 8;
   for (size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x; g < groups;
        g += (size_t)gridDim.x * blockDim.x) {
-    const size_t off = g * 16;
+    const size_t off = g * 8;
     const double2* src = reinterpret_cast<const double2*>(x + off);
-    float mh[16], mlf[16];
-    int ml[16];
+    OzInt M[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
+    for (int q = 0; q < 4; ++q) {
       const double2 v = src[q];
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const double M = S < 0 ? 0.0 : rint((e ? v.y : v.x) * scale);
-        const double h = floor(M * 0x1p-21);
-        const double l = M - h * 0x1p21;
-        mh[2 * q + e] = (float)h;
-        mlf[2 * q + e] = (float)l;
-        ml[2 * q + e] = (int)l;
-      }
+      M[2 * q] = oz_round(S < 0 ? 0.0 : v.x, scale);
+      M[2 * q + 1] = oz_round(S < 0 ? 0.0 : v.y, scale);
     }
-    oz_store_planes<0>(res, plane, off, mh, mlf, ml);
+    oz_store_planes<0>(res, plane, off, M);
   }
 }
 
@@ -459,67 +468,69 @@ __global__ void __launch_bounds__(oz::NTHR, 1)
 //    of the upper tiles.  One CTA per upper 32 x 32 block pair; the mirror goes through
 //    shared memory so both halves are stored row-contiguous.
 // ---------------------------------------------------------------------------------
-// Pairwise (tree) Chinese remaindering: residues modulo m_a, m_b combine into the residue
-// modulo m_a m_b as x = x_a + m_a ((x_b - x_a) m_a^-1 mod m_b).  Eight odd moduli pair up
-// to four 16-bit moduli, then two 32-bit ones, then one 64-bit modulus M07; the last
-// modulus 256 gives the top digit, whose top bit is the sign (Y >= prod/2).
-__host__ __device__ constexpr uint64_t inv_mod64(uint64_t a, uint64_t m) {
-  int64_t t = 0, nt = 1;
-  int64_t r = (int64_t)m, nr = (int64_t)(a % m);
-  while (nr != 0) {
-    const int64_t q = r / nr;
-    int64_t tmp = t - q * nt;
-    t = nt;
-    nt = tmp;
-    tmp = r - q * nr;
-    r = nr;
-    nr = tmp;
-  }
-  return (uint64_t)(t < 0 ? t + (int64_t)m : t);
-}
+// Chinese remaindering in FP64: with W_t the integer that is 1 modulo m_t and 0 modulo the
+// others, Y = sum_t q_t W_t - n P, P = prod(m_t) < 2^71.4, n the nearest integer to the sum
+// over P.  W_t and P are cut at 2^31 into two integers below 2^40.5 and 2^31, so that both
+// partial sums (9 terms, q_t < 256) and both n multiples stay below 2^53: every operation
+// but the last, which joins the two parts, is exact, and Y is the correctly rounded double.
+// 30 FP64 instructions, against the chain of 16-, 32- and 64-bit modular reductions of a
+// pairwise tree.
 namespace ozc {
-constexpr uint32_t M01 = 255u * 253u, M23 = 251u * 247u, M45 = 241u * 239u, M67 = 233u * 229u;
-constexpr uint64_t M0123 = (uint64_t)M01 * M23, M4567 = (uint64_t)M45 * M67;
-constexpr uint64_t M07 = M0123 * M4567;   // < 2^64
-constexpr uint32_t I01 = (uint32_t)inv_mod64(255, 253), I23 = (uint32_t)inv_mod64(251, 247);
-constexpr uint32_t I45 = (uint32_t)inv_mod64(241, 239), I67 = (uint32_t)inv_mod64(233, 229);
-constexpr uint32_t I0123 = (uint32_t)inv_mod64(M01 % M23, M23);
-constexpr uint32_t I4567 = (uint32_t)inv_mod64(M45 % M67, M67);
-constexpr uint64_t I07 = inv_mod64(M0123 % M4567, M4567);
-constexpr uint32_t I8 = (uint32_t)inv_mod64(M07 % 256u, 256u);
+typedef unsigned __int128 u128;
+__host__ __device__ constexpr u128 prod() {
+  u128 p = 1;
+  for (int t = 0; t < oz::T; ++t) p *= (u128)oz::mod(t);
+  return p;
+}
+__host__ __device__ constexpr u128 weight(int t) {
+  const u128 r = prod() / (u128)oz::mod(t);
+  return r * (u128)oz::inv_mod((int)(r % (u128)oz::mod(t)), oz::mod(t));
+}
+__host__ __device__ constexpr double upper(u128 v) { return (double)(uint64_t)(v >> 31); }
+__host__ __device__ constexpr double lower(u128 v) { return (double)(uint64_t)(v & 0x7fffffffu); }
 }  // namespace ozc
 
-// x_a in [0, ma), x_b in [0, mb) (ma < 2 mb) -> x in [0, ma mb); 16-bit moduli
-template <uint32_t ma, uint32_t mb, uint32_t ia>
-__device__ __forceinline__ uint32_t crt_pair16(uint32_t xa, uint32_t xb) {
-  const uint32_t t = (xb + 2u * mb - (xa % mb)) % mb;
-  return xa + ma * ((t * ia) % mb);
+template <int t>
+__device__ __forceinline__ void crt_sums(const uint32_t (&q)[oz::T], double& s1, double& s2) {
+  if constexpr (t < oz::T) {
+    constexpr double w1 = ozc::upper(ozc::weight(t)), w2 = ozc::lower(ozc::weight(t));
+    const double d = __hiloint2double(0x43300000, (int)q[t]) - 0x1p52;   // q_t
+    s1 = fma(d, w1, s1);
+    s2 = fma(d, w2, s2);
+    crt_sums<t + 1>(q, s1, s2);
+  }
 }
-// 32-bit level: moduli below 2^16, products below 2^32
-template <uint32_t ma, uint32_t mb, uint32_t ia>
-__device__ __forceinline__ uint32_t crt_pair32(uint32_t xa, uint32_t xb) {
-  const uint32_t xam = xa >= mb ? xa - mb : xa;   // xa < ma < 2 mb
-  const uint32_t t = xb >= xam ? xb - xam : xb + mb - xam;
-  return xa + ma * ((t * ia) % mb);
+// Residues (q_t in [0, m_t)) -> the symmetric integer Y, |Y| < prod/2 (1 - 1e-12).
+__device__ __forceinline__ double crt_value(const uint32_t (&q)[oz::T]) {
+  constexpr double p1 = ozc::upper(ozc::prod()), p2 = ozc::lower(ozc::prod());
+  constexpr double p = p1 * 0x1p31 + p2, half = 0.5 * p;
+  double s1 = 0.0, s2 = 0.0;
+  crt_sums<0>(q, s1, s2);
+  const double n = fma(s1, 0x1p31 / p, 0x1.8p52) - 0x1.8p52;
+  double d1 = fma(-n, p1, s1), d2 = fma(-n, p2, s2);
+  double y = fma(d1, 0x1p31, d2);
+  // n left out the lower sums (2^-29 of a unit): one unit off near a tie
+  if (fabs(y) > half) {
+    const double sgn = y > 0.0 ? 1.0 : -1.0;
+    d1 = fma(-sgn, p1, d1);
+    d2 = fma(-sgn, p2, d2);
+    y = fma(d1, 0x1p31, d2);
+  }
+  return y;
 }
-// Residues (in [0, m_t)) -> the symmetric integer Y, |Y| < prod/2, as a double
-// (exact below 2^53 in magnitude, one rounding above).
-__device__ __forceinline__ double crt_value(const int (&q)[oz::T]) {
-  using namespace ozc;
-  const uint32_t x01 = crt_pair16<255u, 253u, I01>((uint32_t)q[0], (uint32_t)q[1]);
-  const uint32_t x23 = crt_pair16<251u, 247u, I23>((uint32_t)q[2], (uint32_t)q[3]);
-  const uint32_t x45 = crt_pair16<241u, 239u, I45>((uint32_t)q[4], (uint32_t)q[5]);
-  const uint32_t x67 = crt_pair16<233u, 229u, I67>((uint32_t)q[6], (uint32_t)q[7]);
-  const uint32_t x0123 = crt_pair32<M01, M23, I0123>(x01, x23);
-  const uint32_t x4567 = crt_pair32<M45, M67, I4567>(x45, x67);
-  const uint64_t xam = x0123 >= M4567 ? (uint64_t)x0123 - M4567 : (uint64_t)x0123;
-  const uint64_t t = x4567 >= xam ? x4567 - xam : (uint64_t)x4567 + M4567 - xam;
-  const uint64_t x07 = (uint64_t)x0123 + M0123 * ((t * I07) % M4567);
-  const uint32_t v8 = (((uint32_t)q[8] - (uint32_t)x07) * I8) & 255u;
-  if (v8 == 0) return (double)x07;
-  if (v8 == 255) return -(double)(M07 - x07);
-  const double m07 = (double)M07;
-  return (double)x07 + m07 * (double)(v8 >= 128 ? (int)v8 - 256 : (int)v8);
+// Four consecutive elements of every plane, as the squares' values.
+__device__ __forceinline__ void crt_load4(const uint8_t* __restrict__ q, size_t plane, size_t e,
+                                          double down, double (&x2)[4]) {
+  uint32_t w[oz::T];
+#pragma unroll
+  for (int t = 0; t < oz::T; ++t) w[t] = *reinterpret_cast<const uint32_t*>(q + (size_t)t * plane + e);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    uint32_t v[oz::T];
+#pragma unroll
+    for (int t = 0; t < oz::T; ++t) v[t] = (w[t] >> (8 * j)) & 255u;
+    x2[j] = crt_value(v) * down;
+  }
 }
 
 template <typename T>
@@ -532,40 +543,47 @@ __global__ void __launch_bounds__(256)
   __shared__ T s_rh[32][34], s_rl[32][34];
   int ib, jb;
   upper_tile(blockIdx.x, ib, jb);
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int row = threadIdx.x >> 3, c4 = (threadIdx.x & 7) * 4;   // a thread's four columns
   const int S = sc->S;
   const double down = S < 0 ? __longlong_as_double(0x7ff8000000000000ll) : ldexp(1.0, -2 * S);
   const size_t plane = (size_t)np * np;
+  struct alignas(8) T4 { T v[4]; };
+  {
+    const size_t e = (size_t)(ib * 32 + row) * np + jb * 32 + c4;
+    double x2[4];
+    crt_load4(q, plane, e, down, x2);
+    const T4 xh = *reinterpret_cast<const T4*>(xhi + e), xl = *reinterpret_cast<const T4*>(xlo + e);
+    T4 h, l;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int il = ty + 8 * k;
-    const int i = ib * 32 + il, j = jb * 32 + tx;
-    const size_t e = (size_t)i * np + j;
-    int v[oz::T];
-#pragma unroll
-    for (int t = 0; t < oz::T; ++t) v[t] = q[(size_t)t * plane + e];
-    const double x2 = crt_value(v) * down;
-    const double x = fma(SP::kInv, SP::d(xlo[e]), SP::d(xhi[e]));
-    const double r4 = 4.0 * (x2 - x);
-    const T h = SP::from_d(r4);
-    const T l = SP::from_d((r4 - SP::d(h)) * SP::kScale);
-    x2out[e] = x2;
-    rhi[e] = h;
-    rlo[e] = l;
-    s_x2[il][tx] = x2;
-    s_rh[il][tx] = h;
-    s_rl[il][tx] = l;
+    for (int j = 0; j < 4; ++j) {
+      const double x = fma(SP::kInv, SP::d(xl.v[j]), SP::d(xh.v[j]));
+      const double r4 = 4.0 * (x2[j] - x);
+      h.v[j] = SP::from_d(r4);
+      l.v[j] = SP::from_d((r4 - SP::d(h.v[j])) * SP::kScale);
+      s_x2[row][c4 + j] = x2[j];
+      s_rh[row][c4 + j] = h.v[j];
+      s_rl[row][c4 + j] = l.v[j];
+    }
+    double2* o = reinterpret_cast<double2*>(x2out + e);
+    o[0] = make_double2(x2[0], x2[1]);
+    o[1] = make_double2(x2[2], x2[3]);
+    *reinterpret_cast<T4*>(rhi + e) = h;
+    *reinterpret_cast<T4*>(rlo + e) = l;
   }
   if (ib == jb) return;  // diagonal blocks hold both triangles (the product is symmetric)
   __syncthreads();
+  const size_t e = (size_t)(jb * 32 + row) * np + ib * 32 + c4;
+  T4 h, l;
+  double2* o = reinterpret_cast<double2*>(x2out + e);
+  o[0] = make_double2(s_x2[c4][row], s_x2[c4 + 1][row]);
+  o[1] = make_double2(s_x2[c4 + 2][row], s_x2[c4 + 3][row]);
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int jl = ty + 8 * k;
-    const size_t e = (size_t)(jb * 32 + jl) * np + ib * 32 + tx;
-    x2out[e] = s_x2[tx][jl];
-    rhi[e] = s_rh[tx][jl];
-    rlo[e] = s_rl[tx][jl];
+  for (int j = 0; j < 4; ++j) {
+    h.v[j] = s_rh[c4 + j][row];
+    l.v[j] = s_rl[c4 + j][row];
   }
+  *reinterpret_cast<T4*>(rhi + e) = h;
+  *reinterpret_cast<T4*>(rlo + e) = l;
 }
 
 // ---------------------------------------------------------------------------------
@@ -577,7 +595,8 @@ __global__ void __launch_bounds__(256)
 //    squares are equal bit for bit: the integer products are symmetric).
 // ---------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-    k_oz_crt_step(const uint8_t* __restrict__ q, const OzScale* __restrict__ sc, const StepArgs p) {
+    k_oz_crt_step(const uint8_t* __restrict__ q, const OzScale* __restrict__ sc, const StepArgs p,
+                  double* __restrict__ rown) {
   __shared__ double s_v[32][33];
   __shared__ double red[32 * 4];
   __shared__ int s_flag;
@@ -590,46 +609,99 @@ __global__ void __launch_bounds__(256)
   const int S = sc->S;
   const double down = S < 0 ? __longlong_as_double(0x7ff8000000000000ll) : ldexp(1.0, -2 * S);
   const size_t plane = (size_t)np * np;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int row = threadIdx.x >> 3, c4 = (threadIdx.x & 7) * 4;   // a thread's four columns
   const long long nb = np / 32, nblk = nb * (nb + 1) / 2;
   double s[4] = {0.0, 0.0, 0.0, 0.0};
   for (long long bid = blockIdx.x; bid < nblk; bid += gridDim.x) {
     int ib, jb;
     upper_tile((int)bid, ib, jb);
     const double w = ib == jb ? 1.0 : 2.0;
+    const int i = ib * 32 + row;
+    const size_t e = (size_t)i * np + jb * 32 + c4;
+    double x2[4], nx[4];
+    crt_load4(q, plane, e, down, x2);
+    const double2 xa = *reinterpret_cast<const double2*>(X + e);
+    const double2 xb = *reinterpret_cast<const double2*>(X + e + 2);
+    const double x[4] = {xa.x, xa.y, xb.x, xb.y};
+    double rs = 0.0;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int il = ty + 8 * k;
-      const int i = ib * 32 + il, j = jb * 32 + tx;
-      const size_t e = (size_t)i * np + j;
-      int v[oz::T];
-#pragma unroll
-      for (int t = 0; t < oz::T; ++t) v[t] = q[(size_t)t * plane + e];
-      const double x2 = crt_value(v) * down;
-      const double x = X[e];
-      const double nx = fma(a, x2, b * x);
-      const double d = x - x2;
-      s[0] = fma(w * nx, nx, s[0]);
+    for (int j = 0; j < 4; ++j) {
+      nx[j] = fma(a, x2[j], b * x[j]);
+      const double d = x[j] - x2[j];
+      rs = fma(nx[j], nx[j], rs);
       s[2] = fma(w * d, d, s[2]);
-      if (i == j) {
-        s[1] += nx;
-        s[3] += x2;
+      if (i == jb * 32 + c4 + j) {
+        s[1] += nx[j];
+        s[3] += x2[j];
       }
-      Xo[e] = nx;
-      s_v[il][tx] = nx;
+      s_v[row][c4 + j] = nx[j];
     }
+    s[0] = fma(w, rs, s[0]);
+    double2* o = reinterpret_cast<double2*>(Xo + e);
+    o[0] = make_double2(nx[0], nx[1]);
+    o[1] = make_double2(nx[2], nx[3]);
+    // this block's share of ||row i of X_{k+1}||^2 (the next step's scale)
+    rs += __shfl_xor_sync(0xffffffffu, rs, 1);
+    rs += __shfl_xor_sync(0xffffffffu, rs, 2);
+    rs += __shfl_xor_sync(0xffffffffu, rs, 4);
+    if (c4 == 0) rown[(size_t)i * nb + jb] = rs;
     if (ib != jb) {
       __syncthreads();
+      const int r = jb * 32 + row;
+      double v[4];
+      double cs = 0.0;
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int jl = ty + 8 * k;
-        Xo[(size_t)(jb * 32 + jl) * np + ib * 32 + tx] = s_v[tx][jl];
+      for (int j = 0; j < 4; ++j) {
+        v[j] = s_v[c4 + j][row];
+        cs = fma(v[j], v[j], cs);
       }
+      double2* m = reinterpret_cast<double2*>(Xo + (size_t)r * np + ib * 32 + c4);
+      m[0] = make_double2(v[0], v[1]);
+      m[1] = make_double2(v[2], v[3]);
+      cs += __shfl_xor_sync(0xffffffffu, cs, 1);
+      cs += __shfl_xor_sync(0xffffffffu, cs, 2);
+      cs += __shfl_xor_sync(0xffffffffu, cs, 4);
+      if (c4 == 0) rown[(size_t)r * nb + ib] = cs;
     }
     __syncthreads();
   }
   __threadfence();
   publish_and_finalize(p, s, red, &s_flag);
+}
+
+// Scale of X_k from the per-block row sums that k_oz_crt_step left: one warp per row, the
+// last CTA chooses S.  Reads np^2 / 4 bytes where a pass over X reads 8 np^2.
+__global__ void __launch_bounds__(256)
+    k_oz_rowmax(const double* __restrict__ rown, int np, OzScale* sc, unsigned* counter,
+                const OzStepCtl c) {
+  if (oz_skip(c)) return;
+  __shared__ double s_max[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nb = np / 32;
+  double best = 0.0;
+  for (int row = blockIdx.x * 8 + warp; row < np; row += gridDim.x * 8) {
+    double s = 0.0;
+    for (int j = lane; j < nb; j += 32) s += rown[(size_t)row * nb + j];
+    s = warp_sum(s);
+    if (!(s <= best)) best = s;   // a NaN stays
+    if (best != best) break;
+  }
+  if (lane == 0) s_max[warp] = best;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  unsigned long long bits = 0;
+  for (int w = 0; w < 8; ++w) {
+    // NaN is above every finite value as an unsigned bit pattern
+    const double v = s_max[w];
+    const unsigned long long u = v != v ? 0x7ff8000000000000ull : (unsigned long long)__double_as_longlong(v);
+    bits = u > bits ? u : bits;
+  }
+  atomicMax(&sc->next_bits, bits);
+  __threadfence();
+  if (atomicAdd(counter, 1u) != gridDim.x - 1) return;
+  *counter = 0u;
+  __threadfence();
+  sc->r2max_bits = atomicExch(&sc->next_bits, 0ull);
+  sc->S = oz_choose_scale(__longlong_as_double((long long)sc->r2max_bits), np);
 }
 
 // ---------------------------------------------------------------------------------
@@ -675,7 +747,7 @@ cudaError_t launch_oz_planes(const __half* xhi, const __half* xlo, int np, int b
   else
     k_oz_rownorm<__half><<<rgrid, 256, 0, st>>>(xhi, xlo, np, sc);
   k_oz_scale<<<1, 1, 0, st>>>(sc, np);
-  const size_t groups = (size_t)np * np / 16;
+  const size_t groups = (size_t)np * np / 8;
   const int g = (int)std::min<size_t>((groups + 255) / 256, 148 * 16);
   if (bf16)
     k_oz_residues<__nv_bfloat16><<<g, 256, 0, st>>>((const __nv_bfloat16*)xhi,
@@ -725,26 +797,36 @@ cudaError_t launch_oz_crt(const uint8_t* q, const __half* xhi, const __half* xlo
   return cudaGetLastError();
 }
 
-cudaError_t launch_oz_planes_f64(const double* x, int np, void* scale, int8_t* res,
-                                 const OzStepCtl* ctl, cudaStream_t st) {
+// rown: the row sums launch_oz_crt_step left for this x, or null (they are formed from x).
+cudaError_t launch_oz_planes_f64(const double* x, int np, void* scale, const double* rown,
+                                 int8_t* res, const OzStepCtl* ctl, cudaStream_t st) {
   if (np % oz::BM != 0 || np > 65536) return cudaErrorInvalidValue;
   OzScale* sc = (OzScale*)scale;
-  cudaError_t e = cudaMemsetAsync(sc, 0, sizeof(OzScale), st);
-  if (e != cudaSuccess) return e;
   const int rgrid = std::min((np + 7) / 8, 148 * 8);
-  k_oz_rownorm_f64<<<rgrid, 256, 0, st>>>(x, np, sc, *ctl);
-  k_oz_scale<<<1, 1, 0, st>>>(sc, np);
-  const size_t groups = (size_t)np * np / 16;
+  if (rown) {
+    k_oz_rowmax<<<std::min(rgrid, 148), 256, 0, st>>>(rown, np, sc, &sc->counter, *ctl);
+    note_launch(2);
+  } else {
+    cudaError_t e = cudaMemsetAsync(sc, 0, sizeof(OzScale), st);
+    if (e != cudaSuccess) return e;
+    k_oz_rownorm_f64<<<rgrid, 256, 0, st>>>(x, np, sc, *ctl);
+    k_oz_scale<<<1, 1, 0, st>>>(sc, np);
+    note_launch(3);
+  }
+  const size_t groups = (size_t)np * np / 8;
   const int g = (int)std::min<size_t>((groups + 255) / 256, 148 * 16);
   k_oz_residues_f64<<<g, 256, 0, st>>>(x, np, sc, res, *ctl);
-  note_launch(3);
   return cudaGetLastError();
 }
 
-cudaError_t launch_oz_crt_step(const uint8_t* q, const void* scale, const StepArgs& a,
+size_t oz_rown_doubles(int np) { return (size_t)np * (np / 32); }
+
+cudaError_t launch_oz_crt_step(const uint8_t* q, const void* scale, const StepArgs& a, double* rown,
                                cudaStream_t st) {
   if (a.np % 128 != 0) return cudaErrorInvalidValue;
-  k_oz_crt_step<<<148 * 8, 256, 0, st>>>(q, (const OzScale*)scale, a);
+  const long long nb = a.np / 32;
+  const int grid = (int)std::min<long long>(nb * (nb + 1) / 2, 148 * 8);
+  k_oz_crt_step<<<grid, 256, 0, st>>>(q, (const OzScale*)scale, a, rown);
   note_launch();
   return cudaGetLastError();
 }

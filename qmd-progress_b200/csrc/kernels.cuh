@@ -156,9 +156,10 @@ struct OzStepCtl {
 };
 cudaError_t launch_oz_gemm(const int8_t* res, int np, uint8_t* qout, const int2* tiles,
                            int ntiles, int* err, cudaStream_t st, const OzStepCtl* ctl = nullptr);
-cudaError_t launch_oz_planes_f64(const double* x, int np, void* scale, int8_t* res,
-                                 const OzStepCtl* ctl, cudaStream_t st);
-cudaError_t launch_oz_crt_step(const uint8_t* q, const void* scale, const StepArgs& a,
+cudaError_t launch_oz_planes_f64(const double* x, int np, void* scale, const double* rown,
+                                 int8_t* res, const OzStepCtl* ctl, cudaStream_t st);
+size_t oz_rown_doubles(int np);   // per-block row sums of the iterate a step wrote
+cudaError_t launch_oz_crt_step(const uint8_t* q, const void* scale, const StepArgs& a, double* rown,
                                cudaStream_t st);
 cudaError_t launch_oz_crt(const uint8_t* q, const __half* xhi, const __half* xlo, int np,
                           int bf16, const void* scale, double* x2, __half* rhi, __half* rlo,

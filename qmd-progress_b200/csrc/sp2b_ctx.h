@@ -51,6 +51,8 @@ struct Ctx {
   int2* oz_tiles = nullptr;
   int oz_tiles_np = 0, oz_ntiles = 0;
   void* oz_scale = nullptr;
+  double* oz_rown = nullptr;    // exact steps: per-block row sums of the iterate
+  size_t oz_rown_cap = 0;
   int oz_last_S = 0;            // scale exponent of the last INT8 refinement
   double oz_last_r2max = 0.0;   // its largest squared row norm
   int last_launches = 0;            // SP2 step launches of the last dense solve

@@ -270,6 +270,7 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
       return SP2B_BAD_ARG;
     }
     SP2B_CUDA_TRY(c->ensure_oz(np, st));
+    if (exact) SP2B_CUDA_TRY(grow(c->oz_rown, c->oz_rown_cap, oz_rown_doubles(np)));
   }
 
   // ---- input ----
@@ -391,11 +392,12 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
         oc.ctl = a.ctl;
         oc.k = k;
         oc.active = 1;
-        SP2B_CUDA_TRY(launch_oz_planes_f64(c->x64[bin], np, c->oz_scale, c->oz_res, &oc, st));
+        SP2B_CUDA_TRY(launch_oz_planes_f64(c->x64[bin], np, c->oz_scale, k > 0 ? c->oz_rown : nullptr,
+                                           c->oz_res, &oc, st));
         SP2B_CUDA_TRY(launch_oz_gemm(c->oz_res, np, c->oz_q, c->oz_tiles, c->oz_ntiles, c->err, st, &oc));
         a.E = c->x64[bin];
         a.out = c->x64[bout];
-        SP2B_CUDA_TRY(launch_oz_crt_step(c->oz_q, c->oz_scale, a, st));
+        SP2B_CUDA_TRY(launch_oz_crt_step(c->oz_q, c->oz_scale, a, c->oz_rown, st));
       } else {
         a.A = a.B = a.E = c->hi[bin];
         a.A_lo = a.B_lo = a.E_lo = c->lo[bin];
