@@ -13,6 +13,9 @@
 // place of one FP64 product.  This is the residue-number-system form of the Ozaki scheme
 // (Ozaki, Uchino and Imamura, "Ozaki Scheme II: A GEMM-oriented emulation of
 // floating-point matrix multiplication using an integer modular technique", 2025).
+#include <algorithm>
+#include <vector>
+
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -287,14 +290,15 @@ __global__ void k_oz_residues_f64(const double* __restrict__ x, int np,
 }
 
 // ---------------------------------------------------------------------------------
-// 3. Persistent INT8 product of every plane with itself, upper 128 x 256 tiles,
+// 3. Persistent INT8 product of every plane with itself, upper 128 x 256 tiles (and the
+//    128 x 128 ones left over, oz_work_list),
 //    epilogue P mod m_t -> uint8 plane Q_t.
 //    warp 0: TMA producer; warp 1: TMEM owner + MMA issuer; warps 2..9: epilogue.
 // ---------------------------------------------------------------------------------
 struct OzGemmArgs {
   int np;
-  int ntiles;             // tiles per plane
-  const int2* tiles;      // {bi (128-row block), bjp (256-column block)}
+  int nwork;              // entries of the work list
+  const int4* work;       // {plane, 128-row block, first 128-column block, 128-column blocks}
   uint8_t* q;             // T planes np x np
   int* err;
   OzStepCtl ctl;
@@ -335,7 +339,7 @@ __global__ void __launch_bounds__(oz::NTHR, 1)
   tc_fence_after();
   const uint32_t tmem = tmem_holder;
   const int np = p.np;
-  const int nwork = oz::T * p.ntiles;
+  const int nwork = p.nwork;
   const int KB = np / oz::BK;
 
   if (warp == 0) {
@@ -346,9 +350,10 @@ __global__ void __launch_bounds__(oz::NTHR, 1)
       bool ok = true;
       uint32_t g = 0;
       for (int w = blockIdx.x; w < nwork && ok; w += gridDim.x) {
-        const int t = w / p.ntiles;
-        const int2 tl = p.tiles[w - t * p.ntiles];
-        const int ra = t * np + tl.x * oz::BM, rb = t * np + tl.y * oz::BN;
+        const int4 wk = p.work[w];
+        if (wk.w == 0) break;   // this CTA's list has ended
+        const int ra = wk.x * np + wk.y * oz::BM, rb = wk.x * np + wk.z * oz::BM;
+        const bool wide = wk.w == 2;
         for (int kb = 0; kb < KB; ++kb, ++g) {
           const int s = g % oz::ST;
           const uint32_t u = g / oz::ST;
@@ -358,10 +363,11 @@ __global__ void __launch_bounds__(oz::NTHR, 1)
           }
           const uint32_t fb = smem_u32(&bar_full[s]);
           const uint32_t st = sbase + s * oz::STAGE_BYTES;
-          mbar_expect_tx(fb, oz::STAGE_BYTES);
+          mbar_expect_tx(fb, wide ? oz::STAGE_BYTES : oz::STAGE_BYTES - oz::BM * oz::BK);
           tma_load_2d(st, &tm, fb, kb * oz::BK, ra);
           tma_load_2d(st + oz::A_BYTES, &tm, fb, kb * oz::BK, rb);
-          tma_load_2d(st + oz::A_BYTES + oz::BM * oz::BK, &tm, fb, kb * oz::BK, rb + oz::BM);
+          if (wide)
+            tma_load_2d(st + oz::A_BYTES + oz::BM * oz::BK, &tm, fb, kb * oz::BK, rb + oz::BM);
           issued_phase[s] = u & 1;
         }
       }
@@ -376,10 +382,14 @@ __global__ void __launch_bounds__(oz::NTHR, 1)
   } else if (warp == 1) {
     if (lane == 0) {
       // ---------------- MMA issuer ----------------
-      constexpr uint32_t idesc = make_idesc_s8(oz::BM, oz::BN);
+      constexpr uint32_t idesc2 = make_idesc_s8(oz::BM, oz::BN);
+      constexpr uint32_t idesc1 = make_idesc_s8(oz::BM, oz::BN / 2);
       bool ok = true;
       uint32_t g = 0, tl = 0;
       for (int w = blockIdx.x; w < nwork && ok; w += gridDim.x, ++tl) {
+        const int blocks = p.work[w].w;
+        if (blocks == 0) break;
+        const uint32_t idesc = blocks == 2 ? idesc2 : idesc1;
         const int a = tl & 1;
         const uint32_t v = tl >> 1;
         if (tl >= 2 && !mbar_wait(smem_u32(&bar_tempty[a]), (v - 1) & 1, &s_abort)) {
@@ -421,8 +431,9 @@ __global__ void __launch_bounds__(oz::NTHR, 1)
     const uint32_t lane_base = (uint32_t)(q * 32) << 16;
     uint32_t tl = 0;
     for (int w = blockIdx.x; w < nwork; w += gridDim.x, ++tl) {
-      const int t = w / p.ntiles;
-      const int2 tile = p.tiles[w - t * p.ntiles];
+      const int4 wk = p.work[w];
+      if (wk.w == 0) break;
+      const int t = wk.x;
       const int a = tl & 1;
       if (!mbar_wait_idle(smem_u32(&bar_tfull[a]), (tl >> 1) & 1, &s_abort)) break;
       tc_fence_after();
@@ -431,16 +442,16 @@ __global__ void __launch_bounds__(oz::NTHR, 1)
       const uint32_t m = (uint32_t)oz::mod(t);
       const unsigned long long magic = ~0ull / m + 1ull;
       const uint32_t off = m * ((1u << 30) / m + 1u);
-      const int r = tile.x * oz::BM + q * 32 + lane;
+      const int r = wk.y * oz::BM + q * 32 + lane;
       uint8_t* qrow = p.q + (size_t)t * np * np + (size_t)r * np;
 #pragma unroll 1
-      for (int cc = 0; cc < 4; ++cc) {
-        const int cl = half * 128 + cc * 32;
+      for (int cc = 0; cc < 2 * wk.w; ++cc) {
+        const int cl = half * 64 * wk.w + cc * 32;
         uint32_t v[32];
         tmem_ld32(tmem + lane_base + a * oz::BN + cl, v);
         tmem_wait_ld();
-        const int c0 = tile.y * oz::BN + cl;
-        if (c0 < np) {
+        const int c0 = wk.z * oz::BM + cl;
+        {
           alignas(16) uint8_t out[32];
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
@@ -711,27 +722,68 @@ int oz_nmod() { return oz::T; }
 
 size_t oz_scale_bytes() { return sizeof(OzScale); }
 
-// Upper 128 x 256 tiles of an np x np product: rows of block bi, columns of the 256-wide
-// block bjp, for every bjp that reaches the diagonal or beyond (2 bjp + 1 >= bi).  Ordered
-// in panels of kOzPanel column blocks, row blocks top to bottom inside a panel, so one wave
-// of the persistent grid shares few operand row blocks (their K-slices stay in L2).
-constexpr int kOzPanel = 6;
-void oz_tile_list(int np, std::vector<int2>& out) {
-  out.clear();
-  const int nb = np / oz::BM, nbp = (np + oz::BN - 1) / oz::BN;
-  for (int p0 = 0; p0 < nbp; p0 += kOzPanel) {
-    const int p1 = std::min(nbp, p0 + kOzPanel);
-    for (int bi = 0; bi < nb && bi <= 2 * p1 - 1; ++bi)
-      for (int bjp = std::max(p0, bi / 2); bjp < p1; ++bjp) out.push_back(make_int2(bi, bjp));
-  }
-}
-
 static int oz_sms() {
   int dev = 0, v = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0)
     v = 148;
   return v;
+}
+
+// The product's work for a persistent grid of `grid` CTAs, CTA c taking the entries c,
+// c + grid, ... until one with no blocks.  Upper 128-blocks of every plane: pairs of column
+// blocks as 128 x 256 tiles, the odd one left (the first at or right of the diagonal in odd
+// row blocks, the last of an odd count) as a 128 x 128 tile.  Wide tiles go first in panels
+// of kOzPanel column pairs, row blocks top to bottom inside a panel, so one wave shares few
+// operand row blocks (their K-slices stay in L2).  The wide tiles past the last whole wave
+// and the narrow ones are then dealt to the CTA with the least work, the wide ones cut in
+// two when every CTA can have one half.  In 128 x 128 tiles per SM: n = 2744 takes 16 (15.4
+// on average) where 1188 wide tiles took nine waves, 18; n = 1000 takes 3 instead of 4.
+constexpr int kOzPanel = 6;
+int oz_work_list(int np, std::vector<int4>& out) {
+  const int nb = np / oz::BM;
+  std::vector<int4> wide, narrow;
+  for (int t = 0; t < oz::T; ++t)
+    for (int p0 = 0; p0 < nb; p0 += 2 * kOzPanel) {
+      const int p1 = std::min(nb, p0 + 2 * kOzPanel);
+      for (int bi = 0; bi < p1; ++bi) {
+        int c = std::max(p0, bi);
+        if (c & 1) {   // an odd first block: alone
+          narrow.push_back(make_int4(t, bi, c, 1));
+          ++c;
+        }
+        for (; c + 1 < p1; c += 2) wide.push_back(make_int4(t, bi, c, 2));
+        if (c < p1) narrow.push_back(make_int4(t, bi, c, 1));
+      }
+    }
+  const int grid = (int)std::min<size_t>(2 * wide.size() + narrow.size(), (size_t)oz_sms());
+  const size_t whole = wide.size() / grid * grid;
+  out.assign(wide.begin(), wide.begin() + whole);
+  const size_t rest = wide.size() - whole;
+  const bool cut = 2 * rest + narrow.size() <= (size_t)grid;
+  std::vector<std::vector<int4>> tail(grid);
+  std::vector<int> load(grid, 0);
+  auto deal = [&](const int4& w) {
+    const int c = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+    tail[c].push_back(w);
+    load[c] += w.w;
+  };
+  for (size_t i = whole; i < wide.size(); ++i) {
+    int4 w = wide[i];
+    if (cut) {
+      w.w = 1;
+      deal(w);
+      ++w.z;
+    }
+    deal(w);
+  }
+  for (const int4& w : narrow) deal(w);
+  size_t rounds = 0;
+  for (const auto& v : tail) rounds = std::max(rounds, v.size());
+  for (size_t r = 0; r < rounds; ++r)
+    for (int c = 0; c < grid; ++c)
+      out.push_back(r < tail[c].size() ? tail[c][r] : make_int4(0, 0, 0, 0));
+  return grid;
 }
 
 cudaError_t launch_oz_planes(const __half* xhi, const __half* xlo, int np, int bf16,
@@ -758,9 +810,9 @@ cudaError_t launch_oz_planes(const __half* xhi, const __half* xlo, int np, int b
   return cudaGetLastError();
 }
 
-cudaError_t launch_oz_gemm(const int8_t* res, int np, uint8_t* qout, const int2* tiles,
-                           int ntiles, int* err, cudaStream_t st, const OzStepCtl* ctl) {
-  if (np % oz::BM != 0 || np > 65536 || ntiles <= 0) return cudaErrorInvalidValue;
+cudaError_t launch_oz_gemm(const int8_t* res, int np, uint8_t* qout, const int4* work,
+                           int nwork, int grid, int* err, cudaStream_t st, const OzStepCtl* ctl) {
+  if (np % oz::BM != 0 || np > 65536 || nwork <= 0) return cudaErrorInvalidValue;
   CUtensorMap tm;
   if (!make_tmap_box(&tm, res, (long long)oz::T * np, np, np, TMAP_U8, oz::BM))
     return cudaErrorInvalidValue;
@@ -769,13 +821,12 @@ cudaError_t launch_oz_gemm(const int8_t* res, int np, uint8_t* qout, const int2*
   if (e != cudaSuccess) return e;
   OzGemmArgs a;
   a.np = np;
-  a.ntiles = ntiles;
-  a.tiles = tiles;
+  a.nwork = nwork;
+  a.work = work;
   a.q = qout;
   a.err = err;
   if (ctl) a.ctl = *ctl;
   else memset(&a.ctl, 0, sizeof(a.ctl));
-  const int grid = std::min(oz::T * ntiles, oz_sms());
   k_oz_gemm<<<grid, oz::NTHR, oz::SMEM_BYTES, st>>>(tm, a);
   note_launch();
   return cudaGetLastError();

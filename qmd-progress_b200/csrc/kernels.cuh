@@ -142,7 +142,7 @@ cudaError_t launch_mcweeny_tc(const __half* xhi, const __half* xlo, const __half
 // INT8 (Ozaki residue) refinement products -------------------------------------------
 int oz_nmod();
 size_t oz_scale_bytes();
-void oz_tile_list(int np, std::vector<int2>& out);
+int oz_work_list(int np, std::vector<int4>& out);   // returns the grid it is dealt to
 cudaError_t launch_oz_planes(const __half* xhi, const __half* xlo, int np, int bf16,
                              void* scale, int8_t* res, cudaStream_t st);
 // SP2-step context of the launches that compute one step's X^2 in the exact INT8 mode.
@@ -154,8 +154,9 @@ struct OzStepCtl {
   int k;
   int active;   // 0: not part of an SP2 step (the McWeeny refinement)
 };
-cudaError_t launch_oz_gemm(const int8_t* res, int np, uint8_t* qout, const int2* tiles,
-                           int ntiles, int* err, cudaStream_t st, const OzStepCtl* ctl = nullptr);
+cudaError_t launch_oz_gemm(const int8_t* res, int np, uint8_t* qout, const int4* work,
+                           int nwork, int grid, int* err, cudaStream_t st,
+                           const OzStepCtl* ctl = nullptr);
 cudaError_t launch_oz_planes_f64(const double* x, int np, void* scale, const double* rown,
                                  int8_t* res, const OzStepCtl* ctl, cudaStream_t st);
 size_t oz_rown_doubles(int np);   // per-block row sums of the iterate a step wrote

@@ -44,12 +44,12 @@ struct Ctx {
   SolveOut* sout = nullptr;
   SolveOut* h_sout = nullptr;   // pinned
   int* err = nullptr;
-  // INT8 refinement: residue planes, reduced product planes, tile list, scale state
+  // INT8 refinement: residue planes, reduced product planes, work list, scale state
   int8_t* oz_res = nullptr;
   uint8_t* oz_q = nullptr;
   size_t oz_cap = 0;
-  int2* oz_tiles = nullptr;
-  int oz_tiles_np = 0, oz_ntiles = 0;
+  int4* oz_work = nullptr;
+  int oz_work_np = 0, oz_nwork = 0, oz_grid = 0;
   void* oz_scale = nullptr;
   double* oz_rown = nullptr;    // exact steps: per-block row sums of the iterate
   size_t oz_rown_cap = 0;

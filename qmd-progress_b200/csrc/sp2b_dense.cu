@@ -134,19 +134,20 @@ cudaError_t Ctx::ensure_oz(int np, cudaStream_t st) {
     oz_cap = need;
   }
   if (!oz_scale && (e = cudaMalloc(&oz_scale, oz_scale_bytes())) != cudaSuccess) return e;
-  if (oz_tiles_np != np) {
-    std::vector<int2> t;
-    oz_tile_list(np, t);
-    if (oz_tiles) cudaFree(oz_tiles);
-    oz_tiles = nullptr;
-    oz_tiles_np = 0;
-    if ((e = cudaMalloc((void**)&oz_tiles, t.size() * sizeof(int2))) != cudaSuccess) return e;
-    if ((e = cudaMemcpyAsync(oz_tiles, t.data(), t.size() * sizeof(int2), cudaMemcpyHostToDevice,
+  if (oz_work_np != np) {
+    std::vector<int4> w;
+    const int grid = oz_work_list(np, w);
+    if (oz_work) cudaFree(oz_work);
+    oz_work = nullptr;
+    oz_work_np = 0;
+    if ((e = cudaMalloc((void**)&oz_work, w.size() * sizeof(int4))) != cudaSuccess) return e;
+    if ((e = cudaMemcpyAsync(oz_work, w.data(), w.size() * sizeof(int4), cudaMemcpyHostToDevice,
                              st)) != cudaSuccess)
       return e;
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
-    oz_ntiles = (int)t.size();
-    oz_tiles_np = np;
+    oz_nwork = (int)w.size();
+    oz_grid = grid;
+    oz_work_np = np;
   }
   return cudaSuccess;
 }
@@ -394,7 +395,7 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
         oc.active = 1;
         SP2B_CUDA_TRY(launch_oz_planes_f64(c->x64[bin], np, c->oz_scale, k > 0 ? c->oz_rown : nullptr,
                                            c->oz_res, &oc, st));
-        SP2B_CUDA_TRY(launch_oz_gemm(c->oz_res, np, c->oz_q, c->oz_tiles, c->oz_ntiles, c->err, st, &oc));
+        SP2B_CUDA_TRY(launch_oz_gemm(c->oz_res, np, c->oz_q, c->oz_work, c->oz_nwork, c->oz_grid, c->err, st, &oc));
         a.E = c->x64[bin];
         a.out = c->x64[bout];
         SP2B_CUDA_TRY(launch_oz_crt_step(c->oz_q, c->oz_scale, a, c->oz_rown, st));
@@ -489,7 +490,7 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
     }
     SP2B_CUDA_TRY(launch_oz_planes(c->hi[fb], c->lo[fb], np, bf16, c->oz_scale, c->oz_res, st));
     if (timing) SP2B_CUDA_TRY(cudaEventRecord(c->ev_ref[1], st));
-    SP2B_CUDA_TRY(launch_oz_gemm(c->oz_res, np, c->oz_q, c->oz_tiles, c->oz_ntiles, c->err, st));
+    SP2B_CUDA_TRY(launch_oz_gemm(c->oz_res, np, c->oz_q, c->oz_work, c->oz_nwork, c->oz_grid, c->err, st));
     if (timing) SP2B_CUDA_TRY(cudaEventRecord(c->ev_ref[2], st));
     SP2B_CUDA_TRY(launch_oz_crt(c->oz_q, c->hi[fb], c->lo[fb], np, bf16, c->oz_scale, c->x64[0],
                                 c->hi[ob], c->lo[ob], st));
