@@ -11,7 +11,8 @@ __device__ __forceinline__ double warp_sum(double v) {
 }
 
 // Sum NS values per thread over the block; result valid in thread 0.  Fixed
-// shuffle/warp order, so the result is bitwise reproducible.
+// shuffle/warp order, so the result is bitwise reproducible.  The warps' sums are added by
+// shuffles too: one thread adding 8 to 32 of them in turn took over a microsecond.
 template <int NS>
 __device__ __forceinline__ void block_sum(double (&v)[NS], double* red /*[32][NS]*/) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -21,12 +22,9 @@ __device__ __forceinline__ void block_sum(double (&v)[NS], double* red /*[32][NS
   if (lane == 0)
     for (int q = 0; q < NS; ++q) red[warp * NS + q] = v[q];
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int q = 0; q < NS; ++q) {
-      double s = 0.0;
-      for (int w = 0; w < nw; ++w) s += red[w * NS + q];
-      v[q] = s;
-    }
+  if (warp == 0) {
+#pragma unroll
+    for (int q = 0; q < NS; ++q) v[q] = warp_sum(lane < nw ? red[lane * NS + q] : 0.0);
   }
   __syncthreads();
 }
