@@ -74,6 +74,8 @@ struct OzScale {
   unsigned long long next_bits;   // running maximum of k_oz_rowmax (zero between launches)
   int S;      // -1: no valid scale (non-finite input)
   unsigned counter;               // CTAs of k_oz_rowmax that have arrived
+  int kept;   // the last k_oz_rowmax found the S that the planes were already formed with
+  int pad_;
 };
 
 // SP2-step context of the launches that compute one step's X^2 (the exact INT8 mode):
@@ -241,6 +243,24 @@ __device__ __forceinline__ void oz_store_planes(int8_t* res, size_t plane, size_
   }
 }
 
+// Four consecutive elements x of every plane, rounded to the grid 1 / scale.
+template <int t>
+__device__ __forceinline__ void oz_store_word(int8_t* res, size_t plane, size_t off,
+                                              const OzInt (&M)[4]) {
+  if constexpr (t < oz::T) {
+    *reinterpret_cast<uint32_t*>(res + (size_t)t * plane + off) =
+        low_bytes(oz_residue<t>(M[0]), oz_residue<t>(M[1]), oz_residue<t>(M[2]), oz_residue<t>(M[3]));
+    oz_store_word<t + 1>(res, plane, off, M);
+  }
+}
+__device__ __forceinline__ void oz_store_planes4(int8_t* res, size_t plane, size_t off,
+                                                 const double (&x)[4], double scale) {
+  OzInt M[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) M[j] = oz_round(x[j], scale);
+  oz_store_word<0>(res, plane, off, M);
+}
+
 // Bound by HBM and FP32 issue (8 moduli x 5.75 instructions an element).
 template <typename T>
 __global__ void k_oz_residues(const T* __restrict__ hi, const T* __restrict__ lo, int np,
@@ -268,8 +288,9 @@ __global__ void k_oz_residues(const T* __restrict__ hi, const T* __restrict__ lo
 
 __global__ void k_oz_residues_f64(const double* __restrict__ x, int np,
                                   const OzScale* __restrict__ sc, int8_t* __restrict__ res,
-                                  const OzStepCtl c) {
+                                  const OzStepCtl c, int formed) {
   if (oz_skip(c)) return;
+  if (formed && sc->kept) return;   // the step before formed these planes
   const int S = sc->S;
   const double scale = S < 0 ? 0.0 : ldexp(1.0, S);
   const size_t plane = (size_t)np * np;
@@ -601,13 +622,16 @@ __global__ void __launch_bounds__(256)
 // 5. Exact INT8 mode: the step's last launch.  X_k^2 from the residues, the branch of
 //    step k from its record (control_prologue), X_{k+1} = a X_k^2 + b X_k in FP64 over
 //    both triangles, and the step's sums {||X_{k+1}||^2, Tr X_{k+1}, ||X_k - X_k^2||^2,
-//    Tr X_k^2} through the last-CTA finalisation, like the other step kernels.  A fixed
-//    grid walks the upper 32 x 32 block pairs (diagonal blocks hold both triangles, whose
+//    Tr X_k^2} through the last-CTA finalisation, like the other step kernels.  It also
+//    leaves the residue planes of X_{k+1} with step k's scale, while the values are in
+//    registers: the scale changes two or three times in a solve, and only then does
+//    k_oz_residues_f64 form them again (planes by a pass over X cost 27 us a step at
+//    n = 2744).  A fixed grid walks the upper 32 x 32 block pairs (diagonal blocks hold both triangles, whose
 //    squares are equal bit for bit: the integer products are symmetric).
 // ---------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
     k_oz_crt_step(const uint8_t* __restrict__ q, const OzScale* __restrict__ sc, const StepArgs p,
-                  double* __restrict__ rown) {
+                  double* __restrict__ rown, int8_t* __restrict__ res) {
   __shared__ double s_v[32][33];
   __shared__ double red[32 * 4];
   __shared__ int s_flag;
@@ -619,6 +643,7 @@ __global__ void __launch_bounds__(256)
   double* __restrict__ Xo = (double*)p.out;
   const int S = sc->S;
   const double down = S < 0 ? __longlong_as_double(0x7ff8000000000000ll) : ldexp(1.0, -2 * S);
+  const double up = S < 0 ? 0.0 : ldexp(1.0, S);
   const size_t plane = (size_t)np * np;
   const int row = threadIdx.x >> 3, c4 = (threadIdx.x & 7) * 4;   // a thread's four columns
   const long long nb = np / 32, nblk = nb * (nb + 1) / 2;
@@ -651,6 +676,7 @@ __global__ void __launch_bounds__(256)
     double2* o = reinterpret_cast<double2*>(Xo + e);
     o[0] = make_double2(nx[0], nx[1]);
     o[1] = make_double2(nx[2], nx[3]);
+    oz_store_planes4(res, plane, e, nx, up);
     // this block's share of ||row i of X_{k+1}||^2 (the next step's scale)
     rs += __shfl_xor_sync(0xffffffffu, rs, 1);
     rs += __shfl_xor_sync(0xffffffffu, rs, 2);
@@ -669,6 +695,7 @@ __global__ void __launch_bounds__(256)
       double2* m = reinterpret_cast<double2*>(Xo + (size_t)r * np + ib * 32 + c4);
       m[0] = make_double2(v[0], v[1]);
       m[1] = make_double2(v[2], v[3]);
+      oz_store_planes4(res, plane, (size_t)r * np + ib * 32 + c4, v, up);
       cs += __shfl_xor_sync(0xffffffffu, cs, 1);
       cs += __shfl_xor_sync(0xffffffffu, cs, 2);
       cs += __shfl_xor_sync(0xffffffffu, cs, 4);
@@ -712,7 +739,9 @@ __global__ void __launch_bounds__(256)
   *counter = 0u;
   __threadfence();
   sc->r2max_bits = atomicExch(&sc->next_bits, 0ull);
-  sc->S = oz_choose_scale(__longlong_as_double((long long)sc->r2max_bits), np);
+  const int S = oz_choose_scale(__longlong_as_double((long long)sc->r2max_bits), np);
+  sc->kept = S == sc->S;
+  sc->S = S;
 }
 
 // ---------------------------------------------------------------------------------
@@ -848,14 +877,15 @@ cudaError_t launch_oz_crt(const uint8_t* q, const __half* xhi, const __half* xlo
   return cudaGetLastError();
 }
 
-// rown: the row sums launch_oz_crt_step left for this x, or null (they are formed from x).
+// rown: null for the first step (the scale and the planes from x); else the row sums that
+// launch_oz_crt_step left with its planes of this x, formed again if the scale changed.
 cudaError_t launch_oz_planes_f64(const double* x, int np, void* scale, const double* rown,
                                  int8_t* res, const OzStepCtl* ctl, cudaStream_t st) {
   if (np % oz::BM != 0 || np > 65536) return cudaErrorInvalidValue;
   OzScale* sc = (OzScale*)scale;
   const int rgrid = std::min((np + 7) / 8, 148 * 8);
   if (rown) {
-    k_oz_rowmax<<<std::min(rgrid, 148), 256, 0, st>>>(rown, np, sc, &sc->counter, *ctl);
+    k_oz_rowmax<<<rgrid, 256, 0, st>>>(rown, np, sc, &sc->counter, *ctl);
     note_launch(2);
   } else {
     cudaError_t e = cudaMemsetAsync(sc, 0, sizeof(OzScale), st);
@@ -866,18 +896,18 @@ cudaError_t launch_oz_planes_f64(const double* x, int np, void* scale, const dou
   }
   const size_t groups = (size_t)np * np / 8;
   const int g = (int)std::min<size_t>((groups + 255) / 256, 148 * 16);
-  k_oz_residues_f64<<<g, 256, 0, st>>>(x, np, sc, res, *ctl);
+  k_oz_residues_f64<<<g, 256, 0, st>>>(x, np, sc, res, *ctl, rown != nullptr);
   return cudaGetLastError();
 }
 
 size_t oz_rown_doubles(int np) { return (size_t)np * (np / 32); }
 
 cudaError_t launch_oz_crt_step(const uint8_t* q, const void* scale, const StepArgs& a, double* rown,
-                               cudaStream_t st) {
+                               int8_t* res, cudaStream_t st) {
   if (a.np % 128 != 0) return cudaErrorInvalidValue;
   const long long nb = a.np / 32;
   const int grid = (int)std::min<long long>(nb * (nb + 1) / 2, 148 * 8);
-  k_oz_crt_step<<<grid, 256, 0, st>>>(q, (const OzScale*)scale, a, rown);
+  k_oz_crt_step<<<grid, 256, 0, st>>>(q, (const OzScale*)scale, a, rown, res);
   note_launch();
   return cudaGetLastError();
 }

@@ -161,7 +161,7 @@ cudaError_t launch_oz_planes_f64(const double* x, int np, void* scale, const dou
                                  int8_t* res, const OzStepCtl* ctl, cudaStream_t st);
 size_t oz_rown_doubles(int np);   // per-block row sums of the iterate a step wrote
 cudaError_t launch_oz_crt_step(const uint8_t* q, const void* scale, const StepArgs& a, double* rown,
-                               cudaStream_t st);
+                               int8_t* res, cudaStream_t st);
 cudaError_t launch_oz_crt(const uint8_t* q, const __half* xhi, const __half* xlo, int np,
                           int bf16, const void* scale, double* x2, __half* rhi, __half* rlo,
                           cudaStream_t st);

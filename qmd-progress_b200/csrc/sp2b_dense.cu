@@ -398,7 +398,7 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
         SP2B_CUDA_TRY(launch_oz_gemm(c->oz_res, np, c->oz_q, c->oz_work, c->oz_nwork, c->oz_grid, c->err, st, &oc));
         a.E = c->x64[bin];
         a.out = c->x64[bout];
-        SP2B_CUDA_TRY(launch_oz_crt_step(c->oz_q, c->oz_scale, a, c->oz_rown, st));
+        SP2B_CUDA_TRY(launch_oz_crt_step(c->oz_q, c->oz_scale, a, c->oz_rown, c->oz_res, st));
       } else {
         a.A = a.B = a.E = c->hi[bin];
         a.A_lo = a.B_lo = a.E_lo = c->lo[bin];
