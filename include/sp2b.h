@@ -382,7 +382,7 @@ int sp2b_dev_adjoint_step_f32(const float* g, const float* x, float* g_out, floa
  *   adjoint_step_split: o = {g, x} (branch 1) or 2g - {g, x} (branch 0), g and x
  *                       symmetric, formed as one symmetric product over the
  *                       concatenated K range [g | x][x | g]^T with the branch in its
- *                       epilogue when np is a multiple of 256 (else g x in FP32 and a
+ *                       epilogue when np <= 1280 or a multiple of 256 (else g x in FP32 and a
  *                       combine pass); o must not alias g or x. */
 int sp2b_split_dim(int n);
 int sp2b_dev_normalize_split(const float* h, int n, double mineval, double maxeval, void* x_hi,

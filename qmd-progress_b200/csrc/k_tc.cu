@@ -16,6 +16,7 @@
 #include "tc_ptx.cuh"
 
 #include <map>
+#include <tuple>
 #include <utility>
 #include <vector>
 
@@ -336,12 +337,13 @@ __device__ __forceinline__ TileInfo persist_tile(const StepArgs& p, int t) {
 // mirror of an off-diagonal tile is stored from the registers.  Otherwise each lane reads
 // its row of X_k from global memory and stores the block and its mirror itself.
 // ES: the tile's X_k block is staged in shared memory like ESM's (estage: this half's hi
-// box, then its lo box, 128-byte swizzle), the results leave by the direct stores.
-template <typename T, int EPI, bool ESM, bool ES = false>
+// box, then its lo box, 128-byte swizzle), the results leave by the direct stores.  HC:
+// columns of a half (64; 32 for the 64-column tiles, whose halves share one staged box).
+template <typename T, int EPI, bool ESM, bool ES = false, int HC = 64>
 __device__ __forceinline__ void epi_tile(const StepArgs& p, const TileInfo& ti, uint32_t tacc,
                                          int q, int half, int lane, double alpha, double beta,
                                          double (&sums)[4], uint8_t* scr, uint8_t* estage,
-                                         int cc_lo = 0, int cc_hi = 64 / tcp::CHUNK) {
+                                         int cc_lo = 0, int cc_hi = HC / tcp::CHUNK) {
   using TR = SplitTraits<T>;
   const int ld = p.ld;
   if (EPI == 0 && ti.ok) {
@@ -358,7 +360,7 @@ __device__ __forceinline__ void epi_tile(const StepArgs& p, const TileInfo& ti, 
     // for itself in the sums, every warp has the same four chunks, and the tile leaves by
     // TMA as computed.
     int first = cc_lo;
-    while (!ESM && first < cc_hi && ti.diag && ti.j0 + half * 64 + first * tcp::CHUNK + 15 < r0)
+    while (!ESM && first < cc_hi && ti.diag && ti.j0 + half * HC + first * tcp::CHUNK + 15 < r0)
       ++first;
     // the rows of X_k for the next chunk are fetched while this one is processed
     uint4 pf[4];
@@ -370,11 +372,11 @@ __device__ __forceinline__ void epi_tile(const StepArgs& p, const TileInfo& ti, 
       pf[2] = sl[0];
       pf[3] = sl[1];
     };
-    if (!ESM && !ES && first < cc_hi) fetch_e(ti.j0 + half * 64 + first * tcp::CHUNK);
+    if (!ESM && !ES && first < cc_hi) fetch_e(ti.j0 + half * HC + first * tcp::CHUNK);
     const int rl = q * 32 + lane;   // row inside the tile
 #pragma unroll 1
     for (int cc = first; cc < cc_hi; ++cc) {
-      const int cl = half * 64 + cc * tcp::CHUNK;
+      const int cl = half * HC + cc * tcp::CHUNK;
       uint32_t hh[16], xx[16];
       tmem_ld16(tacc + cl, hh);
       tmem_ld16(tacc + tc::BN + cl, xx);
@@ -383,7 +385,8 @@ __device__ __forceinline__ void epi_tile(const StepArgs& p, const TileInfo& ti, 
       // 16-byte chunk k of row rl of a staged box sits at chunk k ^ (rl & 7) (128-byte
       // swizzle); estage is this half's stage: the hi box, then the lo box
       uint8_t* eb = (ESM || ES) ? estage + rl * 128 : nullptr;
-      const int k0 = ((2 * cc) ^ (rl & 7)) * 16, k1 = ((2 * cc + 1) ^ (rl & 7)) * 16;
+      const int kc = 2 * cc + (HC == 32 ? 4 * half : 0);
+      const int k0 = (kc ^ (rl & 7)) * 16, k1 = ((kc + 1) ^ (rl & 7)) * 16;
       {
         uint4* dh = reinterpret_cast<uint4*>(ehi);
         uint4* dl = reinterpret_cast<uint4*>(elo);
@@ -615,8 +618,8 @@ __device__ __forceinline__ void epi_tile(const StepArgs& p, const TileInfo& ti, 
     double* D = (double*)p.out;
     const int nout = p.n_out, ldo = p.ld_out;
 #pragma unroll 1
-    for (int cc = 0; cc < 64 / tcp::CHUNK; ++cc) {
-      const int cl = half * 64 + cc * tcp::CHUNK;
+    for (int cc = 0; cc < HC / tcp::CHUNK; ++cc) {
+      const int cl = half * HC + cc * tcp::CHUNK;
       uint32_t hh[16], xx[16];
       tmem_ld16(tacc + cl, hh);
       tmem_ld16(tacc + tc::BN + cl, xx);
@@ -918,37 +921,44 @@ __global__ void __launch_bounds__(ESM ? tcp::NTHR_E : tcp::NTHR, 1)
 // instead of from global memory (with one tile per CTA the epilogue is not hidden behind
 // a next tile's products, and its per-row reads from L2 were its latency).
 // ---------------------------------------------------------------------------------
-namespace tcq {
-constexpr int BH = 64;                                  // B rows staged per CTA (N / 2)
-constexpr int A_BYTES = tc::BM * tc::BK * 2;            // 16 KB
-constexpr int BH_BYTES = BH * tc::BK * 2;               // 8 KB
-constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * BH_BYTES; // 48 KB
-constexpr int ST = 4;
-constexpr int SCR_OFF = ST * STAGE_BYTES;
-constexpr int SMEM_BYTES = SCR_OFF + tcp::EPI_WARPS * tcp::SCR_WARP + 1024;
-// single-wave form with the X_k block staged: three operand stages, the epilogue scratch,
-// then the CTA's 128 x 128 block of X_k (hi and lo, two 64-column halves)
-constexpr int ST_ES = 3;
-constexpr int SCR_OFF_ES = ST_ES * STAGE_BYTES;
-constexpr int E_OFF_ES = SCR_OFF_ES + tcp::EPI_WARPS * tcp::SCR_WARP;
-constexpr int E_BYTES_ES = 4 * tc::TILE_BYTES;
-constexpr int SMEM_BYTES_ES = E_OFF_ES + E_BYTES_ES + 1024;
-// 227 KB of shared memory per block on sm_100, less the kernel's ~1.2 KB of static
-// shared memory (barriers, the reduction array)
-static_assert(SMEM_BYTES <= 232448 - 1536 && SMEM_BYTES_ES <= 232448 - 1536,
-              "paired kernel: shared memory beyond the per-block limit");
-}  // namespace tcq
+// NB: columns of a pair's tile.  128, or 64 for the single-wave form when the tiles would
+// occupy at most half of the SMs (np <= 1280): twice the pairs, each with half the products
+// and, what counts more there, half the epilogue.
+template <bool ES, int NB>
+struct PairCfg {
+  static constexpr int BH = NB / 2;                              // B rows staged per CTA
+  static constexpr int A_BYTES = tc::BM * tc::BK * 2;            // 16 KB
+  static constexpr int BH_BYTES = BH * tc::BK * 2;               // 8 KB (4 KB)
+  static constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * BH_BYTES; // 48 KB (40 KB)
+  // single-wave form with the X_k block staged: three operand stages, the epilogue scratch,
+  // then the CTA's 128 x NB block of X_k (hi and lo, in 64-column boxes)
+  static constexpr int ST = ES ? 3 : 4;
+  static constexpr int SCR_OFF = ST * STAGE_BYTES;
+  static constexpr int E_OFF = SCR_OFF + tcp::EPI_WARPS * tcp::SCR_WARP;
+  static constexpr int E_BYTES = ES ? 2 * (NB / 64) * tc::TILE_BYTES : 0;
+  static constexpr int SMEM_BYTES = E_OFF + E_BYTES + 1024;
+  // 227 KB of shared memory per block on sm_100, less the kernel's ~1.2 KB of static
+  // shared memory (barriers, the reduction array)
+  static_assert(SMEM_BYTES <= 232448 - 1536, "paired kernel: shared memory beyond the limit");
+};
 
-template <typename T, int EPI, bool ANTI = false, bool ES = false>
+// TAIL: the work list ends with 64-column tiles (pair_tiles), marked kPairNarrow; their tile.y
+// counts 64-column blocks.  (A form of its own: the choice at run time cost the plain one 4 %
+// at n = 8192.)
+constexpr int kPairNarrow = 1 << 24;
+
+template <typename T, int EPI, bool ANTI = false, bool ES = false, int NB = 128, bool TAIL = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tcp::NTHR, 1)
     k_tc_pair(const __grid_constant__ CUtensorMap tm_ahi, const __grid_constant__ CUtensorMap tm_alo,
               const __grid_constant__ CUtensorMap tm_bhi, const __grid_constant__ CUtensorMap tm_blo,
               const __grid_constant__ CUtensorMap tm_a2hi, const __grid_constant__ CUtensorMap tm_a2lo,
               const __grid_constant__ CUtensorMap tm_b2hi, const __grid_constant__ CUtensorMap tm_b2lo,
               const StepArgs p, const int2* __restrict__ ptiles, int ntiles) {
+  using Q = PairCfg<ES, NB>;
+  constexpr int ST = Q::ST;   // operand stages
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bar_full[tcq::ST];
-  __shared__ __align__(8) uint64_t bar_empty[tcq::ST];
+  __shared__ __align__(8) uint64_t bar_full[ST];
+  __shared__ __align__(8) uint64_t bar_empty[ST];
   __shared__ __align__(8) uint64_t bar_tfull[2];
   __shared__ __align__(8) uint64_t bar_tempty[2];
   __shared__ __align__(8) uint64_t bar_final;
@@ -957,7 +967,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tcp::NTHR, 1)
   __shared__ double red[32 * 4];
   __shared__ int s_flag;
   __shared__ volatile int s_abort;
-  constexpr int ST = ES ? tcq::ST_ES : tcq::ST;   // operand stages
   if (ES && ntiles > (int)(gridDim.x >> 1)) {        // one tile per pair (uniform exit)
     if (threadIdx.x == 0 && p.err) atomicExch(p.err, 1);
     return;
@@ -1007,8 +1016,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tcp::NTHR, 1)
       uint32_t g = 0;
       for (int w = pair; w < ntiles && ok; w += npairs) {
         const int2 tile = ptiles[w];
-        const int ra = tile.x * 2 * tc::BM + (int)rank * tc::BM;
-        const int rb = tile.y * tc::BN + (int)rank * tcq::BH;
+        const bool narrow = TAIL && (tile.x & kPairNarrow);
+        const int ra = (tile.x & (kPairNarrow - 1)) * 2 * tc::BM + (int)rank * tc::BM;
+        // a narrow tile takes 32 rows of B from each CTA (the first ones of its box)
+        const int rb = narrow ? tile.y * 64 + (int)rank * 32 : tile.y * NB + (int)rank * Q::BH;
         for (int kb = 0; kb < KBT; ++kb, ++g) {
           const int s = g % ST;
           const uint32_t u = g / ST;
@@ -1017,25 +1028,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tcp::NTHR, 1)
             break;
           }
           const uint32_t fb0 = map_to_rank(smem_u32(&bar_full[s]), 0);
-          if (rank == 0) mbar_expect_tx(smem_u32(&bar_full[s]), 2 * tcq::STAGE_BYTES);
-          const uint32_t st = sbase + s * tcq::STAGE_BYTES;
+          if (rank == 0) mbar_expect_tx(smem_u32(&bar_full[s]), 2 * Q::STAGE_BYTES);
+          const uint32_t st = sbase + s * Q::STAGE_BYTES;
           const bool sw = ANTI && kb >= KB;    // second pass: roles swapped
           const int kc = (sw ? kb - KB : kb) * tc::BK;
           tma_load_2d_pair(st, sw ? &tm_a2hi : &tm_ahi, fb0, kc, ra);
-          tma_load_2d_pair(st + tcq::A_BYTES, sw ? &tm_a2lo : &tm_alo, fb0, kc, ra);
-          tma_load_2d_pair(st + 2 * tcq::A_BYTES, sw ? &tm_b2hi : &tm_bhi, fb0, kc, rb);
-          tma_load_2d_pair(st + 2 * tcq::A_BYTES + tcq::BH_BYTES, sw ? &tm_b2lo : &tm_blo, fb0, kc,
+          tma_load_2d_pair(st + Q::A_BYTES, sw ? &tm_a2lo : &tm_alo, fb0, kc, ra);
+          tma_load_2d_pair(st + 2 * Q::A_BYTES, sw ? &tm_b2hi : &tm_bhi, fb0, kc, rb);
+          tma_load_2d_pair(st + 2 * Q::A_BYTES + Q::BH_BYTES, sw ? &tm_b2lo : &tm_blo, fb0, kc,
                            rb);
           if (ES && kb == 0 && !e_issued) {
-            // this CTA's block of E (= A): rows ra.., columns 128 bj.., two 64-column halves
+            // this CTA's block of E (= A): rows ra.., columns NB bj.., in 64-column boxes
             e_issued = true;
             const uint32_t eb = smem_u32(&bar_e);
-            const uint32_t es = sbase + tcq::E_OFF_ES;
-            mbar_expect_tx(eb, tcq::E_BYTES_ES);
-            for (int h = 0; h < 2; ++h) {
-              tma_load_2d(es + h * 2 * tc::TILE_BYTES, &tm_ahi, eb, tile.y * tc::BN + h * 64, ra);
+            const uint32_t es = sbase + Q::E_OFF;
+            mbar_expect_tx(eb, Q::E_BYTES);
+            for (int h = 0; h < NB / 64; ++h) {
+              tma_load_2d(es + h * 2 * tc::TILE_BYTES, &tm_ahi, eb, tile.y * NB + h * 64, ra);
               tma_load_2d(es + h * 2 * tc::TILE_BYTES + tc::TILE_BYTES, &tm_alo, eb,
-                          tile.y * tc::BN + h * 64, ra);
+                          tile.y * NB + h * 64, ra);
             }
           }
         }
@@ -1049,7 +1060,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tcp::NTHR, 1)
   } else if (warp == 1) {
     if (lane == 0 && rank == 0) {
       // ---------------- MMA issuer (CTA 0 of the pair) ----------------
-      constexpr uint32_t idesc = make_idesc(SplitTraits<T>::kFmt, 2 * tc::BM, tc::BN);
+      constexpr uint32_t idesc_full = make_idesc(SplitTraits<T>::kFmt, 2 * tc::BM, NB);
+      constexpr uint32_t idesc_narrow = make_idesc(SplitTraits<T>::kFmt, 2 * tc::BM, 64);
       bool ok = true;
       uint32_t g = 0, tl = 0;
       for (int w = pair; w < ntiles && ok; w += npairs, ++tl) {
@@ -1061,6 +1073,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tcp::NTHR, 1)
         }
         tc_fence_after();
         const uint32_t acc_hh = tmem + a * 256, acc_x = tmem + a * 256 + tc::BN;
+        uint32_t idesc = idesc_full;
+        if (TAIL && (ptiles[w].x & kPairNarrow)) idesc = idesc_narrow;
         for (int kb = 0; kb < KBT; ++kb, ++g) {
           const int s = g % ST;
           if (!mbar_wait(smem_u32(&bar_full[s]), (g / ST) & 1, &s_abort)) {
@@ -1068,11 +1082,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tcp::NTHR, 1)
             break;
           }
           tc_fence_after();
-          const uint32_t st = sbase + s * tcq::STAGE_BYTES;
+          const uint32_t st = sbase + s * Q::STAGE_BYTES;
           const uint64_t d_ahi = sw128_desc(st);
-          const uint64_t d_alo = sw128_desc(st + tcq::A_BYTES);
-          const uint64_t d_bhi = sw128_desc(st + 2 * tcq::A_BYTES);
-          const uint64_t d_blo = sw128_desc(st + 2 * tcq::A_BYTES + tcq::BH_BYTES);
+          const uint64_t d_alo = sw128_desc(st + Q::A_BYTES);
+          const uint64_t d_bhi = sw128_desc(st + 2 * Q::A_BYTES);
+          const uint64_t d_blo = sw128_desc(st + 2 * Q::A_BYTES + Q::BH_BYTES);
 #pragma unroll
           for (int kk = 0; kk < tc::BK / tc::UK; ++kk) {
             const uint64_t off = (uint64_t)((kk * tc::UK * 2) >> 4);
@@ -1106,20 +1120,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tcp::NTHR, 1)
       if (!mbar_wait_idle(smem_u32(&bar_tfull[a]), (tl >> 1) & 1, &s_abort)) break;
       tc_fence_after();
       TileInfo ti;
-      const int brow = tile.x * 2 + (int)rank;
+      const bool narrow = TAIL && (tile.x & kPairNarrow);
+      const int brow = (tile.x & (kPairNarrow - 1)) * 2 + (int)rank;
       ti.row0 = 0;
       ti.i0 = brow * tc::BM;
-      ti.j0 = tile.y * tc::BN;
+      ti.j0 = tile.y * (narrow ? 64 : NB);
       ti.kb = KB;
       ti.core = p.core;
-      ti.ok = brow <= tile.y;        // CTA 1's block of a diagonal pair lies below it
-      ti.diag = brow == tile.y;
+      ti.ok = brow <= ti.j0 / tc::BM;   // CTA 1's block of a diagonal pair lies below it
+      ti.diag = brow == ti.j0 / tc::BM;
       if (ES && !mbar_wait_idle(smem_u32(&bar_e), 0, &s_abort)) break;
-      epi_tile<T, EPI, false, ES>(p, ti, tmem + lane_base + a * 256, q, half, lane, alpha, beta,
-                                  sums,
-                                  smem + (ES ? tcq::SCR_OFF_ES : tcq::SCR_OFF) +
-                                      (warp - 2) * tcp::SCR_WARP,
-                                  ES ? smem + tcq::E_OFF_ES + half * 2 * tc::TILE_BYTES : nullptr);
+      uint8_t* scr = smem + Q::SCR_OFF + (warp - 2) * tcp::SCR_WARP;
+      const uint32_t tacc = tmem + lane_base + a * 256;
+      if (narrow)
+        epi_tile<T, EPI, false, ES, 32>(p, ti, tacc, q, half, lane, alpha, beta, sums, scr, nullptr);
+      else
+        epi_tile<T, EPI, false, ES, NB / 2>(
+            p, ti, tacc, q, half, lane, alpha, beta, sums, scr,
+            ES ? smem + Q::E_OFF + (NB == 128 ? half * 2 * tc::TILE_BYTES : 0) : nullptr);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(tempty0[a]);
@@ -1376,8 +1394,8 @@ static const int4* dense_tiles(int np, cudaStream_t st) {
   return d;
 }
 
-// Work items of the paired kernel, {bi2, bj} with bj >= 2 bi2, in panels of kPanel column
-// blocks (row pairs top to bottom inside a panel).  Cached per (device, np).
+// Tiles of the paired kernel, {bi2, bj} with bj >= 2 bi2 (128-column blocks), in panels of
+// kPanel column blocks (row pairs top to bottom inside a panel).
 void pair_tile_order(int nb, int panel, std::vector<int2>& out) {
   out.clear();
   for (int p0 = 0; p0 < nb; p0 += panel) {
@@ -1386,14 +1404,21 @@ void pair_tile_order(int nb, int panel, std::vector<int2>& out) {
       for (int bj = std::max(2 * bi2, p0); bj < p1; ++bj) out.push_back(make_int2(bi2, bj));
   }
 }
+static int pair_tile_count(int np) {
+  const int nb = np / tc::BM, np2 = (nb + 1) / 2;
+  return nb * np2 - np2 * (np2 - 1);   // row pair bi2 has the column blocks from 2 bi2 on
+}
 
-static const int2* pair_tiles(int np, cudaStream_t st, int* count) {
+// Work items of a launch, cached per (device, np, form).  whole: the tiles that stay whole;
+// the others follow as two 64-column tiles each (NB = 64: whole = 0).
+static const int2* pair_tiles(int np, int whole, bool mark, cudaStream_t st, int* count) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
   static std::mutex mu;
-  static std::map<std::pair<int, int>, std::pair<int2*, int>> cache;
+  static std::map<std::tuple<int, int, int>, std::pair<int2*, int>> cache;
+  const std::tuple<int, int, int> key(dev, np, whole);
   std::lock_guard<std::mutex> lk(mu);
-  auto it = cache.find({dev, np});
+  auto it = cache.find(key);
   if (it != cache.end()) {
     *count = it->second.second;
     return it->second.first;
@@ -1402,21 +1427,31 @@ static const int2* pair_tiles(int np, cudaStream_t st, int* count) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
     return nullptr;
-  std::vector<int2> t;
-  pair_tile_order(np / tc::BM, kPanel, t);
+  std::vector<int2> blocks, t;
+  pair_tile_order(np / tc::BM, kPanel, blocks);
+  for (size_t i = 0; i < blocks.size(); ++i) {
+    int2 q = blocks[i];
+    if ((int)i < whole) {
+      t.push_back(q);
+      continue;
+    }
+    if (mark) q.x |= kPairNarrow;
+    t.push_back(make_int2(q.x, 2 * q.y));
+    t.push_back(make_int2(q.x, 2 * q.y + 1));
+  }
   int2* d = nullptr;
   if (cudaMalloc((void**)&d, t.size() * sizeof(int2)) != cudaSuccess) return nullptr;
   if (cudaMemcpy(d, t.data(), t.size() * sizeof(int2), cudaMemcpyHostToDevice) != cudaSuccess) {
     cudaFree(d);
     return nullptr;
   }
-  cache[{dev, np}] = {d, (int)t.size()};
+  cache[key] = {d, (int)t.size()};
   *count = (int)t.size();
   return d;
 }
 
 // Clusters of the paired kernel that can be resident at once (one CTA per SM).
-template <typename T, int EPI, bool ANTI = false, bool ES = false>
+template <typename T, int EPI, bool ANTI = false, bool ES = false, int NB = 128, bool TAIL = false>
 static int pair_clusters() {
   static int per_dev[64] = {0};
   int dev = 0;
@@ -1425,7 +1460,7 @@ static int pair_clusters() {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(num_sms() & ~1, 1, 1);
   cfg.blockDim = dim3(tcp::NTHR, 1, 1);
-  cfg.dynamicSmemBytes = ES ? tcq::SMEM_BYTES_ES : tcq::SMEM_BYTES;
+  cfg.dynamicSmemBytes = PairCfg<ES, NB>::SMEM_BYTES;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeClusterDimension;
   attr.val.clusterDim.x = 2;
@@ -1434,7 +1469,7 @@ static int pair_clusters() {
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, (void*)k_tc_pair<T, EPI, ANTI, ES>, &cfg) !=
+  if (cudaOccupancyMaxActiveClusters(&n, (void*)k_tc_pair<T, EPI, ANTI, ES, NB, TAIL>, &cfg) !=
           cudaSuccess ||
       n <= 0) {
     cudaGetLastError();
@@ -1444,53 +1479,97 @@ static int pair_clusters() {
   return n;
 }
 
-// Paired-CTA launch for np a multiple of 256; returns cudaErrorNotSupported when the
-// caller should use the single-CTA kernel instead.  ANTI: A = G, B = X (see k_tc_pair).
-template <typename T, int EPI, bool ANTI = false>
-static cudaError_t launch_pair(const StepArgs& a, cudaStream_t st) {
-  if (a.np % (2 * tc::BM) != 0 || a.ld != a.np) return cudaErrorNotSupported;
-  int ntiles = 0;
-  const int2* tl = pair_tiles(a.np, st, &ntiles);
-  if (!tl || ntiles <= 0) return cudaErrorNotSupported;
+// The tensor maps of a paired launch with NB-column tiles.
+template <typename T, int EPI, bool ANTI, int NB>
+static bool pair_maps(const StepArgs& a, CUtensorMap (&m)[8]) {
   const int type = std::is_same<T, __nv_bfloat16>::value ? TMAP_BF16 : TMAP_F16;
-  CUtensorMap m[8];
+  const int bh = PairCfg<false, NB>::BH;
   if (!make_tmap_box(&m[0], a.A, a.np, a.np, a.np, type, tc::BM) ||
       !make_tmap_box(&m[1], a.A_lo, a.np, a.np, a.np, type, tc::BM) ||
-      !make_tmap_box(&m[2], a.B, a.np, a.np, a.np, type, tcq::BH) ||
-      !make_tmap_box(&m[3], a.B_lo, a.np, a.np, a.np, type, tcq::BH))
-    return cudaErrorInvalidValue;
-  if (ANTI) {
-    if (!make_tmap_box(&m[4], a.B, a.np, a.np, a.np, type, tc::BM) ||
-        !make_tmap_box(&m[5], a.B_lo, a.np, a.np, a.np, type, tc::BM) ||
-        !make_tmap_box(&m[6], a.A, a.np, a.np, a.np, type, tcq::BH) ||
-        !make_tmap_box(&m[7], a.A_lo, a.np, a.np, a.np, type, tcq::BH))
-      return cudaErrorInvalidValue;
+      !make_tmap_box(&m[2], a.B, a.np, a.np, a.np, type, bh) ||
+      !make_tmap_box(&m[3], a.B_lo, a.np, a.np, a.np, type, bh))
+    return false;
+  if constexpr (ANTI) {
+    return make_tmap_box(&m[4], a.B, a.np, a.np, a.np, type, tc::BM) &&
+           make_tmap_box(&m[5], a.B_lo, a.np, a.np, a.np, type, tc::BM) &&
+           make_tmap_box(&m[6], a.A, a.np, a.np, a.np, type, bh) &&
+           make_tmap_box(&m[7], a.A_lo, a.np, a.np, a.np, type, bh);
   } else {
     for (int i = 0; i < 4; ++i) m[4 + i] = m[i];   // unused
+    return true;
   }
-  // one tile per pair (a single wave): the X_k block staged for the epilogue (the
-  // shared-memory limit is raised before the residency query counts the clusters)
-  if (EPI == 0 && a.E == a.A && a.E_lo == a.A_lo && ntiles <= num_sms() / 2) {
-    auto kes = k_tc_pair<T, EPI, ANTI, true>;
-    if (cudaFuncSetAttribute(kes, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             tcq::SMEM_BYTES_ES) == cudaSuccess &&
-        ntiles <= pair_clusters<T, EPI, ANTI, true>()) {
-      kes<<<2 * ntiles, tcp::NTHR, tcq::SMEM_BYTES_ES, st>>>(m[0], m[1], m[2], m[3], m[4], m[5],
-                                                             m[6], m[7], a, tl, ntiles);
-      note_launch();
-      return cudaGetLastError();
-    }
+}
+
+// The single-wave form with the X_k block staged, if its tiles are all resident at once
+// (the shared-memory limit is raised before the residency query counts the clusters).
+template <typename T, int EPI, bool ANTI, int NB>
+static cudaError_t launch_pair_staged(const StepArgs& a, cudaStream_t st) {
+  const int blocks = pair_tile_count(a.np);
+  if (blocks * (128 / NB) > num_sms() / 2) return cudaErrorNotSupported;
+  int ntiles = 0;
+  const int2* tl = pair_tiles(a.np, NB == 64 ? 0 : blocks, false, st, &ntiles);
+  if (!tl || ntiles <= 0) return cudaErrorNotSupported;
+  auto kes = k_tc_pair<T, EPI, ANTI, true, NB>;
+  constexpr int smem = PairCfg<true, NB>::SMEM_BYTES;
+  if (cudaFuncSetAttribute(kes, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+      ntiles > pair_clusters<T, EPI, ANTI, true, NB>()) {
     (void)cudaGetLastError();
+    return cudaErrorNotSupported;
   }
-  auto kern = k_tc_pair<T, EPI, ANTI>;
-  cudaError_t e =
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, tcq::SMEM_BYTES);
-  if (e != cudaSuccess) return e;
-  const int clusters = std::min(ntiles, pair_clusters<T, EPI, ANTI>());
-  kern<<<2 * clusters, tcp::NTHR, tcq::SMEM_BYTES, st>>>(m[0], m[1], m[2], m[3], m[4], m[5], m[6],
-                                                         m[7], a, tl, ntiles);
+  CUtensorMap m[8];
+  if (!pair_maps<T, EPI, ANTI, NB>(a, m)) return cudaErrorInvalidValue;
+  kes<<<2 * ntiles, tcp::NTHR, smem, st>>>(m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7], a, tl,
+                                           ntiles);
   note_launch();
   return cudaGetLastError();
+}
+
+// The persistent form; the tiles past the first `whole` are cut in two (TAIL).
+template <typename T, int EPI, bool ANTI, bool TAIL>
+static cudaError_t launch_pair_grid(const StepArgs& a, int whole, cudaStream_t st) {
+  int ntiles = 0;
+  const int2* tl = pair_tiles(a.np, whole, TAIL, st, &ntiles);
+  if (!tl || ntiles <= 0) return cudaErrorNotSupported;
+  CUtensorMap m[8];
+  if (!pair_maps<T, EPI, ANTI, 128>(a, m)) return cudaErrorInvalidValue;
+  auto kern = k_tc_pair<T, EPI, ANTI, false, 128, TAIL>;
+  constexpr int smem = PairCfg<false, 128>::SMEM_BYTES;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  const int clusters = std::min(ntiles, pair_clusters<T, EPI, ANTI, false, 128, TAIL>());
+  kern<<<2 * clusters, tcp::NTHR, smem, st>>>(m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7], a, tl,
+                                              ntiles);
+  note_launch();
+  return cudaGetLastError();
+}
+
+constexpr int kTailWaves = 6;
+
+// Paired-CTA launch; returns cudaErrorNotSupported when the caller should use the
+// single-CTA kernel instead.  ANTI: A = G, B = X (see k_tc_pair).  A single wave takes the
+// staged form, with 64-column tiles when those too are one wave (np <= 1280; n = 1000: the
+// step 25 -> 18 us).  In that form np may be an odd multiple of 128: the second CTA of the
+// last row pair then loads zeros past the rows and owns no tile.  The others need np a
+// multiple of 256.
+template <typename T, int EPI, bool ANTI = false>
+static cudaError_t launch_pair(const StepArgs& a, cudaStream_t st) {
+  if (a.ld != a.np) return cudaErrorNotSupported;
+  const bool even = a.np % (2 * tc::BM) == 0;
+  if constexpr (EPI == 0) {
+    if (a.E == a.A && a.E_lo == a.A_lo) {
+      cudaError_t e = launch_pair_staged<T, EPI, ANTI, 64>(a, st);
+      if (e == cudaErrorNotSupported && even) e = launch_pair_staged<T, EPI, ANTI, 128>(a, st);
+      if (e != cudaErrorNotSupported) return e;
+    }
+  }
+  if (!even) return cudaErrorNotSupported;
+  // the tiles past the last whole wave, if they are at most half a wave: cut in two, that
+  // wave takes half the time (below kTailWaves waves, where it shows: n = 3072 3 -> 2.5)
+  const int blocks = pair_tile_count(a.np), rest = blocks % (num_sms() / 2);
+  const int waves = blocks / (num_sms() / 2);
+  if (waves > 0 && waves < kTailWaves && rest > 0 && 2 * rest <= num_sms() / 2)
+    return launch_pair_grid<T, EPI, ANTI, true>(a, blocks - rest, st);
+  return launch_pair_grid<T, EPI, ANTI, false>(a, blocks, st);
 }
 
 // Symmetric launches: A = B (the iterate), so one pair of tensor maps serves both.
@@ -1508,8 +1587,8 @@ cudaError_t launch_sym_gemm_tc(const StepArgs& a0, int bf16, cudaStream_t st) {
 }
 
 // {G, X} on the upper tiles, out = alpha {G, X} + beta E (E = G for the adjoint step):
-// a.A / a.A_lo = G, a.B / a.B_lo = X.  cudaErrorNotSupported when np is not a multiple
-// of 256 (the caller forms G X with launch_tc_plain and combines).
+// a.A / a.A_lo = G, a.B / a.B_lo = X.  cudaErrorNotSupported when np is above 1280 and not a
+// multiple of 256 (the caller forms G X with launch_tc_plain and combines).
 cudaError_t launch_anti_tc(const StepArgs& a0, cudaStream_t st) {
   if (a0.np % tc::BM != 0) return cudaErrorInvalidValue;
   StepArgs a = a0;

@@ -309,7 +309,7 @@ int sp2b_dev_adjoint_step_split(const void* g_hi, const void* g_lo, const void* 
     SP2B_CUDA_TRY(e);
     return SP2B_OK;
   }
-  // np not a multiple of 256: M = G X in FP32 (full product), then the split combine
+  // np above 1280 and not a multiple of 256: M = G X in FP32 (full product), then the split combine
   SP2B_CUDA_TRY(c->ensure_f64(np, 1));
   float* m = reinterpret_cast<float*>(c->x64[0]);
   SP2B_CUDA_TRY(launch_tc_plain((const __half*)g_hi, (const __half*)g_lo, (const __half*)x_hi,
