@@ -33,6 +33,7 @@
 // Entries at or beyond n64 only reach output rows at or beyond n64, which nothing reads.
 // Only the tiles' entries are stored (the upper band: row r from column r & ~127 on);
 // operand blocks left of it are read from their mirrors, transposed by the MMA.
+#include <climits>
 #include "kernels_subgraph.cuh"
 #include "reduce.cuh"
 #include "tc_ptx.cuh"
@@ -651,69 +652,70 @@ __device__ __forceinline__ void i8_store_x(int8_t* base, size_t plane, size_t id
   base[3 * plane + idx] = d3;
 }
 
-// CSR rows of each part straight to X0' = X0 - I/2 in digits (parts up to 512), with the
-// same row construction as the split extraction: one warp per row in shared memory.  The
-// row's digits are collected by plane in shared memory and leave as 16-byte stores.
+// CSR rows of each part straight to X0' = X0 - I/2 in digits (ld up to kFusedLd), with the
+// same row construction as the split extraction: one warp per row in shared memory, four
+// columns a lane, a plane's four digits leaving as one word.  M comes from the low word of
+// x 2^31 + 1.5 2^52 (one rounding to nearest even, like llrint, whose conversion of every
+// element, nearly all of them zero, took most of the pass).
 __global__ void __launch_bounds__(256) k_extract_digits(
     const long long* __restrict__ rp, const int* __restrict__ col, const double* __restrict__ val,
     const PartDesc* __restrict__ parts, const int* __restrict__ halo, const int* __restrict__ skey,
     const int* __restrict__ sval, int ld, long long rows, double emin, double emax,
     int8_t* __restrict__ dig) {
-  __shared__ double rowbuf[8][512];
-  __shared__ __align__(16) int8_t dbuf[8][4][512];
+  extern __shared__ __align__(16) double s_rows[];
+  int* keys = reinterpret_cast<int*>(s_rows + 8 * ld);
+  int* vals = keys + ld;
   const PartDesc P = parts[blockIdx.x];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const double mm = emax - emin;
   const double alpha = -1.0 / mm, beta = emax / mm;
   const int* hl = halo + P.hoff;
-  const int* sk = skey + P.hoff;
-  const int* sv = sval + P.hoff;
+  for (int i = threadIdx.x; i < P.n; i += blockDim.x) {
+    keys[i] = skey[P.hoff + i];
+    vals[i] = sval[P.hoff + i];
+  }
+  __syncthreads();
   const size_t plane = (size_t)rows * ld;
-  double* buf = rowbuf[warp];
+  double* buf = s_rows + warp * ld;
   for (int r = blockIdx.y * 8 + warp; r < P.np; r += gridDim.y * 8) {
-    for (int c = lane; c < P.np; c += 32) buf[c] = 0.0;
-    __syncwarp();
-    if (r < P.n) {
-      const int v = hl[r];
-      for (long long e = rp[v] + lane; e < rp[v + 1]; e += 32) {
-        const int u = col[e];
-        int a = 0, b = P.n - 1;
-        while (a <= b) {
-          const int mid = (a + b) >> 1;
-          const int key = sk[mid];
-          if (key == u) {
-            buf[sv[mid]] = val[e];
-            break;
-          }
-          if (key < u) a = mid + 1;
-          else b = mid - 1;
+    extract_row(rp, col, val, P, r < P.n ? hl[r] : -1, lane, keys, vals, buf);
+    const size_t ro = ((size_t)P.row0 + r) * ld;   // ld, np: multiples of 128
+    for (int c0 = lane * 4; c0 < P.np; c0 += 128) {
+      uint32_t w[4];   // an element's digits, d3 in the low byte
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int c = c0 + e;
+        // separate roundings (no contraction), so a host model forms the same X0'
+        double x = 0.0;
+        if (r < P.n && c < P.n) {
+          x = __dmul_rn(alpha, buf[c]);
+          if (r == c) x = __dadd_rn(x, beta);
+        }
+        if (r == c) x = __dadd_rn(x, -0.5);
+        const int m = x == x ? __double2loint(__dadd_rn(x * 0x1p31, 0x1.8p52)) : 0;
+        // the bytes of M + 0x808080 with the low three flipped (i8_digits clamps the top
+        // digit of an M that bounds not enclosing the spectrum put out of range)
+        w[e] = ((uint32_t)m + 0x808080u) ^ 0x808080u;
+        if (abs(m) >= 0x7f000000 || m == INT_MIN) {
+          int8_t d0, d1, d2, d3;
+          i8_digits(m, d0, d1, d2, d3);
+          w[e] = (uint32_t)(uint8_t)d0 << 24 | (uint32_t)(uint8_t)d1 << 16 |
+                 (uint32_t)(uint8_t)d2 << 8 | (uint8_t)d3;
         }
       }
+      // four elements' words to one word per plane
+      const uint32_t lo01 = __byte_perm(w[0], w[1], 0x5140), lo23 = __byte_perm(w[2], w[3], 0x5140);
+      const uint32_t hi01 = __byte_perm(w[0], w[1], 0x7362), hi23 = __byte_perm(w[2], w[3], 0x7362);
+      *reinterpret_cast<uint32_t*>(dig + ro + c0) = __byte_perm(hi01, hi23, 0x7632);
+      *reinterpret_cast<uint32_t*>(dig + plane + ro + c0) = __byte_perm(hi01, hi23, 0x5410);
+      *reinterpret_cast<uint32_t*>(dig + 2 * plane + ro + c0) = __byte_perm(lo01, lo23, 0x7632);
+      *reinterpret_cast<uint32_t*>(dig + 3 * plane + ro + c0) = __byte_perm(lo01, lo23, 0x5410);
     }
-    __syncwarp();
-    int8_t(*db)[512] = dbuf[warp];
-    for (int c = lane; c < P.np; c += 32) {
-      // separate roundings (no contraction), so a host model forms the same X0'
-      double x = 0.0;
-      if (r < P.n && c < P.n) {
-        x = __dmul_rn(alpha, buf[c]);
-        if (r == c) x = __dadd_rn(x, beta);
-      }
-      const int m = (int)llrint((r == c ? __dadd_rn(x, -0.5) : x) * 0x1p31);
-      i8_digits(m, db[0][c], db[1][c], db[2][c], db[3][c]);
-    }
-    __syncwarp();
-    const size_t ro = ((size_t)P.row0 + r) * ld;   // ld, np: multiples of 128
-    for (int c0 = lane * 16; c0 < P.np; c0 += 512)
-#pragma unroll
-      for (int d = 0; d < 4; ++d)
-        *reinterpret_cast<uint4*>(dig + d * plane + ro + c0) =
-            *reinterpret_cast<const uint4*>(&db[d][c0]);
     __syncwarp();
   }
 }
 
-// The same from the FP64 packed extraction (parts above 512): X0' digits of every
+// The same from the FP64 packed extraction (larger ld): X0' digits of every
 // packed element.
 __global__ void k_norm_digits(const double* __restrict__ xs, const int* __restrict__ row_part,
                               const PartDesc* __restrict__ parts, long long rows, int ld,
@@ -817,8 +819,12 @@ cudaError_t launch_extract_digits(const long long* rp, const int* col, const dou
                                   const PartDesc* parts, int nparts, const int* halo,
                                   const int* skey, const int* sval, int ld, long long rows,
                                   double emin, double emax, int8_t* dig, cudaStream_t st) {
-  if (ld > 512) return cudaErrorInvalidValue;
-  k_extract_digits<<<dim3(nparts, 16), 256, 0, st>>>(rp, col, val, parts, halo, skey, sval, ld,
+  if (ld > kFusedLd) return cudaErrorInvalidValue;
+  const size_t smem = extract_smem(ld);
+  const cudaError_t e =
+      cudaFuncSetAttribute(k_extract_digits, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  k_extract_digits<<<dim3(nparts, 16), 256, smem, st>>>(rp, col, val, parts, halo, skey, sval, ld,
                                                      rows, emin, emax, dig);
   note_launch();
   return cudaGetLastError();

@@ -91,7 +91,7 @@ __global__ void k_norm_parts(double* __restrict__ xs, const int* __restrict__ ro
   }
 }
 
-// Extraction and normalisation in one pass (parts up to 512): straight into the hi/lo
+// Extraction and normalisation in one pass (ld up to kFusedLd): straight into the hi/lo
 // split (split precisions, no FP64 packed block) or into the FP64 packed block, without
 // clearing it first.  Grid (part, row group); each warp builds one row of X0 at a
 // time in shared memory (zero, scatter the row's CSR entries found in the part's node
@@ -104,49 +104,47 @@ __global__ void __launch_bounds__(256) k_extract_split(
     const PartDesc* __restrict__ parts, const int* __restrict__ halo, const int* __restrict__ skey,
     const int* __restrict__ sval, int ld, double emin, double emax, T* __restrict__ hi,
     T* __restrict__ lo, double* __restrict__ xs) {
-  __shared__ double rowbuf[8][512];
+  extern __shared__ __align__(16) double s_rows[];
+  int* keys = reinterpret_cast<int*>(s_rows + 8 * ld);
+  int* vals = keys + ld;
   const PartDesc P = parts[blockIdx.x];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const double mm = emax - emin;
   const double alpha = -1.0 / mm, beta = emax / mm;
   const int* hl = halo + P.hoff;
-  const int* sk = skey + P.hoff;
-  const int* sv = sval + P.hoff;
-  double* buf = rowbuf[warp];
+  for (int i = threadIdx.x; i < P.n; i += blockDim.x) {
+    keys[i] = skey[P.hoff + i];
+    vals[i] = sval[P.hoff + i];
+  }
+  __syncthreads();
+  double* buf = s_rows + warp * ld;
   for (int r = blockIdx.y * 8 + warp; r < P.np; r += gridDim.y * 8) {
-    for (int c = lane; c < P.np; c += 32) buf[c] = 0.0;
-    __syncwarp();
-    if (r < P.n) {
-      const int v = hl[r];
-      for (long long e = rp[v] + lane; e < rp[v + 1]; e += 32) {
-        const int u = col[e];
-        int a = 0, b = P.n - 1;
-        while (a <= b) {
-          const int mid = (a + b) >> 1;
-          const int key = sk[mid];
-          if (key == u) {
-            buf[sv[mid]] = val[e];
-            break;
-          }
-          if (key < u) a = mid + 1;
-          else b = mid - 1;
-        }
-      }
-    }
-    __syncwarp();
+    extract_row(rp, col, val, P, r < P.n ? hl[r] : -1, lane, keys, vals, buf);
     const size_t ro = ((size_t)P.row0 + r) * ld;
-    for (int c = lane; c < P.np; c += 32) {
-      double x = 0.0;
-      if (r < P.n && c < P.n) {
-        x = alpha * buf[c];
-        if (r == c) x += beta;
+    for (int c0 = lane * 4; c0 < P.np; c0 += 128) {
+      double x4[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int c = c0 + e;
+        double x = 0.0;
+        if (r < P.n && c < P.n) {
+          x = alpha * buf[c];
+          if (r == c) x += beta;
+        }
+        x4[e] = x;
       }
       if (F64) {
-        xs[ro + c] = x;
+        *reinterpret_cast<double2*>(xs + ro + c0) = make_double2(x4[0], x4[1]);
+        *reinterpret_cast<double2*>(xs + ro + c0 + 2) = make_double2(x4[2], x4[3]);
       } else {
-        const T a = SplitOps<T>::from_d(x);
-        hi[ro + c] = a;
-        lo[ro + c] = SplitOps<T>::from_d((x - SplitOps<T>::to_d(a)) * SplitOps<T>::kScale);
+        struct alignas(8) T4 { T v[4]; } h, l;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          h.v[e] = SplitOps<T>::from_d(x4[e]);
+          l.v[e] = SplitOps<T>::from_d((x4[e] - SplitOps<T>::to_d(h.v[e])) * SplitOps<T>::kScale);
+        }
+        *reinterpret_cast<T4*>(hi + ro + c0) = h;
+        *reinterpret_cast<T4*>(lo + ro + c0) = l;
       }
     }
     __syncwarp();
@@ -158,20 +156,26 @@ cudaError_t launch_extract_split(const long long* rp, const int* col, const doub
                                  const int* skey, const int* sval, int ld, double emin,
                                  double emax, int prec, void* hi, void* lo, double* xs,
                                  cudaStream_t st) {
+  if (ld > kFusedLd) return cudaErrorInvalidValue;
   const dim3 grid(nparts, 16);
+  const size_t smem = extract_smem(ld);
+  auto run = [&](auto kern, auto* h, auto* l, double* x) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    kern<<<grid, 256, smem, st>>>(rp, col, val, parts, halo, skey, sval, ld, emin, emax, h, l, x);
+    return cudaGetLastError();
+  };
+  cudaError_t e;
   if (prec == SP2B_PREC_FP64)
-    k_extract_split<__half, true><<<grid, 256, 0, st>>>(rp, col, val, parts, halo, skey, sval, ld,
-                                                        emin, emax, nullptr, nullptr, xs);
+    e = run(k_extract_split<__half, true>, (__half*)nullptr, (__half*)nullptr, xs);
   else if (prec == SP2B_PREC_MIXED_BF16)
-    k_extract_split<__nv_bfloat16, false><<<grid, 256, 0, st>>>(
-        rp, col, val, parts, halo, skey, sval, ld, emin, emax, (__nv_bfloat16*)hi,
-        (__nv_bfloat16*)lo, nullptr);
+    e = run(k_extract_split<__nv_bfloat16, false>, (__nv_bfloat16*)hi, (__nv_bfloat16*)lo,
+            (double*)nullptr);
   else
-    k_extract_split<__half, false><<<grid, 256, 0, st>>>(rp, col, val, parts, halo, skey, sval, ld,
-                                                         emin, emax, (__half*)hi, (__half*)lo,
-                                                         nullptr);
+    e = run(k_extract_split<__half, false>, (__half*)hi, (__half*)lo, (double*)nullptr);
   note_launch();
-  return cudaGetLastError();
+  return e;
 }
 
 // rho (core rows) = 2 X: packed per-part output and, optionally, a dense n x n

@@ -26,8 +26,9 @@ cudaError_t launch_scatter_parts(const double* x64, const void* hi, const void* 
                                  const PartDesc* parts, int nparts, const int* halo, int ld,
                                  double* core_out, double* dense, long long n, cudaStream_t st);
 
-// CSR extraction and normalisation with the global bounds in one pass (np <= 512 per
-// part): split precisions into the packed hi/lo buffers, FP64 into xs.
+// CSR extraction and normalisation with the global bounds in one pass (ld <= kFusedLd):
+// split precisions into the packed hi/lo buffers, FP64 into xs.
+constexpr int kFusedLd = 2048;   // eight rows and the node list of a part in shared memory
 cudaError_t launch_extract_split(const long long* rp, const int* col, const double* val,
                                  const PartDesc* parts, int nparts, const int* halo,
                                  const int* skey, const int* sval, int ld, double emin,
@@ -92,5 +93,35 @@ cudaError_t launch_scatter_digits(const int8_t* dig, long long rows, const PartD
                                   double* dense, long long n, cudaStream_t st);
 cudaError_t launch_part_idem_digits(const int8_t* dig, long long rows, const PartDesc* parts,
                                     int nparts, int ld, double* out, cudaStream_t st);
+
+// One warp of the fused extractions: row r of part P as FP64 entries of H in buf[0, np)
+// (zero where the CSR row has none or its column is outside the part).  keys / vals: the
+// part's sorted node list and local positions, in shared memory (a binary search there
+// costs nine shared-memory reads instead of nine dependent trips to L2).
+__device__ __forceinline__ void extract_row(const long long* __restrict__ rp,
+                                            const int* __restrict__ col,
+                                            const double* __restrict__ val, const PartDesc& P,
+                                            int node, int lane, const int* keys, const int* vals,
+                                            double* buf) {
+  for (int c = lane * 2; c < P.np; c += 64) *reinterpret_cast<double2*>(buf + c) = make_double2(0.0, 0.0);
+  __syncwarp();
+  if (node >= 0)
+    for (long long e = rp[node] + lane; e < rp[node + 1]; e += 32) {
+      const int u = col[e];
+      int a = 0, b = P.n - 1;
+      while (a <= b) {
+        const int mid = (a + b) >> 1;
+        const int key = keys[mid];
+        if (key == u) {
+          buf[vals[mid]] = val[e];
+          break;
+        }
+        if (key < u) a = mid + 1;
+        else b = mid - 1;
+      }
+    }
+  __syncwarp();
+}
+constexpr size_t extract_smem(int ld) { return (size_t)ld * (8 * sizeof(double) + 2 * sizeof(int)); }
 
 }  // namespace sp2b

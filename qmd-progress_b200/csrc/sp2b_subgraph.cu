@@ -344,8 +344,8 @@ static int batched_solve(Ctx* c, SubBufs& b, const SubJob& j, cudaStream_t st,
 
   // ---- device buffers ----
   const size_t packed = (size_t)rows * ld;
-  // parts up to 512: CSR straight to X0 (split: hi/lo, no FP64 block; FP64: no clearing)
-  const bool fused = ld <= 512;
+  // CSR straight to X0 (split: hi/lo, no FP64 block; FP64: no clearing)
+  const bool fused = ld <= kFusedLd;
   if ((!split && !dig) || !fused) SP2B_CUDA_TRY(grow_buf(b.xs, b.xs_cap, packed));
   if (split) {
     for (int i = 0; i < 2; ++i) {
