@@ -953,7 +953,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tcp::NTHR, 1)
               const __grid_constant__ CUtensorMap tm_bhi, const __grid_constant__ CUtensorMap tm_blo,
               const __grid_constant__ CUtensorMap tm_a2hi, const __grid_constant__ CUtensorMap tm_a2lo,
               const __grid_constant__ CUtensorMap tm_b2hi, const __grid_constant__ CUtensorMap tm_b2lo,
-              const StepArgs p, const int2* __restrict__ ptiles, int ntiles) {
+              const StepArgs p, const int2* __restrict__ ptiles, int ntiles_in) {
   using Q = PairCfg<ES, NB>;
   constexpr int ST = Q::ST;   // operand stages
   extern __shared__ uint8_t smem_raw[];
@@ -967,25 +967,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tcp::NTHR, 1)
   __shared__ double red[32 * 4];
   __shared__ int s_flag;
   __shared__ volatile int s_abort;
-  if (ES && ntiles > (int)(gridDim.x >> 1)) {        // one tile per pair (uniform exit)
-    if (threadIdx.x == 0 && p.err) atomicExch(p.err, 1);
-    return;
-  }
-
-  double alpha = p.alpha, beta = p.beta;
-  if (EPI == 0 && p.control) {
-    // the decision is the same in every CTA, so both CTAs of a pair leave together
-    const int br = control_prologue(p);
-    if (br < 0) return;
-    if (br == BR_X2) { alpha = 1.0; beta = 0.0; }
-    else { alpha = -1.0; beta = 2.0; }
-  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const uint32_t sbase = smem_u32(smem);
+  // Everything up to grid_wait() touches nothing of the launch before (the next step of a
+  // chain is launched while this one runs and gets this far on SMs it leaves free).
+  grid_launch_dependents();
   if (threadIdx.x == 0) {
     s_abort = 0;
     for (int s = 0; s < ST; ++s) {
@@ -1004,6 +994,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tcp::NTHR, 1)
   tc_fence_before();
   cluster_sync();   // barriers and TMEM of both CTAs exist before either uses the other's
   tc_fence_after();
+  grid_wait();      // the launch before has completed
+  double alpha = p.alpha, beta = p.beta;
+  bool run = true;
+  if (ES && ntiles_in > (int)(gridDim.x >> 1)) {     // one tile per pair (uniform)
+    if (threadIdx.x == 0 && p.err) atomicExch(p.err, 1);
+    run = false;
+  } else if (EPI == 0 && p.control) {
+    // the decision is the same in every CTA, so both CTAs of a pair agree; a launch with
+    // nothing to do has no tiles and publishes nothing
+    const int br = control_prologue(p);
+    run = br >= 0;
+    if (br == BR_X2) { alpha = 1.0; beta = 0.0; }
+    else { alpha = -1.0; beta = 2.0; }
+  }
+  const int ntiles = run ? ntiles_in : 0;
   const uint32_t tmem = tmem_holder;
   const int KB = p.np / tc::BK;
   const int KBT = ANTI ? 2 * KB : KB;   // K-blocks per tile
@@ -1148,6 +1153,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tcp::NTHR, 1)
   tc_fence_after();
   if (warp == 1) tmem_dealloc_pair(tmem, tcp::TMEM_COLS);
   if (s_abort && threadIdx.x == 0 && p.err) atomicExch(p.err, 1);
+  if (!run) return;
   if (p.out) __threadfence();
   publish_and_finalize(p, sums, red, &s_flag);
 }
@@ -1500,6 +1506,29 @@ static bool pair_maps(const StepArgs& a, CUtensorMap (&m)[8]) {
   }
 }
 
+// A paired launch that may start before the launch ahead of it in the stream has completed
+// (programmatic dependent launch): the kernel waits for it (grid_wait) before it reads or
+// writes anything, after its barriers, TMEM and cluster are set up.
+template <typename K>
+static cudaError_t launch_chained(K kern, int grid, int smem, cudaStream_t st,
+                                  const CUtensorMap (&m)[8], const StepArgs& a, const int2* tl,
+                                  int ntiles) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid, 1, 1);
+  cfg.blockDim = dim3(tcp::NTHR, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7],
+                                           a, tl, ntiles);
+  note_launch();
+  return e;
+}
+
 // The single-wave form with the X_k block staged, if its tiles are all resident at once
 // (the shared-memory limit is raised before the residency query counts the clusters).
 template <typename T, int EPI, bool ANTI, int NB>
@@ -1518,10 +1547,7 @@ static cudaError_t launch_pair_staged(const StepArgs& a, cudaStream_t st) {
   }
   CUtensorMap m[8];
   if (!pair_maps<T, EPI, ANTI, NB>(a, m)) return cudaErrorInvalidValue;
-  kes<<<2 * ntiles, tcp::NTHR, smem, st>>>(m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7], a, tl,
-                                           ntiles);
-  note_launch();
-  return cudaGetLastError();
+  return launch_chained(kes, 2 * ntiles, smem, st, m, a, tl, ntiles);
 }
 
 // The persistent form; the tiles past the first `whole` are cut in two (TAIL).
@@ -1537,10 +1563,7 @@ static cudaError_t launch_pair_grid(const StepArgs& a, int whole, cudaStream_t s
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   const int clusters = std::min(ntiles, pair_clusters<T, EPI, ANTI, false, 128, TAIL>());
-  kern<<<2 * clusters, tcp::NTHR, smem, st>>>(m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7], a, tl,
-                                              ntiles);
-  note_launch();
-  return cudaGetLastError();
+  return launch_chained(kern, 2 * clusters, smem, st, m, a, tl, ntiles);
 }
 
 constexpr int kTailWaves = 6;
