@@ -65,15 +65,17 @@ def _check_input(h: torch.Tensor):
 
 
 def _forward_steps(x, pp, checkpoint, n):
-    """Split X_K from split X_0 (consumed), keeping X_k every `checkpoint` steps:
-    (X_K, checkpoints)."""
-    ckpts = [x.clone()]
-    y = torch.empty_like(x)
+    """Split X_K from split X_0, keeping X_k every `checkpoint` steps: (X_K, checkpoints).
+    A checkpoint is the iterate itself; the next step writes another buffer."""
+    ckpts = [x]
+    spare = None
     for k, b in enumerate(pp):
+        y = torch.empty_like(x) if spare is None else spare
         _step(x, y, b, n)
-        x, y = y, x
+        spare = None if x is ckpts[-1] else x
+        x = y
         if (k + 1) % checkpoint == 0 and k + 1 < len(pp):
-            ckpts.append(x.clone())
+            ckpts.append(x)
     return x, ckpts
 
 
