@@ -745,15 +745,23 @@ __device__ __forceinline__ size_t i8_band_off(long long row0, int r, int c, int 
   return c >= (r & ~(i8s::BM - 1)) ? ((size_t)row0 + r) * ld + c : ((size_t)row0 + c) * ld + r;
 }
 
-// rho (core rows) = 2 X = 2^-30 M + I; one warp per core row, the lanes along it.
-__global__ void k_scatter_digits(const int8_t* __restrict__ dig, long long rows,
-                                 const PartDesc* __restrict__ parts, const int* __restrict__ halo,
-                                 int ld, double* __restrict__ core_out, double* __restrict__ dense,
-                                 long long n) {
+// rho (core rows) = 2 X = 2^-30 M + I; one warp per core row, the lanes along it.  With
+// `idem`, also the part's sum over core rows of (X - X^2)_ii = X_ii - sum_j X_ij^2 (the
+// flags of the FP64 re-solve), one partial per row group: the same digits, which a pass of
+// its own read again (43 us on the 32^3 lattice).  Columns j < n only: past the part size X
+// is zero off the diagonal, and past the tiles' columns (the part size rounded up to 64) the
+// iterated buffer holds entries no step writes.
+__global__ void __launch_bounds__(256)
+    k_scatter_digits(const int8_t* __restrict__ dig, long long rows,
+                     const PartDesc* __restrict__ parts, const int* __restrict__ halo, int ld,
+                     double* __restrict__ core_out, double* __restrict__ dense, long long n,
+                     double* __restrict__ idem) {
+  __shared__ double red[32];
   const PartDesc P = parts[blockIdx.x];
   const int* hl = halo + P.hoff;
   const size_t plane = (size_t)rows * ld;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  double s[1] = {0.0};
   for (int r = blockIdx.y * nw + warp; r < P.ncore; r += gridDim.y * nw) {
     double* co = core_out ? core_out + P.coff + (size_t)r * P.n : nullptr;
     for (int c = lane; c < P.n; c += 32) {
@@ -762,57 +770,14 @@ __global__ void k_scatter_digits(const int8_t* __restrict__ dig, long long rows,
       const double v = (double)m * 0x1p-30 + (r == c ? 1.0 : 0.0);
       if (co) co[c] = v;
       if (dense) dense[(size_t)hl[r] + (size_t)hl[c] * n] = v;
+      const double x = 0.5 * v;
+      s[0] = fma(-x, x, s[0]);
+      if (r == c) s[0] += x;
     }
   }
-}
-
-// Sum over each part's core rows of (X - X^2)_ii = X_ii - sum_j X_ij^2, from the digits
-// (upper-band storage).  Columns j < n only: past the part size X is zero off the
-// diagonal, and past the tiles' columns (the part size rounded up to 64) the iterated
-// buffer holds entries no step writes.
-__global__ void k_part_idem_digits(const int8_t* __restrict__ dig, long long rows,
-                                   const PartDesc* __restrict__ parts, int ld,
-                                   double* __restrict__ out) {
-  __shared__ double red[32];
-  const PartDesc P = parts[blockIdx.x];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  const size_t plane = (size_t)rows * ld;
-  double s = 0.0;
-  for (int r = blockIdx.y * nw + warp; r < P.ncore; r += gridDim.y * nw) {
-    const size_t row = ((size_t)P.row0 + r) * ld;
-    // columns left of the row's block from their mirrors (off the diagonal)
-    const int rb = r & ~(i8s::BM - 1);
-    for (int c = lane; c < rb; c += 32) {
-      const size_t o = ((size_t)P.row0 + c) * ld + r;
-      const double x = (double)i8_value(dig[o], dig[plane + o], dig[2 * plane + o], dig[3 * plane + o]) *
-                       0x1p-31;
-      s -= x * x;
-    }
-    for (int c0 = rb + lane * 16; c0 < P.n; c0 += 512) {
-      uint4 v[4];
-#pragma unroll
-      for (int d = 0; d < 4; ++d) v[d] = *reinterpret_cast<const uint4*>(dig + d * plane + row + c0);
-      const int8_t* b0 = reinterpret_cast<const int8_t*>(&v[0]);
-      const int8_t* b1 = reinterpret_cast<const int8_t*>(&v[1]);
-      const int8_t* b2 = reinterpret_cast<const int8_t*>(&v[2]);
-      const int8_t* b3 = reinterpret_cast<const int8_t*>(&v[3]);
-#pragma unroll
-      for (int e = 0; e < 16; ++e) {
-        const double x = (double)i8_value(b0[e], b1[e], b2[e], b3[e]) * 0x1p-31 +
-                         (c0 + e == r ? 0.5 : 0.0);
-        s -= x * x;
-        if (c0 + e == r) s += x;
-      }
-    }
-  }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) red[warp] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < nw; ++w) t += red[w];
-    out[(size_t)blockIdx.x * gridDim.y + blockIdx.y] = t;
-  }
+  if (!idem) return;
+  block_sum<1>(s, red);
+  if (threadIdx.x == 0) idem[(size_t)blockIdx.x * gridDim.y + blockIdx.y] = s[0];
 }
 
 cudaError_t launch_extract_digits(const long long* rp, const int* col, const double* val,
@@ -842,16 +807,9 @@ cudaError_t launch_norm_digits(const double* xs, const int* row_part, const Part
 
 cudaError_t launch_scatter_digits(const int8_t* dig, long long rows, const PartDesc* parts,
                                   int nparts, const int* halo, int ld, double* core_out,
-                                  double* dense, long long n, cudaStream_t st) {
-  k_scatter_digits<<<dim3(nparts, 16), 256, 0, st>>>(dig, rows, parts, halo, ld, core_out, dense,
-                                                     n);
-  note_launch();
-  return cudaGetLastError();
-}
-
-cudaError_t launch_part_idem_digits(const int8_t* dig, long long rows, const PartDesc* parts,
-                                    int nparts, int ld, double* out, cudaStream_t st) {
-  k_part_idem_digits<<<dim3(nparts, kPartIdemGroups), 256, 0, st>>>(dig, rows, parts, ld, out);
+                                  double* dense, long long n, double* idem, cudaStream_t st) {
+  k_scatter_digits<<<dim3(nparts, kPartIdemGroups), 256, 0, st>>>(dig, rows, parts, halo, ld,
+                                                                  core_out, dense, n, idem);
   note_launch();
   return cudaGetLastError();
 }

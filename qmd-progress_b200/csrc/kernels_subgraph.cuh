@@ -90,9 +90,7 @@ cudaError_t launch_norm_digits(const double* xs, const int* row_part, const Part
                                cudaStream_t st);
 cudaError_t launch_scatter_digits(const int8_t* dig, long long rows, const PartDesc* parts,
                                   int nparts, const int* halo, int ld, double* core_out,
-                                  double* dense, long long n, cudaStream_t st);
-cudaError_t launch_part_idem_digits(const int8_t* dig, long long rows, const PartDesc* parts,
-                                    int nparts, int ld, double* out, cudaStream_t st);
+                                  double* dense, long long n, double* idem, cudaStream_t st);
 
 // One warp of the fused extractions: row r of part P as FP64 entries of H in buf[0, np)
 // (zero where the CSR row has none or its column is outside the part).  keys / vals: the

@@ -569,12 +569,8 @@ static int batched_solve(Ctx* c, SubBufs& b, const SubJob& j, cudaStream_t st,
       }
       const int fb = maxiter & 1;
       if (dig) {
-        if ((e = launch_scatter_digits(b.dig[fb], rows, b.parts, nparts, b.halo, ld, core_d,
-                                       dense_d, n, cap)) != cudaSuccess)
-          return e;
-        if (idem)
-          return launch_part_idem_digits(b.dig[fb], rows, b.parts, nparts, ld, b.idem, cap);
-        return cudaSuccess;
+        return launch_scatter_digits(b.dig[fb], rows, b.parts, nparts, b.halo, ld, core_d, dense_d,
+                                     n, idem ? b.idem : nullptr, cap);
       }
       if ((e = launch_scatter_parts(fb ? b.x2 : b.xs, split ? (void*)b.hi[fb] : nullptr,
                                     split ? (void*)b.lo[fb] : nullptr, prec, b.parts, nparts,
@@ -603,7 +599,8 @@ static int batched_solve(Ctx* c, SubBufs& b, const SubJob& j, cudaStream_t st,
   }
   cudaError_t le = cudaGraphLaunch(exec, st);
   // extract, normalise, the steps (FP64, INT8: one persistent launch and its sums), scatter
-  note_launch((split ? maxiter : maxiter > 0 ? 2 : 0) + (fused ? 1 : 2) + 1 + (idem ? 1 : 0));
+  note_launch((split ? maxiter : maxiter > 0 ? 2 : 0) + (fused ? 1 : 2) + 1 +
+              (idem && split ? 1 : 0));
   if (le != cudaSuccess) {
     set_last_error("graph launch failed: %s", cudaGetErrorString(le));
     return SP2B_CUDA_ERROR;
