@@ -29,6 +29,7 @@ struct F64Tile {
   static constexpr int WM = BT == 32 ? 2 : 4, WN = 4, NW = WM * WN, NT = NW * 32;
   static constexpr int ST = BT == 128 ? 6 : 8;
   static constexpr int TM = BT / WM, TN = BT / WN, MI = TM / 8, NI = TN / 8;
+  static constexpr bool EARLY_E = BT == 32;   // registers for the epilogue's operand
   static constexpr int OPERAND = BT * BK * 8, STAGE = 2 * OPERAND;   // bytes
   static constexpr size_t SMEM = (size_t)ST * STAGE + 1024;
 
@@ -96,6 +97,13 @@ struct F64Tile {
   }
 };
 
+__device__ __forceinline__ void prefetch_tmap(const CUtensorMap* tm) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tm)) : "memory");
+}
+// Adds one to a counter after everything this thread has done or seen (gpu scope).
+__device__ __forceinline__ void add_release(unsigned* word) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(word) : "memory");
+}
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* tm, uint32_t mbar,
                                             int x, int y, int z) {
   asm volatile(

@@ -58,6 +58,8 @@ __global__ void __launch_bounds__(F64Tile<BT>::NT + 32, BT == 32 ? 2 : 1)
   if (warp == C::NW) {
     // ---------------- loader ----------------
     if (lane == 0) {
+      prefetch_tmap(&maps.x[0]);
+      prefetch_tmap(&maps.x[1]);
       uint32_t g = 0;
       bool ok = true;
       while (ok) {
@@ -134,6 +136,18 @@ __global__ void __launch_bounds__(F64Tile<BT>::NT + 32, BT == 32 ? 2 : 1)
     for (int mi = 0; mi < C::MI; ++mi)
 #pragma unroll
       for (int ni = 0; ni < C::NI; ++ni) acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
+    const size_t base = (size_t)tl.x * ld;
+    const double* E = ((k & 1) ? p.x[1] : p.x[0]) + base;
+    // E of the tile: read ahead of the products where the registers allow
+    double2 ev[C::EARLY_E ? C::MI : 1][C::EARLY_E ? C::NI : 1];
+    if (C::EARLY_E) {
+#pragma unroll
+      for (int mi = 0; mi < C::MI; ++mi)
+#pragma unroll
+        for (int ni = 0; ni < C::NI; ++ni)
+          ev[mi][ni] = __ldcg(reinterpret_cast<const double2*>(
+              E + (size_t)(bi * BT + C::row(mi)) * ld + bj * BT + C::col(ni)));
+    }
     bool ok = true;
     for (int kk = 0; kk < tl.z; kk += C::BK, ++g) {
       const int st = g % C::ST;
@@ -148,16 +162,16 @@ __global__ void __launch_bounds__(F64Tile<BT>::NT + 32, BT == 32 ? 2 : 1)
     // out = alpha acc + beta E, mirrored store, the residual over the part's core rows
     const bool sq = p.pp[k] != 0;
     const double alpha = sq ? 1.0 : -1.0, beta = sq ? 0.0 : 2.0;
-    const size_t base = (size_t)tl.x * ld;
-    const double* E = p.x[k & 1] + base;
-    double* out = p.x[(k + 1) & 1] + base;
+    double* out = ((k & 1) ? p.x[0] : p.x[1]) + base;
     double res = 0.0;
 #pragma unroll
     for (int mi = 0; mi < C::MI; ++mi) {
 #pragma unroll
       for (int ni = 0; ni < C::NI; ++ni) {
         const int r = bi * BT + C::row(mi), c = bj * BT + C::col(ni);
-        const double2 e = __ldcg(reinterpret_cast<const double2*>(E + (size_t)r * ld + c));
+        const double2 e = C::EARLY_E
+                              ? ev[C::EARLY_E ? mi : 0][C::EARLY_E ? ni : 0]
+                              : __ldcg(reinterpret_cast<const double2*>(E + (size_t)r * ld + c));
         const double a0 = acc[mi][ni][0], a1 = acc[mi][ni][1];
         const double v0 = alpha * a0 + beta * e.x;
         const double v1 = alpha * a1 + beta * e.y;
@@ -175,10 +189,9 @@ __global__ void __launch_bounds__(F64Tile<BT>::NT + 32, BT == 32 ? 2 : 1)
       }
     }
     fence_proxy_async_global();   // these stores, then the other CTAs' TMA reads
-    __threadfence();
+    // (the barrier and the release order the whole block's stores)
     asm volatile("bar.sync 1, %0;" ::"n"(C::NT) : "memory");
-    if (tid == 0)
-      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.done + p.tpart[t]) : "memory");
+    if (tid == 0) add_release(p.done + p.tpart[t]);
     if (p.partials) {
       res = warp_sum(res);
       if (lane == 0) p.partials[(size_t)item * C::NW + warp] = res;

@@ -169,6 +169,7 @@ __global__ void __launch_bounds__(F64Tile<BT>::NT + 32, 1)
     }
   }
   __syncthreads();
+  if (warp == C::NW && lane < 4) prefetch_tmap(lane < 2 ? &maps.x[lane] : &maps.d[lane - 2]);
   typename C::Frag frag;
   frag.init(lane);
   uint32_t g = 0;   // units loaded (loader) or consumed so far, over all steps
@@ -235,6 +236,17 @@ __global__ void __launch_bounds__(F64Tile<BT>::NT + 32, 1)
         for (int mi = 0; mi < C::MI; ++mi)
 #pragma unroll
           for (int ni = 0; ni < C::NI; ++ni) acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
+        // E of the tile: read ahead of the products where the registers allow
+        const double* E = isx ? p.x[k & 1] : p.d[k & 1];
+        double2 ev[C::EARLY_E ? C::MI : 1][C::EARLY_E ? C::NI : 1];
+        if (C::EARLY_E) {
+#pragma unroll
+          for (int mi = 0; mi < C::MI; ++mi)
+#pragma unroll
+            for (int ni = 0; ni < C::NI; ++ni)
+              ev[mi][ni] = __ldcg(reinterpret_cast<const double2*>(
+                  E + (size_t)(bi * BT + C::row(mi)) * ld + bj * BT + C::col(ni)));
+        }
         // X Delta and Delta X are summed apart (one chain of 2 n terms has more rounding
         // error than two of n): the first waits in shared memory
         const bool both = !isx && k0 < p.kb && k1 > p.kb;
@@ -273,7 +285,6 @@ __global__ void __launch_bounds__(F64Tile<BT>::NT + 32, 1)
 #pragma unroll
             for (int ni = 0; ni < C::NI; ++ni)
               w[(mi * C::NI + ni) * C::NT] = make_double2(acc[mi][ni][0], acc[mi][ni][1]);
-          __threadfence();
           consumer_sync<C::NT>();
           if (tid == 0)
             asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p.flags + cta),
@@ -301,14 +312,15 @@ __global__ void __launch_bounds__(F64Tile<BT>::NT + 32, 1)
           }
         }
         // out = alpha acc + beta E, mirrored store, FP64 sums (of X, and Tr Delta')
-        const double* E = isx ? p.x[k & 1] : p.d[k & 1];
         double* out = isx ? p.x[(k + 1) & 1] : p.d[(k + 1) & 1];
 #pragma unroll
         for (int mi = 0; mi < C::MI; ++mi) {
 #pragma unroll
           for (int ni = 0; ni < C::NI; ++ni) {
             const int r = bi * BT + C::row(mi), c = bj * BT + C::col(ni);
-            const double2 e = __ldcg(reinterpret_cast<const double2*>(E + (size_t)r * ld + c));
+            const double2 e = C::EARLY_E
+                                  ? ev[C::EARLY_E ? mi : 0][C::EARLY_E ? ni : 0]
+                                  : __ldcg(reinterpret_cast<const double2*>(E + (size_t)r * ld + c));
             const double a0 = acc[mi][ni][0], a1 = acc[mi][ni][1];
             const double v0 = alpha * a0 + beta * e.x;
             const double v1 = alpha * a1 + beta * e.y;
@@ -341,7 +353,6 @@ __global__ void __launch_bounds__(F64Tile<BT>::NT + 32, 1)
         }
       }
       fence_proxy_async_global();   // these stores, then the other CTAs' TMA reads
-      __threadfence();
     }
 
     // ---- grid barrier, the step's sums and the next decision ----
@@ -356,9 +367,9 @@ __global__ void __launch_bounds__(F64Tile<BT>::NT + 32, 1)
       for (int q = 0; q < kSums; ++q) s[q] = warp_sum(lane < C::NW ? s_red[q][lane] : 0.0);
     }
     if (tid == 0) {
+      // (the barrier above and this release order the whole block's stores)
       for (int q = 0; q < kSums; ++q) part[(size_t)q * G + cta] = s[q];
-      __threadfence();
-      atomicAdd(p.bar, 1u);
+      add_release(p.bar);
       if (!s_abort && !spin_until(p.bar, (unsigned)G * (unsigned)(k + 1 - p.k0), p.err)) s_abort = 1;
       if (s_abort) {
         // the call reports SP2B_TIMEOUT; the other CTAs leave at their next wait
@@ -367,7 +378,6 @@ __global__ void __launch_bounds__(F64Tile<BT>::NT + 32, 1)
         __threadfence();
         p.sout->done = 1;
       }
-      __threadfence();
     }
     __syncthreads();
     if (s_abort) {
