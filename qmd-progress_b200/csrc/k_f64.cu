@@ -303,6 +303,29 @@ cudaError_t launch_finish_f64(const double* x, int np, int n, double scale, doub
   return cudaGetLastError();
 }
 
+__global__ void k_finish_solve_f64(const double* __restrict__ x0, const double* __restrict__ x1,
+                                   const SolveOut* __restrict__ sout,
+                                   const double* __restrict__ norm, int np, int n,
+                                   double* __restrict__ rho, int ld) {
+  // (each test is false for a NaN; an infinite norm fails the last)
+  if (!sout->done || !(norm[1] - norm[0] > 0.0) || !(norm[3] <= 1e300)) return;
+  const double* __restrict__ x = (sout->nupd & 1) ? x1 : x0;
+  const size_t total = (size_t)n * n;
+  for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
+       idx += (size_t)gridDim.x * blockDim.x) {
+    const int r = (int)(idx / n), c = (int)(idx % n);
+    rho[(size_t)r * ld + c] = 2.0 * x[(size_t)r * np + c];
+  }
+}
+
+cudaError_t launch_finish_solve_f64(const double* x0, const double* x1, const SolveOut* sout,
+                                    const double* norm, int np, int n, double* rho, int ld,
+                                    cudaStream_t st) {
+  k_finish_solve_f64<<<elem_grid(np), 256, 0, st>>>(x0, x1, sout, norm, np, n, rho, ld);
+  note_launch();
+  return cudaGetLastError();
+}
+
 // ------------------------------------------------------------------------------------
 // Symmetric-tile FP64 product with the SP2 epilogue.
 // One CTA per upper tile (bi <= bj) of BT x BT; WM x WN warps, each owning a

@@ -912,18 +912,16 @@ cudaError_t launch_oz_crt_step(const uint8_t* q, const void* scale, const StepAr
   return cudaGetLastError();
 }
 
-// Reads back the scale exponent and the largest squared row norm (diagnostics / checks).
-cudaError_t oz_read_scale(const void* scale, int* S, double* r2max, cudaStream_t st) {
+// Scale exponent and largest squared row norm (diagnostics / checks): queued into pinned
+// memory of oz_scale_bytes(), read after the caller's wait.
+cudaError_t oz_copy_scale(const void* scale, void* pinned, cudaStream_t st) {
+  return cudaMemcpyAsync(pinned, scale, sizeof(OzScale), cudaMemcpyDeviceToHost, st);
+}
+void oz_scale_values(const void* pinned, int* S, double* r2max) {
   OzScale h;
-  cudaError_t e = cudaMemcpyAsync(&h, scale, sizeof(h), cudaMemcpyDeviceToHost, st);
-  if (e != cudaSuccess) return e;
-  if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
+  memcpy(&h, pinned, sizeof(h));
   *S = h.S;
-  unsigned long long b = h.r2max_bits;
-  double d;
-  memcpy(&d, &b, sizeof(d));
-  *r2max = d;
-  return cudaSuccess;
+  memcpy(r2max, &h.r2max_bits, sizeof(double));
 }
 
 }  // namespace sp2b

@@ -18,6 +18,7 @@ struct SolveOut {
   int nupd;     // number of X updates applied (final X lives in buffer nupd & 1)
   int status;   // SP2B_* code
   int iter;     // Fortran iteration count ("icount")
+  double err;   // ALGO_MIXED: Tr X - Tr P of the last update (its stop reason)
 };
 
 // Arguments of one symmetric-tile product launch (FP64 or split precision).
@@ -104,6 +105,12 @@ cudaError_t launch_f64_solve(const F64SolveArgs& a, int n, int np, double* work,
 
 cudaError_t launch_finish_f64(const double* x, int np, int n, double scale, double* rho,
                               int ld, cudaStream_t st);
+// rho = 2 X of the iterate that a finished solve left in x[nupd & 1], chosen on the device;
+// nothing when the solve has not ended or its normalisation (norm: bounds, trace,
+// ||X0||_F^2) was not finite.
+cudaError_t launch_finish_solve_f64(const double* x0, const double* x1, const SolveOut* sout,
+                                    const double* norm, int np, int n, double* rho, int ld,
+                                    cudaStream_t st);
 cudaError_t launch_copy_in(const double* src, int n, int ld, int np, double* x,
                            cudaStream_t st);
 cudaError_t launch_mirror_lower(double* a, int n, int ld, cudaStream_t st);
@@ -165,7 +172,8 @@ cudaError_t launch_oz_crt_step(const uint8_t* q, const void* scale, const StepAr
 cudaError_t launch_oz_crt(const uint8_t* q, const __half* xhi, const __half* xlo, int np,
                           int bf16, const void* scale, double* x2, __half* rhi, __half* rlo,
                           cudaStream_t st);
-cudaError_t oz_read_scale(const void* scale, int* S, double* r2max, cudaStream_t st);
+cudaError_t oz_copy_scale(const void* scale, void* pinned, cudaStream_t st);
+void oz_scale_values(const void* pinned, int* S, double* r2max);
 cudaError_t launch_tc_plain(const __half* ahi, const __half* alo, const __half* bhi,
                             const __half* blo, int np, float* c, int n, cudaStream_t st,
                             int* err);

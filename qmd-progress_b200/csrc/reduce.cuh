@@ -83,6 +83,7 @@ __device__ inline void publish_and_finalize(const StepArgs& p, double (&s)[4], d
   p.sout->nupd = p.k + 1;
   p.sout->iter = nx.iter;
   p.sout->status = nx.status;
+  p.sout->err = nx.err_hist[1];
   if (nx.done) p.sout->done = 1;
 }
 

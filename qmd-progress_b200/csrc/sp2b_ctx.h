@@ -39,11 +39,19 @@ struct Ctx {
   size_t vv_cap = 0;
   double* rowsum = nullptr;
   size_t rowsum_cap = 0;
-  double* small = nullptr;      // device scratch scalars
-  double* h_small = nullptr;    // pinned host mirror
-  SolveOut* sout = nullptr;
-  SolveOut* h_sout = nullptr;   // pinned
+  // one small device block and its pinned mirror: scratch scalars, then what a solve reads
+  // back in one copy (the normalisation's {min, max, trace, ||X0||^2} and the outcome), then
+  // the reduction counters and the error word
+  double* small = nullptr;
+  double* h_small = nullptr;
+  double* norm_out = nullptr;   // small + kNorm
+  SolveOut* sout = nullptr;     // behind norm_out
+  SolveOut* h_sout = nullptr;
   int* err = nullptr;
+  static constexpr int kNorm = 48, kBack = 7;   // doubles read back: 4 + sizeof(SolveOut) / 8
+  cudaEvent_t poll = nullptr;   // the outcome copy of a poll
+  char* pin = nullptr;          // pinned: pp, vv and the refinement's scale of a solve
+  size_t pin_cap = 0;
   // INT8 refinement: residue planes, reduced product planes, work list, scale state
   int8_t* oz_res = nullptr;
   uint8_t* oz_q = nullptr;
@@ -59,12 +67,24 @@ struct Ctx {
   std::vector<cudaEvent_t> ev;      // step timing events (pairs)
   std::vector<cudaEvent_t> ev_ref;  // INT8 refinement phase boundaries
 
+  // zeroes the outcome, the counters and the error word
+  cudaError_t clear_control(cudaStream_t st) {
+    return cudaMemsetAsync(sout, 0, (char*)(err + 1) - (char*)sout, st);
+  }
+  // norm_out and the outcome into the pinned mirror
+  cudaError_t read_back(cudaStream_t st) {
+    return cudaMemcpyAsync(h_small + kNorm, norm_out, kBack * sizeof(double),
+                           cudaMemcpyDeviceToHost, st);
+  }
+  cudaError_t ensure_pin(size_t bytes);
   cudaError_t ensure_f64(int np, int nbuf);
   cudaError_t ensure_f64_solve(int n, bool resp);
   cudaError_t ensure_split(int np);
   cudaError_t ensure_common(size_t nin, int np, int maxlaunch, int n);
   cudaError_t ensure_oz(int np, cudaStream_t st);
 };
+
+static_assert(sizeof(SolveOut) == 24, "the outcome follows norm_out in one read-back");
 
 Ctx* get_ctx(int* status);
 

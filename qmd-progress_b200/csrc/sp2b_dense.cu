@@ -61,22 +61,33 @@ Ctx* get_ctx(int* status) {
   Ctx& c = g_ctx[dev];
   if (!c.init) {
     if (cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaMallocHost((void**)&c.h_sout, sizeof(SolveOut)) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c.poll, cudaEventDisableTiming) != cudaSuccess ||
         cudaMallocHost((void**)&c.h_small, 64 * sizeof(double)) != cudaSuccess ||
-        cudaMalloc((void**)&c.small, 64 * sizeof(double)) != cudaSuccess ||
-        cudaMalloc((void**)&c.counter, 4 * sizeof(unsigned)) != cudaSuccess ||
-        cudaMalloc((void**)&c.sout, sizeof(SolveOut)) != cudaSuccess ||
-        cudaMalloc((void**)&c.err, sizeof(int)) != cudaSuccess ||
-        cudaMemset(c.counter, 0, 4 * sizeof(unsigned)) != cudaSuccess ||
-        cudaMemset(c.err, 0, sizeof(int)) != cudaSuccess) {
+        cudaMalloc((void**)&c.small, 72 * sizeof(double)) != cudaSuccess ||
+        cudaMemset(c.small, 0, 72 * sizeof(double)) != cudaSuccess) {
       set_last_error("context setup failed: %s", cudaGetErrorString(cudaGetLastError()));
       *status = SP2B_CUDA_ERROR;
       return nullptr;
     }
+    c.norm_out = c.small + Ctx::kNorm;
+    c.sout = reinterpret_cast<SolveOut*>(c.norm_out + 4);
+    c.h_sout = reinterpret_cast<SolveOut*>(c.h_small + Ctx::kNorm + 4);
+    c.counter = reinterpret_cast<unsigned*>(c.sout + 1);
+    c.err = reinterpret_cast<int*>(c.counter + 4);
     c.dev = dev;
     c.init = true;
   }
   return &c;
+}
+
+cudaError_t Ctx::ensure_pin(size_t bytes) {
+  if (bytes <= pin_cap) return cudaSuccess;
+  if (pin) cudaFreeHost(pin);
+  pin = nullptr;
+  pin_cap = 0;
+  const cudaError_t e = cudaMallocHost((void**)&pin, bytes);
+  if (e == cudaSuccess) pin_cap = bytes;
+  return e;
 }
 
 cudaError_t Ctx::ensure_f64(int np, int nbuf) {
@@ -282,25 +293,21 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
     hdev = c->hin;
   }
   double* bounds = c->small;       // [0..1]
-  double* norm_out = c->small + 4; // [4..7]
+  SP2B_CUDA_TRY(c->clear_control(st));
   if (j.given_bounds) {
     c->h_small[0] = j.mineval;
     c->h_small[1] = j.maxeval;
     SP2B_CUDA_TRY(cudaMemcpyAsync(bounds, c->h_small, 2 * sizeof(double), cudaMemcpyHostToDevice, st));
   } else {
-    SP2B_CUDA_TRY(cudaMemsetAsync(c->counter, 0, 4 * sizeof(unsigned), st));
     SP2B_CUDA_TRY(launch_gersh(hdev, n, n, c->rowsum, gersh_nsplit(n), bounds, c->partials,
                                c->counter, st));
   }
-  SP2B_CUDA_TRY(cudaMemsetAsync(c->counter, 0, 4 * sizeof(unsigned), st));
-  SP2B_CUDA_TRY(cudaMemsetAsync(c->err, 0, sizeof(int), st));
-  SP2B_CUDA_TRY(cudaMemsetAsync(c->sout, 0, sizeof(SolveOut), st));
   if (split)
     SP2B_CUDA_TRY(launch_normalize_split(hdev, n, n, np, bounds, c->hi[0], c->lo[0], bf16,
-                                         c->partials, c->counter, c->rec, norm_out, st));
+                                         c->partials, c->counter, c->rec, c->norm_out, st));
   else
     SP2B_CUDA_TRY(launch_normalize_f64(hdev, n, n, np, bounds, c->x64[0], c->partials, c->counter,
-                                       c->rec, norm_out, st));
+                                       c->rec, c->norm_out, st));
   if (resp) {
     // Delta_0 = alpha H1 (src/prg_response_mod.F90:700); a host H1 is staged in x64[4]
     const double* h1dev = j.h1;
@@ -317,7 +324,7 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
     SP2B_CUDA_TRY(cudaMemcpyAsync(c->pp_dev, j.pp_in, j.ctl.icount * sizeof(int), cudaMemcpyHostToDevice, st));
   if (j.vv_out && j.vv_accumulate && maxlaunch > 0) {
     SP2B_CUDA_TRY(cudaMemcpyAsync(c->vv_dev, j.vv_out, maxlaunch * sizeof(double), cudaMemcpyHostToDevice, st));
-  } else {
+  } else if (j.vv_out) {
     SP2B_CUDA_TRY(cudaMemsetAsync(c->vv_dev, 0, (maxlaunch + 2) * sizeof(double), st));
   }
   int* pp_out_dev = (j.ctl.algo == ALGO_SEQ) ? nullptr : c->pp_dev;
@@ -351,13 +358,77 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
   fa.pp_out = pp_out_dev;
   fa.vv_out = c->vv_dev;
   fa.vv_accumulate = j.vv_accumulate;
+  // pp and vv leave through pinned memory, all that a solve of maxlaunch steps can write
+  const size_t pin_vv = 0, pin_pp = (size_t)(maxlaunch + 2) * sizeof(double);
+  const size_t pin_sc = (pin_pp + (size_t)(maxlaunch + 2) * sizeof(int) + 7) / 8 * 8;
+  const size_t pin_err = pin_sc + oz_scale_bytes();
+  SP2B_CUDA_TRY(c->ensure_pin(pin_err + sizeof(int)));
+  auto queue_sequences = [&]() -> cudaError_t {
+    cudaError_t e = cudaSuccess;
+    if (j.vv_out && maxlaunch > 0)
+      e = cudaMemcpyAsync(c->pin + pin_vv, c->vv_dev, maxlaunch * sizeof(double),
+                          cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess && j.pp_out && maxlaunch > 0)
+      e = cudaMemcpyAsync(c->pin + pin_pp, c->pp_dev, maxlaunch * sizeof(int),
+                          cudaMemcpyDeviceToHost, st);
+    return e;
+  };
   int k = 0;
   int chunk = fp64 ? f64_solve_chunk(n, resp) : 4;
   bool done = (maxlaunch == 0);
   const bool timing = g_step_timing.load() != 0;
-  while (!done && k < maxlaunch) {
-    if (fallback && k >= j.exact_switch) {   // still running: a nearly gapless spectrum
-      *want_exact = true;
+  // An FP64 solve whose steps fit one launch: its density and sequences follow it at once,
+  // and one wait ends the call.
+  const bool at_once = fp64 && j.dev_ptrs && chunk >= maxlaunch && maxlaunch > 0;
+  // While the host waits for a poll's outcome, kAhead more steps keep the GPU busy; they do
+  // nothing if the loop had ended.
+  constexpr int kAhead = 2;
+  int polled = 0;   // steps issued before the last outcome read
+  auto poll = [&]() -> cudaError_t {
+    cudaError_t e = c->read_back(st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    done = c->h_sout->done != 0;
+    polled = k;
+    return e;
+  };
+  // one step of the split or the exact form
+  auto issue_step = [&](int s) -> int {
+    a.k = s;
+    const int bin = s & 1, bout = (s + 1) & 1;
+    if (exact) {
+      // X_k^2 exactly: residue planes of rint(2^S X_k), nine INT8 products, then the
+      // CRT kernel applies step k's branch and publishes the step's record
+      OzStepCtl oc;
+      oc.sout = c->sout;
+      oc.rec = c->rec;
+      oc.pp_in = c->pp_dev;
+      oc.ctl = a.ctl;
+      oc.k = s;
+      oc.active = 1;
+      SP2B_CUDA_TRY(launch_oz_planes_f64(c->x64[bin], np, c->oz_scale, s > 0 ? c->oz_rown : nullptr,
+                                         c->oz_res, &oc, st));
+      SP2B_CUDA_TRY(launch_oz_gemm(c->oz_res, np, c->oz_q, c->oz_work, c->oz_nwork, c->oz_grid,
+                                   c->err, st, &oc));
+      a.E = c->x64[bin];
+      a.out = c->x64[bout];
+      SP2B_CUDA_TRY(launch_oz_crt_step(c->oz_q, c->oz_scale, a, c->oz_rown, c->oz_res, st));
+    } else {
+      a.A = a.B = a.E = c->hi[bin];
+      a.A_lo = a.B_lo = a.E_lo = c->lo[bin];
+      a.out = c->hi[bout];
+      a.out_lo = c->lo[bout];
+      a.ntiles = tc_ntiles(np);
+      SP2B_CUDA_TRY(launch_sym_gemm_tc(a, bf16, st));
+    }
+    return SP2B_OK;
+  };
+  while (!done && (k < maxlaunch || polled < k)) {
+    if (k >= maxlaunch || (fallback && k >= j.exact_switch)) {
+      if (polled < k) {   // the steps issued ahead of the last outcome
+        SP2B_CUDA_TRY(poll());
+        continue;
+      }
+      *want_exact = true;   // still running: a nearly gapless spectrum
       return SP2B_OK;
     }
     int kend = std::min(maxlaunch, k + chunk);
@@ -378,40 +449,34 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
       SP2B_CUDA_TRY(launch_f64_solve(fa, n, np, c->f64w, st));
       if (timing) SP2B_CUDA_TRY(cudaEventRecord(c->ev[1], st));
       k = kend;
-    }
-    for (; k < kend; ++k) {
-      a.k = k;
-      if (timing) SP2B_CUDA_TRY(cudaEventRecord(c->ev[2 * (k - k0)], st));
-      const int bin = k & 1, bout = (k + 1) & 1;
-      if (exact) {
-        // X_k^2 exactly: residue planes of rint(2^S X_k), nine INT8 products, then the
-        // CRT kernel applies step k's branch and publishes the step's record
-        OzStepCtl oc;
-        oc.sout = c->sout;
-        oc.rec = c->rec;
-        oc.pp_in = c->pp_dev;
-        oc.ctl = a.ctl;
-        oc.k = k;
-        oc.active = 1;
-        SP2B_CUDA_TRY(launch_oz_planes_f64(c->x64[bin], np, c->oz_scale, k > 0 ? c->oz_rown : nullptr,
-                                           c->oz_res, &oc, st));
-        SP2B_CUDA_TRY(launch_oz_gemm(c->oz_res, np, c->oz_q, c->oz_work, c->oz_nwork, c->oz_grid, c->err, st, &oc));
-        a.E = c->x64[bin];
-        a.out = c->x64[bout];
-        SP2B_CUDA_TRY(launch_oz_crt_step(c->oz_q, c->oz_scale, a, c->oz_rown, c->oz_res, st));
-      } else {
-        a.A = a.B = a.E = c->hi[bin];
-        a.A_lo = a.B_lo = a.E_lo = c->lo[bin];
-        a.out = c->hi[bout];
-        a.out_lo = c->lo[bout];
-        a.ntiles = tc_ntiles(np);
-        SP2B_CUDA_TRY(launch_sym_gemm_tc(a, bf16, st));
+      if (at_once) {
+        SP2B_CUDA_TRY(launch_finish_solve_f64(c->x64[0], c->x64[1], c->sout, c->norm_out, np, n,
+                                              j.rho, n, st));
+        if (resp)
+          SP2B_CUDA_TRY(launch_finish_solve_f64(c->x64[2], c->x64[3], c->sout, c->norm_out, np, n,
+                                                j.rsp, n, st));
+        SP2B_CUDA_TRY(queue_sequences());
       }
-      if (timing) SP2B_CUDA_TRY(cudaEventRecord(c->ev[2 * (k - k0) + 1], st));
+      SP2B_CUDA_TRY(poll());
+    } else {
+      for (; k < kend; ++k) {
+        if (timing) SP2B_CUDA_TRY(cudaEventRecord(c->ev[2 * (k - k0)], st));
+        const int rc = issue_step(k);
+        if (rc != SP2B_OK) return rc;
+        if (timing) SP2B_CUDA_TRY(cudaEventRecord(c->ev[2 * (k - k0) + 1], st));
+      }
+      int ahead = timing ? k : std::min(maxlaunch, k + kAhead);
+      if (fallback) ahead = std::min(ahead, std::max(k, j.exact_switch));
+      SP2B_CUDA_TRY(c->read_back(st));
+      SP2B_CUDA_TRY(cudaEventRecord(c->poll, st));
+      polled = k;
+      for (; k < ahead; ++k) {
+        const int rc = issue_step(k);
+        if (rc != SP2B_OK) return rc;
+      }
+      SP2B_CUDA_TRY(cudaEventSynchronize(c->poll));
+      done = c->h_sout->done != 0;
     }
-    SP2B_CUDA_TRY(cudaMemcpyAsync(c->h_sout, c->sout, sizeof(SolveOut), cudaMemcpyDeviceToHost, st));
-    SP2B_CUDA_TRY(cudaStreamSynchronize(st));
-    done = c->h_sout->done != 0;
     if (timing && fp64) {
       float ms = 0.f;
       SP2B_CUDA_TRY(cudaEventElapsedTime(&ms, c->ev[0], c->ev[1]));
@@ -436,35 +501,27 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
     if (!fp64) chunk = std::min(chunk * 2, 16);
   }
   c->last_launches = k;
+  if (maxlaunch == 0) SP2B_CUDA_TRY(poll());   // the normalisation's results
   SolveOut so = *c->h_sout;
   if (maxlaunch == 0) so.nupd = 0;
-  if (fallback && so.nupd > 0) {
-    // the stop reason: Tr X - Tr P of the last update above mixed_tol means the
-    // stagnation test (or maxsp2iter) ended the loop
-    SP2Rec last;
-    SP2B_CUDA_TRY(cudaMemcpyAsync(&last, c->rec + so.nupd, sizeof(SP2Rec), cudaMemcpyDeviceToHost, st));
-    SP2B_CUDA_TRY(cudaStreamSynchronize(st));
-    if (so.status == SP2B_OK && (last.err_hist[1] > j.ctl.mixed_tol ||
-                                 !(last.err_hist[1] == last.err_hist[1]))) {
-      *want_exact = true;
-      return SP2B_OK;
-    }
-    if (so.status == SP2B_NOT_CONVERGED) {
-      *want_exact = true;
-      return SP2B_OK;
-    }
+  // the stop reason: Tr X - Tr P of the last update above mixed_tol means the stagnation
+  // test (or maxsp2iter) ended the loop
+  if (fallback && so.nupd > 0 &&
+      ((so.status == SP2B_OK && !(so.err <= j.ctl.mixed_tol)) ||
+       so.status == SP2B_NOT_CONVERGED)) {
+    *want_exact = true;
+    return SP2B_OK;
   }
   // normalisation itself may have flagged bad input
-  SP2B_CUDA_TRY(cudaMemcpyAsync(c->h_small + 8, norm_out, 4 * sizeof(double), cudaMemcpyDeviceToHost, st));
-  SP2B_CUDA_TRY(cudaStreamSynchronize(st));
-  const double emin = c->h_small[8], emax = c->h_small[9];
+  const double* norm = c->h_small + Ctx::kNorm;
+  const double emin = norm[0], emax = norm[1];
   if (!(emax - emin > 0.0) || !(emin == emin) || !(emax == emax)) {
     set_last_error("non-finite or degenerate spectral bounds (%g, %g)", emin, emax);
     return SP2B_BAD_INPUT;
   }
   // ||X0||_F^2 of the normalised input: a NaN / Inf in H shows here even when no SP2
   // step runs (icount = 0) to flag it
-  if (!(c->h_small[11] == c->h_small[11]) || c->h_small[11] > 1e300) {
+  if (!(norm[3] == norm[3]) || norm[3] > 1e300) {
     set_last_error("non-finite values in the input matrix");
     return SP2B_BAD_INPUT;
   }
@@ -533,21 +590,31 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
     } else {
       xfin = c->x64[fb];
     }
-    SP2B_CUDA_TRY(launch_finish_f64(xfin, np, n, 2.0, rho_dev, n, st));
+    if (!at_once) SP2B_CUDA_TRY(launch_finish_f64(xfin, np, n, 2.0, rho_dev, n, st));
   }
   if (!j.dev_ptrs)
     SP2B_CUDA_TRY(cudaMemcpyAsync(j.rho, rho_dev, nn * sizeof(double), cudaMemcpyDeviceToHost, st));
-  if (resp) {
+  if (resp && !at_once) {
     // rho1 = 2 Delta (src/prg_response_mod.F90:771); host output staged in x64[4]
     double* rsp_dev = j.dev_ptrs ? j.rsp : c->x64[4];
     SP2B_CUDA_TRY(launch_finish_f64(c->x64[2 + fb], np, n, 2.0, rsp_dev, n, st));
     if (!j.dev_ptrs)
       SP2B_CUDA_TRY(cudaMemcpyAsync(j.rsp, rsp_dev, nn * sizeof(double), cudaMemcpyDeviceToHost, st));
   }
+  // ---- sequence outputs and the refinement's scale and status: one wait ----
+  if (!at_once) {
+    SP2B_CUDA_TRY(queue_sequences());
+    if (oz) {
+      SP2B_CUDA_TRY(oz_copy_scale(c->oz_scale, c->pin + pin_sc, st));
+      SP2B_CUDA_TRY(cudaMemcpyAsync(c->pin + pin_err, c->err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    }
+    SP2B_CUDA_TRY(cudaStreamSynchronize(st));
+  }
   if (oz) {
-    int S = 0;
+    int S = 0, herr = 0;
     double r2max = 0.0;
-    SP2B_CUDA_TRY(oz_read_scale(c->oz_scale, &S, &r2max, st));
+    oz_scale_values(c->pin + pin_sc, &S, &r2max);
+    memcpy(&herr, c->pin + pin_err, sizeof(int));
     c->oz_last_S = S;
     c->oz_last_r2max = r2max;
     if (timing) {
@@ -559,9 +626,6 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
       }
       ++g_ref_timed;
     }
-    int herr = 0;
-    SP2B_CUDA_TRY(cudaMemcpyAsync(&herr, c->err, sizeof(int), cudaMemcpyDeviceToHost, st));
-    SP2B_CUDA_TRY(cudaStreamSynchronize(st));
     if (herr) {
       set_last_error("a device-side wait timed out in the INT8 McWeeny refinement");
       return SP2B_TIMEOUT;
@@ -571,19 +635,16 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
       return SP2B_BAD_INPUT;
     }
   }
-
-  // ---- sequence outputs ----
   // (the response loop counts its break iteration, src/prg_response_mod.F90:751; its
   // icount is the number of applied updates, the length of pp)
   const int iters = (j.ctl.algo == ALGO_RESP) ? so.nupd : so.iter;
-  if (j.pp_out && iters > 0)
-    SP2B_CUDA_TRY(cudaMemcpyAsync(j.pp_out, c->pp_dev, iters * sizeof(int), cudaMemcpyDeviceToHost, st));
+  if (j.pp_out && iters > 0 && maxlaunch > 0)
+    memcpy(j.pp_out, c->pin + pin_pp, std::min(iters, maxlaunch) * sizeof(int));
   if (j.vv_out) {
     const int nvv = j.vv_accumulate ? maxlaunch : (j.ctl.algo == ALGO_SEQ ? j.ctl.icount : iters);
-    if (nvv > 0)
-      SP2B_CUDA_TRY(cudaMemcpyAsync(j.vv_out, c->vv_dev, nvv * sizeof(double), cudaMemcpyDeviceToHost, st));
+    if (nvv > 0 && maxlaunch > 0)
+      memcpy(j.vv_out, c->pin + pin_vv, std::min(nvv, maxlaunch) * sizeof(double));
   }
-  SP2B_CUDA_TRY(cudaStreamSynchronize(st));
   if (j.icount_out) *j.icount_out = iters;
   if (j.iters_out) *j.iters_out = iters;
   if (j.bounds_out) {
@@ -922,7 +983,7 @@ int sp2b_normalize(double* h, int n, double* mineval, double* maxeval, const sp2
   SP2B_CUDA_TRY(cudaMemcpyAsync(c->small, c->h_small, 2 * sizeof(double), cudaMemcpyHostToDevice, st));
   SP2B_CUDA_TRY(cudaMemsetAsync(c->counter, 0, 4 * sizeof(unsigned), st));
   SP2B_CUDA_TRY(launch_normalize_f64(hd, n, n, np, c->small, c->x64[0], c->partials, c->counter,
-                                     c->rec, c->small + 4, st));
+                                     c->rec, c->norm_out, st));
   double* out = dev ? h : c->hin;
   SP2B_CUDA_TRY(launch_finish_f64(c->x64[0], np, n, 1.0, out, n, st));
   if (!dev) SP2B_CUDA_TRY(cudaMemcpyAsync(h, out, nn * sizeof(double), cudaMemcpyDeviceToHost, st));

@@ -31,16 +31,13 @@ int fermi_pass(Ctx* c, const double* hdev, int n, int nsteps, double nocc, doubl
                double mu, bool gen, bool deriv, cudaStream_t st, FermiPass* out) {
   const int np = padded(n);
   double* bounds = c->small;
-  double* norm_out = c->small + 4;
   c->h_small[0] = h1 - mu;
   c->h_small[1] = hN - mu;
   SP2B_CUDA_TRY(cudaMemcpyAsync(bounds, c->h_small, 2 * sizeof(double), cudaMemcpyHostToDevice, st));
-  SP2B_CUDA_TRY(cudaMemsetAsync(c->counter, 0, 4 * sizeof(unsigned), st));
-  SP2B_CUDA_TRY(cudaMemsetAsync(c->err, 0, sizeof(int), st));
-  SP2B_CUDA_TRY(cudaMemsetAsync(c->sout, 0, sizeof(SolveOut), st));
+  SP2B_CUDA_TRY(c->clear_control(st));
   SP2B_CUDA_TRY(cudaMemsetAsync(c->small + 24, 0, sizeof(double), st));
   SP2B_CUDA_TRY(launch_normalize_f64(hdev, n, n, np, bounds, c->x64[0], c->partials, c->counter,
-                                     c->rec, norm_out, st));
+                                     c->rec, c->norm_out, st));
   if (deriv) SP2B_CUDA_TRY(launch_resp_init(nullptr, n, n, np, bounds, c->x64[2], st));
   // X <- X^2 or 2X - X^2, and X1 <- {X, X1} or 2 X1 - {X, X1} with X = X_k
   // (src/prg_sp2_fermi_mod.F90:113-120)
@@ -68,11 +65,10 @@ int fermi_pass(Ctx* c, const double* hdev, int n, int nsteps, double nocc, doubl
     SP2B_CUDA_TRY(launch_f64_solve(a, n, np, c->f64w, st));
   }
   SP2Rec r;
-  SP2B_CUDA_TRY(cudaMemcpyAsync(c->h_sout, c->sout, sizeof(SolveOut), cudaMemcpyDeviceToHost, st));
+  SP2B_CUDA_TRY(c->read_back(st));
   SP2B_CUDA_TRY(cudaMemcpyAsync(&r, c->rec + nsteps, sizeof(SP2Rec), cudaMemcpyDeviceToHost, st));
   SP2B_CUDA_TRY(cudaMemcpyAsync(c->h_small + 24, c->small + 24, sizeof(double),
                                 cudaMemcpyDeviceToHost, st));
-  SP2B_CUDA_TRY(cudaMemcpyAsync(c->h_small + 8, norm_out, 4 * sizeof(double), cudaMemcpyDeviceToHost, st));
   SP2B_CUDA_TRY(cudaStreamSynchronize(st));
   int herr = 0;
   SP2B_CUDA_TRY(cudaMemcpy(&herr, c->err, sizeof(int), cudaMemcpyDeviceToHost));
