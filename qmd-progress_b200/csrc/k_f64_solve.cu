@@ -9,45 +9,11 @@
 #include "f64_tile.cuh"
 #include "reduce.cuh"
 #include "sp2b_tune.h"
+#include "work_lists.h"
 
 namespace sp2b {
 
 namespace {
-
-// The work of one step in units of one 16-row k-block of one tile, tile after tile: first
-// the ntiles products X^2 (kb units each), then, with a response, the ntiles
-// anticommutator tiles X Delta + Delta X (2 kb units each, K concatenated).  CTA c takes
-// the units [bound(c), bound(c + 1)): equal shares, so no partial last wave of tiles leaves
-// SMs idle.  A tile cut by a bound is summed by the CTA that holds its last units; the
-// others leave their accumulators in a workspace slot.  A bound closer than `snap` units to
-// a tile edge moves to that edge.
-struct F64Split {
-  int kb, ntiles, snap, G;
-  long long total;
-
-  __device__ __forceinline__ int len(int job) const { return job < ntiles ? kb : 2 * kb; }
-  __device__ __forceinline__ void locate(long long u, int& job, int& off) const {
-    const long long first = (long long)ntiles * kb;
-    if (u < first) {
-      job = (int)(u / kb);
-      off = (int)(u - (long long)job * kb);
-    } else {
-      const long long v = u - first;
-      const int q = (int)(v / (2 * kb));
-      job = ntiles + q;
-      off = (int)(v - (long long)q * 2 * kb);
-    }
-  }
-  __device__ __forceinline__ long long bound(int c) const {
-    const long long u = total * c / G;
-    int job, off;
-    locate(u, job, off);
-    if (off == 0) return u;
-    if (off < snap) return u - off;
-    const int rest = len(job) - off;
-    return rest < snap ? u + rest : u;
-  }
-};
 
 // Waits (bounded) until *word >= target; false when the wait ran out or another CTA gave up.
 __device__ __forceinline__ bool spin_until(const unsigned* word, unsigned target, const int* err) {
@@ -60,7 +26,6 @@ __device__ __forceinline__ bool spin_until(const unsigned* word, unsigned target
   return false;
 }
 
-constexpr int kMaxPieces = 64;   // pieces of one tile other CTAs hold (see f64_plan)
 constexpr int kSums = 5;   // ||X'||^2, Tr X', ||X - X^2||^2 (core rows), Tr X^2, Tr Delta'
 
 // Barrier of the consumer warps.
@@ -434,25 +399,6 @@ __global__ void __launch_bounds__(F64Tile<BT>::NT + 32, 1)
 
 namespace {
 
-struct F64Plan {
-  int bt, tiles, grid, snap;
-};
-
-// Grid of an order-n solve: one CTA per SM, but at least kMinUnits k-blocks each (a cut tile
-// costs its owner and the others ~2 us of workspace traffic, four to eight k-blocks of a
-// 64-edge tile; cutting 32-edge tiles, 0.13 us a k-block, pays only for longer pieces).
-F64Plan f64_plan(int n, int bt, bool resp) {
-  F64Plan pl;
-  pl.bt = bt;
-  pl.tiles = (n + bt - 1) / bt;
-  const int kb = (n + 15) / 16, min_units = bt == 32 ? 24 : 8;
-  const long long tiles = (long long)pl.tiles * (pl.tiles + 1) / 2;
-  const long long units = tiles * kb * (resp ? 3 : 1), jobs = tiles * (resp ? 2 : 1);
-  pl.snap = 4;
-  pl.grid = (int)std::min<long long>(device_sms(), std::max(jobs, units / min_units));
-  return pl;
-}
-
 template <int BT>
 cudaError_t launch_solve(const F64SolveArgs& a, int grid, cudaStream_t st) {
   using C = F64Tile<BT>;
@@ -497,15 +443,15 @@ static size_t solve_work(const F64Plan& pl) {
 
 // Workspace of an order-n solve, for either tile edge the tuner may try.
 size_t f64_solve_ws_doubles(int n, bool resp) {
-  if (n <= kSmallN) return solve_work(f64_plan(n, 32, resp));
-  if (resp) return solve_work(f64_plan(n, 64, resp));
-  return std::max(solve_work(f64_plan(n, 64, resp)), solve_work(f64_plan(n, 128, resp)));
+  if (n <= kSmallN) return solve_work(f64_plan(n, 32, resp, device_sms()));
+  if (resp) return solve_work(f64_plan(n, 64, resp, device_sms()));
+  return std::max(solve_work(f64_plan(n, 64, resp, device_sms())), solve_work(f64_plan(n, 128, resp, device_sms())));
 }
 
 static cudaError_t launch_f64_solve_bt(const F64SolveArgs& a0, int n, int np, int bt, double* work,
                                        cudaStream_t st) {
   F64SolveArgs a = a0;
-  const F64Plan pl = f64_plan(n, bt, a.d[0] != nullptr);
+  const F64Plan pl = f64_plan(n, bt, a.d[0] != nullptr, device_sms());
   a.ld = np;
   a.kb = (n + 15) / 16;
   a.ntiles = pl.tiles * (pl.tiles + 1) / 2;

@@ -21,6 +21,7 @@
 
 #include "reduce.cuh"
 #include "tc_ptx.cuh"
+#include "work_lists.h"
 
 namespace sp2b {
 namespace oz {
@@ -759,60 +760,8 @@ static int oz_sms() {
   return v;
 }
 
-// The product's work for a persistent grid of `grid` CTAs, CTA c taking the entries c,
-// c + grid, ... until one with no blocks.  Upper 128-blocks of every plane: pairs of column
-// blocks as 128 x 256 tiles, the odd one left (the first at or right of the diagonal in odd
-// row blocks, the last of an odd count) as a 128 x 128 tile.  Wide tiles go first in panels
-// of kOzPanel column pairs, row blocks top to bottom inside a panel, so one wave shares few
-// operand row blocks (their K-slices stay in L2).  The wide tiles past the last whole wave
-// and the narrow ones are then dealt to the CTA with the least work, the wide ones cut in
-// two when every CTA can have one half.  In 128 x 128 tiles per SM: n = 2744 takes 16 (15.4
-// on average) where 1188 wide tiles took nine waves, 18; n = 1000 takes 3 instead of 4.
-constexpr int kOzPanel = 6;
 int oz_work_list(int np, std::vector<int4>& out) {
-  const int nb = np / oz::BM;
-  std::vector<int4> wide, narrow;
-  for (int t = 0; t < oz::T; ++t)
-    for (int p0 = 0; p0 < nb; p0 += 2 * kOzPanel) {
-      const int p1 = std::min(nb, p0 + 2 * kOzPanel);
-      for (int bi = 0; bi < p1; ++bi) {
-        int c = std::max(p0, bi);
-        if (c & 1) {   // an odd first block: alone
-          narrow.push_back(make_int4(t, bi, c, 1));
-          ++c;
-        }
-        for (; c + 1 < p1; c += 2) wide.push_back(make_int4(t, bi, c, 2));
-        if (c < p1) narrow.push_back(make_int4(t, bi, c, 1));
-      }
-    }
-  const int grid = (int)std::min<size_t>(2 * wide.size() + narrow.size(), (size_t)oz_sms());
-  const size_t whole = wide.size() / grid * grid;
-  out.assign(wide.begin(), wide.begin() + whole);
-  const size_t rest = wide.size() - whole;
-  const bool cut = 2 * rest + narrow.size() <= (size_t)grid;
-  std::vector<std::vector<int4>> tail(grid);
-  std::vector<int> load(grid, 0);
-  auto deal = [&](const int4& w) {
-    const int c = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-    tail[c].push_back(w);
-    load[c] += w.w;
-  };
-  for (size_t i = whole; i < wide.size(); ++i) {
-    int4 w = wide[i];
-    if (cut) {
-      w.w = 1;
-      deal(w);
-      ++w.z;
-    }
-    deal(w);
-  }
-  for (const int4& w : narrow) deal(w);
-  size_t rounds = 0;
-  for (const auto& v : tail) rounds = std::max(rounds, v.size());
-  for (size_t r = 0; r < rounds; ++r)
-    for (int c = 0; c < grid; ++c)
-      out.push_back(r < tail[c].size() ? tail[c][r] : make_int4(0, 0, 0, 0));
-  return grid;
+  return oz_work_items(np / oz::BM, oz::T, oz_sms(), out);
 }
 
 cudaError_t launch_oz_planes(const __half* xhi, const __half* xlo, int np, int bf16,

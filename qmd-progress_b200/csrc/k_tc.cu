@@ -14,6 +14,7 @@
 
 #include "reduce.cuh"
 #include "tc_ptx.cuh"
+#include "work_lists.h"
 
 #include <map>
 #include <tuple>
@@ -945,7 +946,6 @@ struct PairCfg {
 // TAIL: the work list ends with 64-column tiles (pair_tiles), marked kPairNarrow; their tile.y
 // counts 64-column blocks.  (A form of its own: the choice at run time cost the plain one 4 %
 // at n = 8192.)
-constexpr int kPairNarrow = 1 << 24;
 
 template <typename T, int EPI, bool ANTI = false, bool ES = false, int NB = 128, bool TAIL = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tcp::NTHR, 1)
@@ -1400,21 +1400,6 @@ static const int4* dense_tiles(int np, cudaStream_t st) {
   return d;
 }
 
-// Tiles of the paired kernel, {bi2, bj} with bj >= 2 bi2 (128-column blocks), in panels of
-// kPanel column blocks (row pairs top to bottom inside a panel).
-void pair_tile_order(int nb, int panel, std::vector<int2>& out) {
-  out.clear();
-  for (int p0 = 0; p0 < nb; p0 += panel) {
-    const int p1 = std::min(nb, p0 + panel);
-    for (int bi2 = 0; 2 * bi2 < p1; ++bi2)
-      for (int bj = std::max(2 * bi2, p0); bj < p1; ++bj) out.push_back(make_int2(bi2, bj));
-  }
-}
-static int pair_tile_count(int np) {
-  const int nb = np / tc::BM, np2 = (nb + 1) / 2;
-  return nb * np2 - np2 * (np2 - 1);   // row pair bi2 has the column blocks from 2 bi2 on
-}
-
 // Work items of a launch, cached per (device, np, form).  whole: the tiles that stay whole;
 // the others follow as two 64-column tiles each (NB = 64: whole = 0).
 static const int2* pair_tiles(int np, int whole, bool mark, cudaStream_t st, int* count) {
@@ -1433,18 +1418,8 @@ static const int2* pair_tiles(int np, int whole, bool mark, cudaStream_t st, int
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
     return nullptr;
-  std::vector<int2> blocks, t;
-  pair_tile_order(np / tc::BM, kPanel, blocks);
-  for (size_t i = 0; i < blocks.size(); ++i) {
-    int2 q = blocks[i];
-    if ((int)i < whole) {
-      t.push_back(q);
-      continue;
-    }
-    if (mark) q.x |= kPairNarrow;
-    t.push_back(make_int2(q.x, 2 * q.y));
-    t.push_back(make_int2(q.x, 2 * q.y + 1));
-  }
+  std::vector<int2> t;
+  pair_work_items(np / tc::BM, kPanel, whole, mark, t);
   int2* d = nullptr;
   if (cudaMalloc((void**)&d, t.size() * sizeof(int2)) != cudaSuccess) return nullptr;
   if (cudaMemcpy(d, t.data(), t.size() * sizeof(int2), cudaMemcpyHostToDevice) != cudaSuccess) {
@@ -1533,7 +1508,7 @@ static cudaError_t launch_chained(K kern, int grid, int smem, cudaStream_t st,
 // (the shared-memory limit is raised before the residency query counts the clusters).
 template <typename T, int EPI, bool ANTI, int NB>
 static cudaError_t launch_pair_staged(const StepArgs& a, cudaStream_t st) {
-  const int blocks = pair_tile_count(a.np);
+  const int blocks = pair_tile_count(a.np / tc::BM);
   if (blocks * (128 / NB) > num_sms() / 2) return cudaErrorNotSupported;
   int ntiles = 0;
   const int2* tl = pair_tiles(a.np, NB == 64 ? 0 : blocks, false, st, &ntiles);
@@ -1588,7 +1563,7 @@ static cudaError_t launch_pair(const StepArgs& a, cudaStream_t st) {
   if (!even) return cudaErrorNotSupported;
   // the tiles past the last whole wave, if they are at most half a wave: cut in two, that
   // wave takes half the time (below kTailWaves waves, where it shows: n = 3072 3 -> 2.5)
-  const int blocks = pair_tile_count(a.np), rest = blocks % (num_sms() / 2);
+  const int blocks = pair_tile_count(a.np / tc::BM), rest = blocks % (num_sms() / 2);
   const int waves = blocks / (num_sms() / 2);
   if (waves > 0 && waves < kTailWaves && rest > 0 && 2 * rest <= num_sms() / 2)
     return launch_pair_grid<T, EPI, ANTI, true>(a, blocks - rest, st);
