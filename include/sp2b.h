@@ -399,8 +399,9 @@ int sp2b_dev_adjoint_step_split(const void* g_hi, const void* g_lo, const void* 
 /* ---- diagnostics ------------------------------------------------------------------ */
 
 /* State of the last dense solve on the current device: SP2 step launches issued by
- * the host, X updates applied, Fortran iteration count, status; and, if recs != NULL,
- * up to max_recs control records as 9 doubles each
+ * the host (FP64, whose steps run inside few launches: the steps taken), X updates
+ * applied, Fortran iteration count, status; and, if recs != NULL, up to max_recs control
+ * records as 9 doubles each
  * {trx, trx_data, fro2, idemperr, iter, done, status, last_branch, trp}; record k + 1
  * holds the sums of X_{k+1} and trp = Tr X_k^2 as step k computed it. */
 int sp2b_last_solve_info(int* launches, int* nupd, int* iter, int* status, double* recs,

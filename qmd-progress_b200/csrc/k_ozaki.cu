@@ -14,6 +14,7 @@
 // (Ozaki, Uchino and Imamura, "Ozaki Scheme II: A GEMM-oriented emulation of
 // floating-point matrix multiplication using an integer modular technique", 2025).
 #include <algorithm>
+#include <atomic>
 #include <vector>
 
 #include <cuda_bf16.h>
@@ -72,11 +73,8 @@ constexpr int TMEM_COLS = 2 * BN;
 // (as the bits of a non-negative double, for atomicMax) and the chosen exponent S.
 struct OzScale {
   unsigned long long r2max_bits;
-  unsigned long long next_bits;   // running maximum of k_oz_rowmax (zero between launches)
   int S;      // -1: no valid scale (non-finite input)
-  unsigned counter;               // CTAs of k_oz_rowmax that have arrived
-  int kept;   // the last k_oz_rowmax found the S that the planes were already formed with
-  int pad_;
+  int kept;   // exact steps: the planes of X_k were formed with this S by the step before
 };
 
 // SP2-step context of the launches that compute one step's X^2 (the exact INT8 mode):
@@ -627,12 +625,27 @@ __global__ void __launch_bounds__(256)
 //    leaves the residue planes of X_{k+1} with step k's scale, while the values are in
 //    registers: the scale changes two or three times in a solve, and only then does
 //    k_oz_residues_f64 form them again (planes by a pass over X cost 27 us a step at
-//    n = 2744).  A fixed grid walks the upper 32 x 32 block pairs (diagonal blocks hold both triangles, whose
-//    squares are equal bit for bit: the integer products are symmetric).
+//    n = 2744).  The row norms that the scale needs are integer sums on the way; the last
+//    CTA takes their maximum (stored per block and summed by a pass of its own: 6 us a step
+//    more).  One resident wave of CTAs walks the upper 32 x 32 block pairs (diagonal blocks
+//    hold both triangles, whose squares are equal bit for bit: the integer products are
+//    symmetric).
 // ---------------------------------------------------------------------------------
+// ||row||^2 shares in units of 2^-44, rounded up: integer sums do not depend on their order,
+// and the scale's bound only needs the norm from above (at most np/32 units too much, 1e-10).
+// np/32 <= 2048 shares below 2^8 stay below 2^63.  Larger shares (32 elements of a diverging
+// iterate; with X in [0, 1] a whole row has at most 1) enter as their largest, which NaN
+// exceeds as a bit pattern; the bound then takes it for every share of the row.
+__device__ __forceinline__ void oz_add_row(unsigned long long* rsum, int row, int np, double share) {
+  if (share < 256.0) atomicAdd(rsum + row, __double2ull_ru(share * 0x1p44));
+  else
+    atomicMax(rsum + np, share == share ? (unsigned long long)__double_as_longlong(share)
+                                        : 0x7ff8000000000000ull);
+}
+
 __global__ void __launch_bounds__(256)
-    k_oz_crt_step(const uint8_t* __restrict__ q, const OzScale* __restrict__ sc, const StepArgs p,
-                  double* __restrict__ rown, int8_t* __restrict__ res) {
+    k_oz_crt_step(const uint8_t* __restrict__ q, const OzScale* sc, const StepArgs p,
+                  OzScale* next, unsigned long long* rsum, int8_t* __restrict__ res) {
   __shared__ double s_v[32][33];
   __shared__ double red[32 * 4];
   __shared__ int s_flag;
@@ -682,7 +695,7 @@ __global__ void __launch_bounds__(256)
     rs += __shfl_xor_sync(0xffffffffu, rs, 1);
     rs += __shfl_xor_sync(0xffffffffu, rs, 2);
     rs += __shfl_xor_sync(0xffffffffu, rs, 4);
-    if (c4 == 0) rown[(size_t)i * nb + jb] = rs;
+    if (c4 == 0) oz_add_row(rsum, i, np, rs);
     if (ib != jb) {
       __syncthreads();
       const int r = jb * 32 + row;
@@ -700,49 +713,35 @@ __global__ void __launch_bounds__(256)
       cs += __shfl_xor_sync(0xffffffffu, cs, 1);
       cs += __shfl_xor_sync(0xffffffffu, cs, 2);
       cs += __shfl_xor_sync(0xffffffffu, cs, 4);
-      if (c4 == 0) rown[(size_t)r * nb + ib] = cs;
+      if (c4 == 0) oz_add_row(rsum, r, np, cs);
     }
     __syncthreads();
   }
   __threadfence();
   publish_and_finalize(p, s, red, &s_flag);
-}
-
-// Scale of X_k from the per-block row sums that k_oz_crt_step left: one warp per row, the
-// last CTA chooses S.  Reads np^2 / 4 bytes where a pass over X reads 8 np^2.
-__global__ void __launch_bounds__(256)
-    k_oz_rowmax(const double* __restrict__ rown, int np, OzScale* sc, unsigned* counter,
-                const OzStepCtl c) {
-  if (oz_skip(c)) return;
-  __shared__ double s_max[8];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nb = np / 32;
-  double best = 0.0;
-  for (int row = blockIdx.x * 8 + warp; row < np; row += gridDim.x * 8) {
-    double s = 0.0;
-    for (int j = lane; j < nb; j += 32) s += rown[(size_t)row * nb + j];
-    s = warp_sum(s);
-    if (!(s <= best)) best = s;   // a NaN stays
-    if (best != best) break;
+  if (!s_flag) return;
+  // the last CTA: the scale of X_{k+1} from its row norms, which it clears for the next step
+  unsigned long long best = 0;
+  for (int r = threadIdx.x; r < np; r += blockDim.x) {
+    const unsigned long long v = atomicExch(rsum + r, 0ull);
+    best = v > best ? v : best;
   }
-  if (lane == 0) s_max[warp] = best;
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long v = __shfl_xor_sync(0xffffffffu, best, o);
+    best = v > best ? v : best;
+  }
+  __shared__ unsigned long long s_best[8];
+  if ((threadIdx.x & 31) == 0) s_best[threadIdx.x >> 5] = best;
   __syncthreads();
   if (threadIdx.x != 0) return;
-  unsigned long long bits = 0;
-  for (int w = 0; w < 8; ++w) {
-    // NaN is above every finite value as an unsigned bit pattern
-    const double v = s_max[w];
-    const unsigned long long u = v != v ? 0x7ff8000000000000ull : (unsigned long long)__double_as_longlong(v);
-    bits = u > bits ? u : bits;
-  }
-  atomicMax(&sc->next_bits, bits);
-  __threadfence();
-  if (atomicAdd(counter, 1u) != gridDim.x - 1) return;
-  *counter = 0u;
-  __threadfence();
-  sc->r2max_bits = atomicExch(&sc->next_bits, 0ull);
-  const int S = oz_choose_scale(__longlong_as_double((long long)sc->r2max_bits), np);
-  sc->kept = S == sc->S;
-  sc->S = S;
+  for (int w = 0; w < 8; ++w) best = s_best[w] > best ? s_best[w] : best;
+  const unsigned long long large = atomicExch(rsum + np, 0ull);
+  double r2 = (double)best * 0x1p-44;
+  if (large) r2 += (np / 32) * __longlong_as_double((long long)large);
+  const int Sn = oz_choose_scale(r2, np);
+  next->r2max_bits = (unsigned long long)__double_as_longlong(r2);
+  next->kept = Sn == S;
+  next->S = Sn;
 }
 
 // ---------------------------------------------------------------------------------
@@ -826,37 +825,45 @@ cudaError_t launch_oz_crt(const uint8_t* q, const __half* xhi, const __half* xlo
   return cudaGetLastError();
 }
 
-// rown: null for the first step (the scale and the planes from x); else the row sums that
-// launch_oz_crt_step left with its planes of this x, formed again if the scale changed.
-cudaError_t launch_oz_planes_f64(const double* x, int np, void* scale, const double* rown,
-                                 int8_t* res, const OzStepCtl* ctl, cudaStream_t st) {
+// First step: the scale and the planes from x (and rsum cleared).  Later steps: the planes
+// that launch_oz_crt_step left, formed again if it found another scale for this x.
+cudaError_t launch_oz_planes_f64(const double* x, int np, void* scale, unsigned long long* rsum,
+                                 bool first, int8_t* res, const OzStepCtl* ctl, cudaStream_t st) {
   if (np % oz::BM != 0 || np > 65536) return cudaErrorInvalidValue;
   OzScale* sc = (OzScale*)scale;
-  const int rgrid = std::min((np + 7) / 8, 148 * 8);
-  if (rown) {
-    k_oz_rowmax<<<rgrid, 256, 0, st>>>(rown, np, sc, &sc->counter, *ctl);
-    note_launch(2);
-  } else {
+  if (first) {
     cudaError_t e = cudaMemsetAsync(sc, 0, sizeof(OzScale), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(rsum, 0, oz_rsum_words(np) * sizeof(*rsum), st);
     if (e != cudaSuccess) return e;
-    k_oz_rownorm_f64<<<rgrid, 256, 0, st>>>(x, np, sc, *ctl);
+    k_oz_rownorm_f64<<<std::min((np + 7) / 8, 148 * 8), 256, 0, st>>>(x, np, sc, *ctl);
     k_oz_scale<<<1, 1, 0, st>>>(sc, np);
-    note_launch(3);
+    note_launch(2);
   }
   const size_t groups = (size_t)np * np / 8;
   const int g = (int)std::min<size_t>((groups + 255) / 256, 148 * 16);
-  k_oz_residues_f64<<<g, 256, 0, st>>>(x, np, sc, res, *ctl, rown != nullptr);
+  k_oz_residues_f64<<<g, 256, 0, st>>>(x, np, sc, res, *ctl, !first);
+  note_launch();
   return cudaGetLastError();
 }
 
-size_t oz_rown_doubles(int np) { return (size_t)np * (np / 32); }
+size_t oz_rsum_words(int np) { return (size_t)np + 1; }
 
-cudaError_t launch_oz_crt_step(const uint8_t* q, const void* scale, const StepArgs& a, double* rown,
-                               int8_t* res, cudaStream_t st) {
+cudaError_t launch_oz_crt_step(const uint8_t* q, void* scale, const StepArgs& a,
+                               unsigned long long* rsum, int8_t* res, cudaStream_t st) {
   if (a.np % 128 != 0) return cudaErrorInvalidValue;
   const long long nb = a.np / 32;
-  const int grid = (int)std::min<long long>(nb * (nb + 1) / 2, 148 * 8);
-  k_oz_crt_step<<<grid, 256, 0, st>>>(q, (const OzScale*)scale, a, rown, res);
+  // one resident wave: every CTA walks its share of the blocks (more CTAs than fit end in a
+  // second wave that is mostly empty)
+  static std::atomic<int> resident{0};
+  int per_sm = resident.load(std::memory_order_relaxed);
+  if (per_sm == 0) {
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_oz_crt_step, 256, 0);
+    if (e != cudaSuccess) return e;
+    per_sm = std::min(std::max(per_sm, 1), 8);   // the partial sums have room for eight
+    resident.store(per_sm, std::memory_order_relaxed);
+  }
+  const int grid = (int)std::min<long long>(nb * (nb + 1) / 2, (long long)oz_sms() * per_sm);
+  k_oz_crt_step<<<grid, 256, 0, st>>>(q, (const OzScale*)scale, a, (OzScale*)scale, rsum, res);
   note_launch();
   return cudaGetLastError();
 }

@@ -164,11 +164,11 @@ struct OzStepCtl {
 cudaError_t launch_oz_gemm(const int8_t* res, int np, uint8_t* qout, const int4* work,
                            int nwork, int grid, int* err, cudaStream_t st,
                            const OzStepCtl* ctl = nullptr);
-cudaError_t launch_oz_planes_f64(const double* x, int np, void* scale, const double* rown,
-                                 int8_t* res, const OzStepCtl* ctl, cudaStream_t st);
-size_t oz_rown_doubles(int np);   // per-block row sums of the iterate a step wrote
-cudaError_t launch_oz_crt_step(const uint8_t* q, const void* scale, const StepArgs& a, double* rown,
-                               int8_t* res, cudaStream_t st);
+cudaError_t launch_oz_planes_f64(const double* x, int np, void* scale, unsigned long long* rsum,
+                                 bool first, int8_t* res, const OzStepCtl* ctl, cudaStream_t st);
+size_t oz_rsum_words(int np);   // row norm sums of the iterate a step writes
+cudaError_t launch_oz_crt_step(const uint8_t* q, void* scale, const StepArgs& a,
+                               unsigned long long* rsum, int8_t* res, cudaStream_t st);
 cudaError_t launch_oz_crt(const uint8_t* q, const __half* xhi, const __half* xlo, int np,
                           int bf16, const void* scale, double* x2, __half* rhi, __half* rlo,
                           cudaStream_t st);

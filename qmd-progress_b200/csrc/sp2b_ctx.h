@@ -59,8 +59,8 @@ struct Ctx {
   int4* oz_work = nullptr;
   int oz_work_np = 0, oz_nwork = 0, oz_grid = 0;
   void* oz_scale = nullptr;
-  double* oz_rown = nullptr;    // exact steps: per-block row sums of the iterate
-  size_t oz_rown_cap = 0;
+  unsigned long long* oz_rsum = nullptr;   // exact steps: row norm sums of the iterate
+  size_t oz_rsum_cap = 0;
   int oz_last_S = 0;            // scale exponent of the last INT8 refinement
   double oz_last_r2max = 0.0;   // its largest squared row norm
   int last_launches = 0;            // SP2 step launches of the last dense solve

@@ -282,7 +282,7 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
       return SP2B_BAD_ARG;
     }
     SP2B_CUDA_TRY(c->ensure_oz(np, st));
-    if (exact) SP2B_CUDA_TRY(grow(c->oz_rown, c->oz_rown_cap, oz_rown_doubles(np)));
+    if (exact) SP2B_CUDA_TRY(grow(c->oz_rsum, c->oz_rsum_cap, oz_rsum_words(np)));
   }
 
   // ---- input ----
@@ -405,13 +405,13 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
       oc.ctl = a.ctl;
       oc.k = s;
       oc.active = 1;
-      SP2B_CUDA_TRY(launch_oz_planes_f64(c->x64[bin], np, c->oz_scale, s > 0 ? c->oz_rown : nullptr,
-                                         c->oz_res, &oc, st));
+      SP2B_CUDA_TRY(launch_oz_planes_f64(c->x64[bin], np, c->oz_scale, c->oz_rsum, s == 0, c->oz_res,
+                                         &oc, st));
       SP2B_CUDA_TRY(launch_oz_gemm(c->oz_res, np, c->oz_q, c->oz_work, c->oz_nwork, c->oz_grid,
                                    c->err, st, &oc));
       a.E = c->x64[bin];
       a.out = c->x64[bout];
-      SP2B_CUDA_TRY(launch_oz_crt_step(c->oz_q, c->oz_scale, a, c->oz_rown, c->oz_res, st));
+      SP2B_CUDA_TRY(launch_oz_crt_step(c->oz_q, c->oz_scale, a, c->oz_rsum, c->oz_res, st));
     } else {
       a.A = a.B = a.E = c->hi[bin];
       a.A_lo = a.B_lo = a.E_lo = c->lo[bin];
@@ -500,10 +500,10 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
     }
     if (!fp64) chunk = std::min(chunk * 2, 16);
   }
-  c->last_launches = k;
   if (maxlaunch == 0) SP2B_CUDA_TRY(poll());   // the normalisation's results
   SolveOut so = *c->h_sout;
   if (maxlaunch == 0) so.nupd = 0;
+  c->last_launches = fp64 ? so.nupd : k;   // FP64: the steps taken inside the launches
   // the stop reason: Tr X - Tr P of the last update above mixed_tol means the stagnation
   // test (or maxsp2iter) ended the loop
   if (fallback && so.nupd > 0 &&

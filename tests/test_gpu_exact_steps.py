@@ -44,3 +44,23 @@ def test_exact_steps_against_integers(cuda, n):
     # 2^-S grid (S ~ 35) can turn into one grid step of single elements
     assert np.linalg.norm(got.rho - 2.0 * x) <= 2.0 ** -33 * np.sqrt(n) * np.linalg.norm(x)
     assert np.allclose(got.vv, vv, rtol=1e-8, atol=2.0 ** -32 * n)
+
+
+@pytest.mark.parametrize("n", [33, 130])
+def test_row_norms_above_the_integer_range(cuda, n):
+    """Bounds narrower than the spectrum: the iterate grows, and 32-element shares of its row
+    norms pass 2^8, where the scale's bound takes the largest share for every one of a row."""
+    h = M.two_band_1d(n, seed=n)
+    emin, emax = O.gershgorin(h)
+    mid, half = 0.5 * (emin + emax), 0.05 * (emax - emin)
+    pp = [1, 1, 1]
+    got = sp2b.sp2_alg2_seq_inplace(h, pp, len(pp), mid - half, mid + half,
+                                    precision=sp2b.PREC_EXACT_INT8)
+    x = (mid + half) / (2 * half) * np.eye(n) - h / (2 * half)
+    for _ in pp[1:]:
+        x = x @ x
+    assert np.max(np.sum(x * x, axis=1)) > 2.0 ** 13   # so one of its shares is above 2^8
+    x = x @ x
+    # 2^S r >= 2^35.9 / (2 * 2) for rows of up to 5 shares: elements are rounded by 2^-35 r, the
+    # matrix by e = 2^-35 sqrt(n) r, and each squaring doubles the relative error: 14 e
+    assert np.linalg.norm(got.rho - 2.0 * x) <= 2.0 ** -31 * np.sqrt(n) * np.linalg.norm(2.0 * x)
