@@ -285,11 +285,15 @@ __global__ void k_oz_residues(const T* __restrict__ hi, const T* __restrict__ lo
   }
 }
 
-__global__ void k_oz_residues_f64(const double* __restrict__ x, int np,
-                                  const OzScale* __restrict__ sc, int8_t* __restrict__ res,
+// (No __restrict__ on what the launch before writes here and in k_oz_crt_step: this launch
+// begins before that one ends, and a read-only load may be moved ahead of the wait.)
+__global__ void k_oz_residues_f64(const double* x, int np, const OzScale* sc, int8_t* res,
                                   const OzStepCtl c, int formed) {
-  if (oz_skip(c)) return;
+  // (the three launches of a step are chained: each waits for the one before here)
+  grid_launch_dependents();
+  grid_wait();
   if (formed && sc->kept) return;   // the step before formed these planes
+  if (oz_skip(c)) return;
   const int S = sc->S;
   const double scale = S < 0 ? 0.0 : ldexp(1.0, S);
   const size_t plane = (size_t)np * np;
@@ -326,7 +330,6 @@ struct OzGemmArgs {
 
 __global__ void __launch_bounds__(oz::NTHR, 1)
     k_oz_gemm(const __grid_constant__ CUtensorMap tm, const OzGemmArgs p) {
-  if (oz_skip(p.ctl)) return;   // the same answer in every CTA
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[oz::ST];
   __shared__ __align__(8) uint64_t bar_empty[oz::ST];
@@ -340,6 +343,8 @@ __global__ void __launch_bounds__(oz::NTHR, 1)
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const uint32_t sbase = smem_u32(smem);
+  // up to grid_wait() nothing of the launch before is touched
+  grid_launch_dependents();
   if (threadIdx.x == 0) {
     s_abort = 0;
     for (int s = 0; s < oz::ST; ++s) {
@@ -357,9 +362,10 @@ __global__ void __launch_bounds__(oz::NTHR, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  grid_wait();
   const uint32_t tmem = tmem_holder;
   const int np = p.np;
-  const int nwork = p.nwork;
+  const int nwork = oz_skip(p.ctl) ? 0 : p.nwork;   // the same answer in every CTA
   const int KB = np / oz::BK;
 
   if (warp == 0) {
@@ -550,7 +556,7 @@ __device__ __forceinline__ double crt_value(const uint32_t (&q)[oz::T]) {
   return y;
 }
 // Four consecutive elements of every plane, as the squares' values.
-__device__ __forceinline__ void crt_load4(const uint8_t* __restrict__ q, size_t plane, size_t e,
+__device__ __forceinline__ void crt_load4(const uint8_t* q, size_t plane, size_t e,
                                           double down, double (&x2)[4]) {
   uint32_t w[oz::T];
 #pragma unroll
@@ -626,8 +632,8 @@ __global__ void __launch_bounds__(256)
 //    registers: the scale changes two or three times in a solve, and only then does
 //    k_oz_residues_f64 form them again (planes by a pass over X cost 27 us a step at
 //    n = 2744).  The row norms that the scale needs are integer sums on the way; the last
-//    CTA takes their maximum (stored per block and summed by a pass of its own: 6 us a step
-//    more).  One resident wave of CTAs walks the upper 32 x 32 block pairs (diagonal blocks
+//    CTA takes their maximum (stored per block and summed by a launch of its own: 6 us a step
+//    more).  50 us at n = 2744, where the bytes take 30 at the measured copy rate.  One resident wave of CTAs walks the upper 32 x 32 block pairs (diagonal blocks
 //    hold both triangles, whose squares are equal bit for bit: the integer products are
 //    symmetric).
 // ---------------------------------------------------------------------------------
@@ -644,17 +650,19 @@ __device__ __forceinline__ void oz_add_row(unsigned long long* rsum, int row, in
 }
 
 __global__ void __launch_bounds__(256)
-    k_oz_crt_step(const uint8_t* __restrict__ q, const OzScale* sc, const StepArgs p,
-                  OzScale* next, unsigned long long* rsum, int8_t* __restrict__ res) {
+    k_oz_crt_step(const uint8_t* q, const OzScale* sc, const StepArgs p, OzScale* next,
+                  unsigned long long* rsum, int8_t* res) {
   __shared__ double s_v[32][33];
   __shared__ double red[32 * 4];
   __shared__ int s_flag;
+  grid_launch_dependents();
+  grid_wait();
   const int br = control_prologue(p);
   if (br < 0) return;
   const double a = br == BR_X2 ? 1.0 : -1.0, b = br == BR_X2 ? 0.0 : 2.0;
   const int np = p.np;
-  const double* __restrict__ X = (const double*)p.E;
-  double* __restrict__ Xo = (double*)p.out;
+  const double* X = (const double*)p.E;
+  double* Xo = (double*)p.out;
   const int S = sc->S;
   const double down = S < 0 ? __longlong_as_double(0x7ff8000000000000ll) : ldexp(1.0, -2 * S);
   const double up = S < 0 ? 0.0 : ldexp(1.0, S);
@@ -804,9 +812,7 @@ cudaError_t launch_oz_gemm(const int8_t* res, int np, uint8_t* qout, const int4*
   a.err = err;
   if (ctl) a.ctl = *ctl;
   else memset(&a.ctl, 0, sizeof(a.ctl));
-  k_oz_gemm<<<grid, oz::NTHR, oz::SMEM_BYTES, st>>>(tm, a);
-  note_launch();
-  return cudaGetLastError();
+  return launch_chained(k_oz_gemm, grid, oz::NTHR, oz::SMEM_BYTES, st, tm, a);
 }
 
 cudaError_t launch_oz_crt(const uint8_t* q, const __half* xhi, const __half* xlo, int np,
@@ -840,10 +846,11 @@ cudaError_t launch_oz_planes_f64(const double* x, int np, void* scale, unsigned 
     note_launch(2);
   }
   const size_t groups = (size_t)np * np / 8;
-  const int g = (int)std::min<size_t>((groups + 255) / 256, 148 * 16);
-  k_oz_residues_f64<<<g, 256, 0, st>>>(x, np, sc, res, *ctl, !first);
-  note_launch();
-  return cudaGetLastError();
+  // one wave: most launches only find the planes formed (9 us each with two waves of CTAs
+  // that read the record first; this and the chained launches: 8.99 -> 8.73 ms for the 60
+  // steps of n = 2744)
+  const int g = (int)std::min<size_t>((groups + 255) / 256, (size_t)oz_sms() * 4);
+  return launch_chained(k_oz_residues_f64, g, 256, 0, st, x, np, (const OzScale*)sc, res, *ctl, (int)!first);
 }
 
 size_t oz_rsum_words(int np) { return (size_t)np + 1; }
@@ -863,9 +870,8 @@ cudaError_t launch_oz_crt_step(const uint8_t* q, void* scale, const StepArgs& a,
     resident.store(per_sm, std::memory_order_relaxed);
   }
   const int grid = (int)std::min<long long>(nb * (nb + 1) / 2, (long long)oz_sms() * per_sm);
-  k_oz_crt_step<<<grid, 256, 0, st>>>(q, (const OzScale*)scale, a, (OzScale*)scale, rsum, res);
-  note_launch();
-  return cudaGetLastError();
+  return launch_chained(k_oz_crt_step, grid, 256, 0, st, q, (const OzScale*)scale, a, (OzScale*)scale,
+                        rsum, res);
 }
 
 // Scale exponent and largest squared row norm (diagnostics / checks): queued into pinned

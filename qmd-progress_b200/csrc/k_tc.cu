@@ -1481,29 +1481,6 @@ static bool pair_maps(const StepArgs& a, CUtensorMap (&m)[8]) {
   }
 }
 
-// A paired launch that may start before the launch ahead of it in the stream has completed
-// (programmatic dependent launch): the kernel waits for it (grid_wait) before it reads or
-// writes anything, after its barriers, TMEM and cluster are set up.
-template <typename K>
-static cudaError_t launch_chained(K kern, int grid, int smem, cudaStream_t st,
-                                  const CUtensorMap (&m)[8], const StepArgs& a, const int2* tl,
-                                  int ntiles) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid, 1, 1);
-  cfg.blockDim = dim3(tcp::NTHR, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7],
-                                           a, tl, ntiles);
-  note_launch();
-  return e;
-}
-
 // The single-wave form with the X_k block staged, if its tiles are all resident at once
 // (the shared-memory limit is raised before the residency query counts the clusters).
 template <typename T, int EPI, bool ANTI, int NB>
@@ -1522,7 +1499,8 @@ static cudaError_t launch_pair_staged(const StepArgs& a, cudaStream_t st) {
   }
   CUtensorMap m[8];
   if (!pair_maps<T, EPI, ANTI, NB>(a, m)) return cudaErrorInvalidValue;
-  return launch_chained(kes, 2 * ntiles, smem, st, m, a, tl, ntiles);
+  return launch_chained(kes, 2 * ntiles, tcp::NTHR, smem, st, m[0], m[1], m[2], m[3], m[4], m[5],
+                        m[6], m[7], a, tl, ntiles);
 }
 
 // The persistent form; the tiles past the first `whole` are cut in two (TAIL).
@@ -1538,7 +1516,8 @@ static cudaError_t launch_pair_grid(const StepArgs& a, int whole, cudaStream_t s
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   const int clusters = std::min(ntiles, pair_clusters<T, EPI, ANTI, false, 128, TAIL>());
-  return launch_chained(kern, 2 * clusters, smem, st, m, a, tl, ntiles);
+  return launch_chained(kern, 2 * clusters, tcp::NTHR, smem, st, m[0], m[1], m[2], m[3], m[4], m[5],
+                        m[6], m[7], a, tl, ntiles);
 }
 
 constexpr int kTailWaves = 6;

@@ -12,6 +12,27 @@ void note_launch(int k = 1);
 long long launch_count();
 void set_launch_count(long long v);
 
+// A launch that may start before the launch ahead of it in the stream has completed
+// (programmatic dependent launch): the kernel waits for it (grid_wait) before it reads or
+// writes anything of another launch.
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(void (*kern)(P...), int grid, int threads, int smem,
+                                  cudaStream_t st, const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid, 1, 1);
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
+  note_launch();
+  return e;
+}
+
 // Outcome of a dense solve, written by the device.
 struct SolveOut {
   int done;     // loop finished

@@ -50,7 +50,7 @@ struct F64Plan {
   int bt, tiles, grid, snap;
 };
 
-// Grid of an order-n solve: one CTA per SM, but at least kMinUnits k-blocks each (a cut tile
+// Grid of an order-n solve: one CTA per SM, but at least min_units k-blocks each (a cut tile
 // costs its owner and the others ~2 us of workspace traffic, four to eight k-blocks of a
 // 64-edge tile; cutting 32-edge tiles, 0.13 us a k-block, pays only for longer pieces).
 inline F64Plan f64_plan(int n, int bt, bool resp, int sms) {
