@@ -509,7 +509,7 @@ def main():
         fp64 = {"solves_per_s": world * args.fp64_steps / (tf / 1e3), "iters": it64,
                 "ms_per_solve": tf / args.fp64_steps,
                 "tflops": world * args.fp64_steps * 2.0 * n ** 3 * it64 / (tf / 1e3) / 1e12,
-                "kernel": "k_sym_gemm_f64 (FP64 DMMA SP2 step)"}
+                "kernel": "k_f64_solve (FP64 DMMA, every SP2 step in one launch)"}
         # accuracy of the mixed solve against the FP64 one (same H): ||dD||_F / N
         dd = float((rho_mixed - rho_dev).norm().item())
         fp64["mixed_err_fro_over_n"] = dd / n
@@ -532,7 +532,7 @@ def main():
             kernel = "k_oz_gemm (exact INT8 SP2 step: 9 residue products)"
     else:
         peak_key, peak = None, None
-        kernel = "k_sym_gemm_f64 (FP64 DMMA SP2 step)"
+        kernel = "k_f64_solve (FP64 DMMA, every SP2 step in one launch; per step)"
     traffic = None
     tpath = os.path.join(REPO, "profiles", "traffic.json")
     if os.path.exists(tpath):
@@ -557,13 +557,11 @@ def main():
     refinement = None
     if ref_n.value > 0:
         per = [ref_ms[i] / ref_n.value for i in range(4)]
-        nbp = -(-npad // 256)
-        oz_tiles = sum(nbp - bi // 2 for bi in range(nb))
-        int8_ops = 9 * 2.0 * 128 * 256 * npad * oz_tiles       # executed, 9 residue products
+        int8_ops = 9 * 2.0 * 128 * 128 * npad * (nb * (nb + 1) // 2)   # executed, 9 residue products
         refinement = {"ms_per_solve": sum(per),
                       "phases_ms": {"residue_planes": per[0], "int8_products": per[1], "crt": per[2],
                                     "combine_product": per[3]},
-                      "kernel": "k_oz_gemm (9 INT8 residue products, upper 128x256 tiles)",
+                      "kernel": "k_oz_gemm (9 INT8 residue products, upper 128x128 blocks)",
                       "int8_tops_executed": int8_ops / (per[1] / 1e3) / 1e12,
                       "int8_peak_nominal_tops": 4500.0,
                       "int8_frac_of_nominal": int8_ops / (per[1] / 1e3) / 1e12 / 4500.0}
