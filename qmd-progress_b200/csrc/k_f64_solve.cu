@@ -26,7 +26,7 @@ __device__ __forceinline__ bool spin_until(const unsigned* word, unsigned target
   return false;
 }
 
-constexpr int kSums = 5;   // ||X'||^2, Tr X', ||X - X^2||^2 (core rows), Tr X^2, Tr Delta'
+constexpr int kSums = kF64Sums;
 
 // Barrier of the consumer warps.
 template <int NT>
@@ -419,12 +419,11 @@ cudaError_t launch_solve(const F64SolveArgs& a, int grid, cudaStream_t st) {
 
 }  // namespace
 
-// Tile edge of an order-n solve: 32 up to kSmallN, where 64-edge tiles are too few for the
+// Tile edge of an order-n solve: 32 up to kF64SmallN, where 64-edge tiles are too few for the
 // SMs (n = 300: 235 us a solve with 32, 270 us with 64; n = 500: 296 and 284); above it the
 // measured choice for this device and padded size (tune_f64_solve), else 64.
-constexpr int kSmallN = 416;
 int f64_solve_tile(int n, int np, bool resp) {
-  if (n <= kSmallN) return 32;
+  if (n <= kF64SmallN) return 32;
   int c = 0;
   if (resp) return 64;   // a 128-edge tile of sums does not fit beside the stages
   return tune_lookup(f64_tune_key(np), &c) && (c == 64 || c == 128) ? c : 64;
@@ -437,21 +436,13 @@ int f64_solve_chunk(int n, bool resp) {
   return (int)std::max(1.0, std::min(1e6, 2e12 / flops));
 }
 
-static size_t solve_work(const F64Plan& pl) {
-  return (size_t)pl.grid * pl.bt * pl.bt + 2 * (size_t)pl.grid * kSums + pl.grid / 2 + 2;
-}
-
-// Workspace of an order-n solve, for either tile edge the tuner may try.
-size_t f64_solve_ws_doubles(int n, bool resp) {
-  if (n <= kSmallN) return solve_work(f64_plan(n, 32, resp, device_sms()));
-  if (resp) return solve_work(f64_plan(n, 64, resp, device_sms()));
-  return std::max(solve_work(f64_plan(n, 64, resp, device_sms())), solve_work(f64_plan(n, 128, resp, device_sms())));
-}
+size_t f64_solve_ws_doubles(int n, bool resp) { return f64_solve_doubles(n, resp, device_sms()); }
 
 static cudaError_t launch_f64_solve_bt(const F64SolveArgs& a0, int n, int np, int bt, double* work,
-                                       cudaStream_t st) {
+                                       size_t cap, cudaStream_t st) {
   F64SolveArgs a = a0;
   const F64Plan pl = f64_plan(n, bt, a.d[0] != nullptr, device_sms());
+  if (!work || f64_plan_doubles(pl) > cap) return cudaErrorInvalidValue;
   a.ld = np;
   a.kb = (n + 15) / 16;
   a.ntiles = pl.tiles * (pl.tiles + 1) / 2;
@@ -469,16 +460,18 @@ static cudaError_t launch_f64_solve_bt(const F64SolveArgs& a0, int n, int np, in
   return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
-cudaError_t launch_f64_solve(const F64SolveArgs& a, int n, int np, double* work, cudaStream_t st) {
-  return launch_f64_solve_bt(a, n, np, f64_solve_tile(n, np, a.d[0] != nullptr), work, st);
+cudaError_t launch_f64_solve(const F64SolveArgs& a, int n, int np, double* work, size_t cap,
+                             cudaStream_t st) {
+  return launch_f64_solve_bt(a, n, np, f64_solve_tile(n, np, a.d[0] != nullptr), work, cap, st);
 }
 
 // Measures the tile edges 128 and 64 at np (one SP2 step each) and records the faster one
 // for f64_solve_tile.  `a` as for a solve; its records, sums and iterates are overwritten.
-int tune_f64_solve(int n, int np, const F64SolveArgs& a0, double* work, cudaStream_t st) {
+int tune_f64_solve(int n, int np, const F64SolveArgs& a0, double* work, size_t cap,
+                   cudaStream_t st) {
   int c = 0;
   const std::string key = f64_tune_key(np);
-  if (n <= kSmallN || a0.d[0] || !tune_enabled() || tune_lookup(key, &c)) return SP2B_OK;
+  if (n <= kF64SmallN || a0.d[0] || !tune_enabled() || tune_lookup(key, &c)) return SP2B_OK;
   F64SolveArgs a = a0;
   a.k0 = 0;
   a.k1 = 1;
@@ -498,8 +491,8 @@ int tune_f64_solve(int n, int np, const F64SolveArgs& a0, double* work, cudaStre
   std::vector<float> ms;
   int best = 0;
   const int rc = tune_measure(2, 2, st, [&](int cand) -> int {
-    return launch_f64_solve_bt(a, n, np, edges[cand], work, st) == cudaSuccess ? SP2B_OK
-                                                                             : SP2B_CUDA_ERROR;
+    return launch_f64_solve_bt(a, n, np, edges[cand], work, cap, st) == cudaSuccess ? SP2B_OK
+                                                                                  : SP2B_CUDA_ERROR;
   }, &ms, &best);
   if (rc == SP2B_OK) tune_store(key, edges[best], ms);
   return rc;

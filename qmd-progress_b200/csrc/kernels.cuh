@@ -119,10 +119,13 @@ struct F64SolveArgs {
   unsigned* bar;        // grid barrier counter
 };
 int f64_solve_tile(int n, int np, bool resp);
-int tune_f64_solve(int n, int np, const F64SolveArgs& a, double* work, cudaStream_t st);
+int tune_f64_solve(int n, int np, const F64SolveArgs& a, double* work, size_t cap, cudaStream_t st);
+// Workspace of an order-n solve: with a response also of solves of that order without one.
 size_t f64_solve_ws_doubles(int n, bool resp);
 int f64_solve_chunk(int n, bool resp);
-cudaError_t launch_f64_solve(const F64SolveArgs& a, int n, int np, double* work, cudaStream_t st);
+// cudaErrorInvalidValue when the launch would not fit the `cap` doubles at `work`.
+cudaError_t launch_f64_solve(const F64SolveArgs& a, int n, int np, double* work, size_t cap,
+                             cudaStream_t st);
 
 cudaError_t launch_finish_f64(const double* x, int np, int n, double scale, double* rho,
                               int ld, cudaStream_t st);

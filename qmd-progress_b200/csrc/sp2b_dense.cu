@@ -270,7 +270,7 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
     fa.err = c->err;
     SP2B_CUDA_TRY(c->ensure_f64_solve(n, resp));
     // the measured tile edge for this size (first solve at np on this device)
-    const int trc = tune_f64_solve(n, np, fa, c->f64w, st);
+    const int trc = tune_f64_solve(n, np, fa, c->f64w, c->f64w_cap, st);
     if (trc != SP2B_OK) {
       set_last_error("FP64 tile tuning failed");
       return trc;
@@ -446,7 +446,7 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
       fa.k0 = k;
       fa.k1 = kend;
       if (timing) SP2B_CUDA_TRY(cudaEventRecord(c->ev[0], st));
-      SP2B_CUDA_TRY(launch_f64_solve(fa, n, np, c->f64w, st));
+      SP2B_CUDA_TRY(launch_f64_solve(fa, n, np, c->f64w, c->f64w_cap, st));
       if (timing) SP2B_CUDA_TRY(cudaEventRecord(c->ev[1], st));
       k = kend;
       if (at_once) {

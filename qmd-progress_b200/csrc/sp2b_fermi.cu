@@ -62,7 +62,7 @@ int fermi_pass(Ctx* c, const double* hdev, int n, int nsteps, double nocc, doubl
   for (int k = 0; k < nsteps; k += chunk) {
     a.k0 = k;
     a.k1 = std::min(nsteps, k + chunk);
-    SP2B_CUDA_TRY(launch_f64_solve(a, n, np, c->f64w, st));
+    SP2B_CUDA_TRY(launch_f64_solve(a, n, np, c->f64w, c->f64w_cap, st));
   }
   SP2Rec r;
   SP2B_CUDA_TRY(c->read_back(st));

@@ -65,6 +65,36 @@ inline F64Plan f64_plan(int n, int bt, bool resp, int sms) {
   return pl;
 }
 
+// Edge 32 up to here, larger ones above (f64_solve_tile).
+constexpr int kF64SmallN = 416;
+constexpr int kF64Sums = 5;   // ||X'||^2, Tr X', ||X - X^2||^2 (core rows), Tr X^2, Tr Delta'
+
+// Workspace of a launch, in doubles: one piece per CTA, the partial sums of two steps, then
+// a flag per CTA and the barrier counter.
+inline size_t f64_plan_doubles(const F64Plan& pl) {
+  return (size_t)pl.grid * pl.bt * pl.bt + 2 * (size_t)pl.grid * kF64Sums + pl.grid / 2 + 2;
+}
+
+// The tile edges that a launch of order n may take (returns how many).
+inline int f64_edges(int n, bool resp, int (&bt)[2]) {
+  bt[0] = n <= kF64SmallN ? 32 : 64;
+  bt[1] = 128;
+  return n <= kF64SmallN || resp ? 1 : 2;
+}
+
+// Workspace that covers every launch of order n.  With a response also the launches without
+// one: a set-up for X and Delta serves passes over X alone too (SP2-Fermi generates its
+// sequence that way).
+inline size_t f64_solve_doubles(int n, bool resp, int sms) {
+  size_t w = 0;
+  for (int r = 0; r <= (resp ? 1 : 0); ++r) {
+    int bt[2];
+    const int m = f64_edges(n, r != 0, bt);
+    for (int i = 0; i < m; ++i) w = std::max(w, f64_plan_doubles(f64_plan(n, bt[i], r != 0, sms)));
+  }
+  return w;
+}
+
 // ---- INT8 residue products (k_oz_gemm) ----
 // INT8 residue products of nb x nb 128-blocks: {plane, 128-row block, first 128-column
 // block, 128-column blocks} for a persistent grid (returned: its CTAs), CTA c taking the entries c,

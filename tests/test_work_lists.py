@@ -34,6 +34,13 @@ def test_fp64_shares(lists, sms, resp):
             assert lists.check_f64(n, bt, resp, sms) == 0, (n, bt)
 
 
+@pytest.mark.parametrize("sms", [148, 132, 7])
+def test_fp64_workspace_covers_every_launch(lists, sms):
+    for n in list(range(1, 1300)) + [2000, 4097, 8192, 20011]:
+        for resp in (0, 1):
+            assert lists.check_f64_workspace(n, resp, sms) == 0, (n, resp)
+
+
 @pytest.mark.parametrize("sms", [148, 20])
 def test_int8_product_lists(lists, sms):
     for nb in list(range(1, 40)) + [64, 65, 97]:

@@ -48,6 +48,21 @@ extern "C" int check_f64(int n, int bt, int resp, int sms) {
   return 0;
 }
 
+// The workspace of an order-n set-up holds every launch that may use it: with a response both
+// the launches with it and those without, at every edge.
+extern "C" int check_f64_workspace(int n, int resp, int sms) {
+  const size_t have = f64_solve_doubles(n, resp != 0, sms);
+  for (int r = 0; r <= resp; ++r)
+    for (int bt : {32, 64, 128}) {
+      if ((bt == 32) != (n <= 416) || (r && bt == 128)) continue;
+      const F64Plan pl = f64_plan(n, bt, r != 0, sms);
+      // pieces, sums of two steps, flags and the barrier counter
+      const size_t words = (size_t)pl.grid + 1;
+      if ((size_t)pl.grid * bt * bt + 10 * (size_t)pl.grid + (words + 1) / 2 > have) return 1 + bt + r;
+    }
+  return 0;
+}
+
 // Every upper 128-block of every plane once, lists without holes, tiles inside the matrix.
 extern "C" int check_oz(int nb, int planes, int sms) {
   std::vector<int4> w;
