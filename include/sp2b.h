@@ -437,6 +437,10 @@ int sp2b_last_refinement_info(int* scale_exp, double* r2max);
  * Returns SP2B_TIMEOUT when the wait ran out and the kernel returned normally, which
  * is the expected outcome; the device stays usable. */
 int sp2b_selftest_wait_timeout(int spin_limit);
+/* The same through a whole dense FP64 solve (one step, n = 449, host memory): the waits of its
+ * persistent launch for another block's piece of a tile (wait = 1) or at its grid barrier (2)
+ * run out at once.  SP2B_TIMEOUT when the call reports it. */
+int sp2b_selftest_solve_timeout(int wait);
 int sp2b_set_step_timing(int enable);
 int sp2b_step_timing(double* ms, long long* launches);
 /* With step timing on: summed device time of the INT8 McWeeny refinement phases over

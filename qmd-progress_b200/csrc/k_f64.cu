@@ -304,11 +304,11 @@ cudaError_t launch_finish_f64(const double* x, int np, int n, double scale, doub
 }
 
 __global__ void k_finish_solve_f64(const double* __restrict__ x0, const double* __restrict__ x1,
-                                   const SolveOut* __restrict__ sout,
+                                   const SolveOut* __restrict__ sout, const int* __restrict__ err,
                                    const double* __restrict__ norm, int np, int n,
                                    double* __restrict__ rho, int ld) {
   // (each test is false for a NaN; an infinite norm fails the last)
-  if (!sout->done || !(norm[1] - norm[0] > 0.0) || !(norm[3] <= 1e300)) return;
+  if (!sout->done || *err || !(norm[1] - norm[0] > 0.0) || !(norm[3] <= 1e300)) return;
   const double* __restrict__ x = (sout->nupd & 1) ? x1 : x0;
   const size_t total = (size_t)n * n;
   for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -319,9 +319,9 @@ __global__ void k_finish_solve_f64(const double* __restrict__ x0, const double* 
 }
 
 cudaError_t launch_finish_solve_f64(const double* x0, const double* x1, const SolveOut* sout,
-                                    const double* norm, int np, int n, double* rho, int ld,
-                                    cudaStream_t st) {
-  k_finish_solve_f64<<<elem_grid(np), 256, 0, st>>>(x0, x1, sout, norm, np, n, rho, ld);
+                                    const int* err, const double* norm, int np, int n, double* rho,
+                                    int ld, cudaStream_t st) {
+  k_finish_solve_f64<<<elem_grid(np), 256, 0, st>>>(x0, x1, sout, err, norm, np, n, rho, ld);
   note_launch();
   return cudaGetLastError();
 }

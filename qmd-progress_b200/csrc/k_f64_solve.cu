@@ -15,12 +15,18 @@ namespace sp2b {
 
 namespace {
 
-// Waits (bounded) until *word >= target; false when the wait ran out or another CTA gave up.
-__device__ __forceinline__ bool spin_until(const unsigned* word, unsigned target, const int* err) {
-  for (uint32_t it = 0; it < kSpinLimit; ++it) {
+// Set in the barrier counter by a CTA that gave up, before it arrives: the others learn of it
+// from the word they poll (counts stay below it: CTAs x steps of a launch).
+constexpr unsigned kGaveUp = 0x80000000u;
+
+// Waits (at most `limit` polls) until *word >= target; false when the wait ran out or another
+// CTA gave up.
+__device__ __forceinline__ bool spin_until(const unsigned* word, unsigned target, const int* err,
+                                           uint32_t limit) {
+  for (uint32_t it = 0; it < limit; ++it) {
     unsigned v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
-    if (v >= target) return true;
+    if (v >= target) return !(v & kGaveUp);
     if ((it & 63) == 63 && *(volatile const int*)err) return false;
   }
   return false;
@@ -163,7 +169,8 @@ __global__ void __launch_bounds__(F64Tile<BT>::NT + 32, 1)
         fence_proxy_async_global();   // the other CTAs' X_k, then the TMA reads
         const CUtensorMap* mx = &maps.x[k & 1];
         const CUtensorMap* md = &maps.d[k & 1];
-        for (int seg = 0; seg < nseg; ++seg) {
+        bool ok = true;
+        for (int seg = 0; seg < nseg && ok; ++seg) {
           int job, k0, k1, bi, bj;
           segment(seg, job, k0, k1);
           const bool isx = job < p.ntiles;
@@ -171,8 +178,11 @@ __global__ void __launch_bounds__(F64Tile<BT>::NT + 32, 1)
           const bool one = isx && bi == bj;   // a diagonal tile of X^2: A and B are the same
           for (int kk = k0; kk < k1; ++kk, ++g) {
             const int st = g % C::ST;
-            if (g >= (uint32_t)C::ST)
-              mbar_wait(smem_u32(&bar_empty[st]), (g / C::ST - 1) & 1, &s_abort);
+            if (g >= (uint32_t)C::ST &&
+                !mbar_wait(smem_u32(&bar_empty[st]), (g / C::ST - 1) & 1, &s_abort)) {
+              ok = false;   // no copy into a stage that may still be read
+              break;
+            }
             const uint32_t fb = smem_u32(&bar_full[st]), dst = sbase + st * C::STAGE;
             const bool second = kk >= p.kb;   // Delta X after X Delta
             const int row = (second ? kk - p.kb : kk) * C::BK;
@@ -226,7 +236,8 @@ __global__ void __launch_bounds__(F64Tile<BT>::NT + 32, 1)
                 acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
               }
           }
-          mbar_wait(smem_u32(&bar_full[st]), (g / C::ST) & 1, &s_abort);
+          // (after a wait that ran out s_abort is set: the step's sums and tiles are void)
+          if (!mbar_wait(smem_u32(&bar_full[st]), (g / C::ST) & 1, &s_abort)) break;
           const uint32_t a = sbase + st * C::STAGE;
           C::mma(a, a + boff, am8, bn8, frag, acc);
           __syncwarp();
@@ -262,7 +273,8 @@ __global__ void __launch_bounds__(F64Tile<BT>::NT + 32, 1)
           for (int q = 0; q < s_npiece; ++q) {
             const int c = s_piece[q];
             if (tid == 0 && !s_abort &&
-                !spin_until(p.flags + c, (unsigned)(k + 1 - p.k0), p.err))
+                !spin_until(p.flags + c, (unsigned)(k + 1 - p.k0), p.err,
+                            p.test_wait == 1 ? 0u : kSpinLimit))
               s_abort = 1;
             consumer_sync<C::NT>();
             const double2* w = reinterpret_cast<const double2*>(p.ws) + (size_t)c * (BT * BT / 2) + tid;
@@ -334,11 +346,21 @@ __global__ void __launch_bounds__(F64Tile<BT>::NT + 32, 1)
     if (tid == 0) {
       // (the barrier above and this release order the whole block's stores)
       for (int q = 0; q < kSums; ++q) part[(size_t)q * G + cta] = s[q];
-      add_release(p.bar);
-      if (!s_abort && !spin_until(p.bar, (unsigned)G * (unsigned)(k + 1 - p.k0), p.err)) s_abort = 1;
+      // A wait that ran out is on record before this CTA arrives, so that no CTA passes the
+      // barrier on its account and publishes the step as good.
       if (s_abort) {
-        // the call reports SP2B_TIMEOUT; the other CTAs leave at their next wait
         atomicExch(p.err, 1);
+        atomicOr(p.bar, kGaveUp);
+      }
+      add_release(p.bar);
+      if (!s_abort && !spin_until(p.bar, (unsigned)G * (unsigned)(k + 1 - p.k0), p.err,
+                                  p.test_wait == 2 ? 0u : kSpinLimit))
+        s_abort = 1;
+      if (s_abort) {
+        // the call reports SP2B_TIMEOUT (it reads the error word); the other CTAs leave at
+        // this barrier or at their next wait
+        atomicExch(p.err, 1);
+        atomicOr(p.bar, kGaveUp);
         p.sout->status = SP2B_TIMEOUT;
         __threadfence();
         p.sout->done = 1;

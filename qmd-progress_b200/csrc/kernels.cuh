@@ -111,6 +111,7 @@ struct F64SolveArgs {
   double* trd_out;      // Tr Delta' of the last step taken (may be null)
   SolveOut* sout;
   int* err;
+  int test_wait;        // self-test: 1 the waits for pieces run out, 2 the grid barrier's
   // set by launch_f64_solve
   int ld, kb, ntiles, snap;
   double* ws;           // one BT x BT piece per CTA
@@ -130,11 +131,11 @@ cudaError_t launch_f64_solve(const F64SolveArgs& a, int n, int np, double* work,
 cudaError_t launch_finish_f64(const double* x, int np, int n, double scale, double* rho,
                               int ld, cudaStream_t st);
 // rho = 2 X of the iterate that a finished solve left in x[nupd & 1], chosen on the device;
-// nothing when the solve has not ended or its normalisation (norm: bounds, trace,
-// ||X0||_F^2) was not finite.
+// nothing when the solve has not ended, a wait in it ran out (*err) or its normalisation
+// (norm: bounds, trace, ||X0||_F^2) was not finite.
 cudaError_t launch_finish_solve_f64(const double* x0, const double* x1, const SolveOut* sout,
-                                    const double* norm, int np, int n, double* rho, int ld,
-                                    cudaStream_t st);
+                                    const int* err, const double* norm, int np, int n, double* rho,
+                                    int ld, cudaStream_t st);
 cudaError_t launch_copy_in(const double* src, int n, int ld, int np, double* x,
                            cudaStream_t st);
 cudaError_t launch_mirror_lower(double* a, int n, int ld, cudaStream_t st);

@@ -40,15 +40,17 @@ struct Ctx {
   double* rowsum = nullptr;
   size_t rowsum_cap = 0;
   // one small device block and its pinned mirror: scratch scalars, then what a solve reads
-  // back in one copy (the normalisation's {min, max, trace, ||X0||^2} and the outcome), then
-  // the reduction counters and the error word
+  // back in one copy: the normalisation's {min, max, trace, ||X0||^2}, the outcome, the
+  // reduction counters and the error word
   double* small = nullptr;
   double* h_small = nullptr;
   double* norm_out = nullptr;   // small + kNorm
   SolveOut* sout = nullptr;     // behind norm_out
   SolveOut* h_sout = nullptr;
   int* err = nullptr;
-  static constexpr int kNorm = 48, kBack = 7;   // doubles read back: 4 + sizeof(SolveOut) / 8
+  const int* h_err = nullptr;
+  // doubles read back: 4, sizeof(SolveOut) / 8, four counters, the error word
+  static constexpr int kNorm = 48, kBack = 4 + 3 + 2 + 1;
   cudaEvent_t poll = nullptr;   // the outcome copy of a poll
   char* pin = nullptr;          // pinned: pp, vv and the refinement's scale of a solve
   size_t pin_cap = 0;
@@ -71,7 +73,7 @@ struct Ctx {
   cudaError_t clear_control(cudaStream_t st) {
     return cudaMemsetAsync(sout, 0, (char*)(err + 1) - (char*)sout, st);
   }
-  // norm_out and the outcome into the pinned mirror
+  // norm_out, the outcome and the error word into the pinned mirror
   cudaError_t read_back(cudaStream_t st) {
     return cudaMemcpyAsync(h_small + kNorm, norm_out, kBack * sizeof(double),
                            cudaMemcpyDeviceToHost, st);
@@ -112,6 +114,7 @@ struct DenseJob {
   int exact_switch;      // mixed: steps after which a still-running loop restarts exact
   const double* h1;      // forward-mode response: perturbation H1 (nullptr: plain solve)
   double* rsp;           // ... and its output, the response rho1 = 2 Delta
+  int test_wait;         // self-test of an FP64 solve's bounded waits (F64SolveArgs)
 };
 
 int dense_solve(const DenseJob& j);

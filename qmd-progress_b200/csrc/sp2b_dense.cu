@@ -74,6 +74,7 @@ Ctx* get_ctx(int* status) {
     c.h_sout = reinterpret_cast<SolveOut*>(c.h_small + Ctx::kNorm + 4);
     c.counter = reinterpret_cast<unsigned*>(c.sout + 1);
     c.err = reinterpret_cast<int*>(c.counter + 4);
+    c.h_err = reinterpret_cast<const int*>(c.h_small + (reinterpret_cast<double*>(c.err) - c.small));
     c.dev = dev;
     c.init = true;
   }
@@ -358,6 +359,7 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
   fa.pp_out = pp_out_dev;
   fa.vv_out = c->vv_dev;
   fa.vv_accumulate = j.vv_accumulate;
+  fa.test_wait = j.test_wait;
   // pp and vv leave through pinned memory, all that a solve of maxlaunch steps can write
   const size_t pin_vv = 0, pin_pp = (size_t)(maxlaunch + 2) * sizeof(double);
   const size_t pin_sc = (pin_pp + (size_t)(maxlaunch + 2) * sizeof(int) + 7) / 8 * 8;
@@ -450,11 +452,11 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
       if (timing) SP2B_CUDA_TRY(cudaEventRecord(c->ev[1], st));
       k = kend;
       if (at_once) {
-        SP2B_CUDA_TRY(launch_finish_solve_f64(c->x64[0], c->x64[1], c->sout, c->norm_out, np, n,
-                                              j.rho, n, st));
+        SP2B_CUDA_TRY(launch_finish_solve_f64(c->x64[0], c->x64[1], c->sout, c->err, c->norm_out,
+                                              np, n, j.rho, n, st));
         if (resp)
-          SP2B_CUDA_TRY(launch_finish_solve_f64(c->x64[2], c->x64[3], c->sout, c->norm_out, np, n,
-                                                j.rsp, n, st));
+          SP2B_CUDA_TRY(launch_finish_solve_f64(c->x64[2], c->x64[3], c->sout, c->err, c->norm_out,
+                                                np, n, j.rsp, n, st));
         SP2B_CUDA_TRY(queue_sequences());
       }
       SP2B_CUDA_TRY(poll());
@@ -504,6 +506,12 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
   SolveOut so = *c->h_sout;
   if (maxlaunch == 0) so.nupd = 0;
   c->last_launches = fp64 ? so.nupd : k;   // FP64: the steps taken inside the launches
+  // The error word, not the outcome's status alone: a CTA may have published its step before
+  // another one's wait ran out.
+  if (*c->h_err) {
+    set_last_error("a device-side wait timed out");
+    return SP2B_TIMEOUT;
+  }
   // the stop reason: Tr X - Tr P of the last update above mixed_tol means the stagnation
   // test (or maxsp2iter) ended the loop
   if (fallback && so.nupd > 0 &&
@@ -1053,6 +1061,23 @@ int sp2b_selftest_wait_timeout(int spin_limit) {
     return SP2B_TIMEOUT;
   }
   return SP2B_OK;
+}
+
+int sp2b_selftest_solve_timeout(int wait) {
+  if (wait != 1 && wait != 2) {
+    set_last_error("wait must be 1 or 2");
+    return SP2B_BAD_ARG;
+  }
+  // one step of an order whose tiles are cut between CTAs
+  const int n = 449, pp = BR_X2;
+  std::vector<double> h((size_t)n * n, 0.0), rho((size_t)n * n);
+  for (int i = 0; i < n; ++i) h[(size_t)i * n + i] = (double)i / n;
+  DenseJob j = base_job(h.data(), rho.data(), n, nullptr);
+  j.ctl.algo = ALGO_SEQ;
+  j.ctl.icount = 1;
+  j.pp_in = &pp;
+  j.test_wait = wait;
+  return dense_solve(j);
 }
 
 long long sp2b_launch_count(void) { return g_launches.load(); }

@@ -115,6 +115,7 @@ _SIGS = {
                                        C.c_char_p, C.c_double, C.c_double, _i, _vp, _ip, _vp]),
     "sp2b_refinement_timing": (_i, [_dp, C.POINTER(C.c_longlong)]),
     "sp2b_selftest_wait_timeout": (_i, [_i]),
+    "sp2b_selftest_solve_timeout": (_i, [_i]),
     "sp2b_set_step_timing": (_i, [_i]),
     "sp2b_step_timing": (_i, [_dp, _llp]),
     # PROGRESS-named exports

@@ -79,3 +79,19 @@ def test_solve_of_several_launches(cuda):
     assert np.linalg.norm(got.rho - ref) <= 1e-9 * np.linalg.norm(ref)
     seq = sp2b.sp2_alg2_seq(h, got.pp, got.icount)
     assert np.array_equal(seq.rho, got.rho)
+
+
+@pytest.mark.parametrize("wait", [1, 2])
+def test_a_wait_that_runs_out_is_reported(cuda, wait):
+    """The waits for another CTA's piece of a tile, or at the grid barrier, run out in the last
+    step of a solve: the call says so although other CTAs finished and published that step,
+    and the next solve is sound."""
+    from sp2b import _lib
+    L = _lib.lib()
+    for _ in range(3):
+        assert L.sp2b_selftest_solve_timeout(wait) == _lib.SP2B_TIMEOUT
+        assert "timed out" in _lib.last_error()
+    h = M.two_band_1d(448, seed=448)
+    ref = O.sp2_alg2(h, 0.5, 0, 100, "None", 1e-10)
+    got = sp2b.sp2_alg2(h, 0.5, 0, 100, "None", 1e-10)
+    assert np.linalg.norm(got.rho - ref.rho) <= TOL * np.linalg.norm(ref.rho)
