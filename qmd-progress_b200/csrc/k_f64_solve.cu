@@ -236,8 +236,9 @@ __global__ void __launch_bounds__(F64Tile<BT>::NT + 32, 1)
                 acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
               }
           }
-          // (after a wait that ran out s_abort is set: the step's sums and tiles are void)
-          if (!mbar_wait(smem_u32(&bar_full[st]), (g / C::ST) & 1, &s_abort)) break;
+          // A wait that ran out leaves s_abort set and the step void, but every lane goes on: the
+          // multiply needs the whole warp, and lanes give up each for itself.
+          mbar_wait(smem_u32(&bar_full[st]), (g / C::ST) & 1, &s_abort);
           const uint32_t a = sbase + st * C::STAGE;
           C::mma(a, a + boff, am8, bn8, frag, acc);
           __syncwarp();
