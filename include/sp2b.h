@@ -439,7 +439,8 @@ int sp2b_last_refinement_info(int* scale_exp, double* r2max);
 int sp2b_selftest_wait_timeout(int spin_limit);
 /* The same through a whole dense FP64 solve (one step, n = 449, host memory): the waits of its
  * persistent launch for another block's piece of a tile (wait = 1) or at its grid barrier (2)
- * run out at once.  SP2B_TIMEOUT when the call reports it. */
+ * run out at once; wait = 3: the wait of the FP64 sub-graph launch for a part's step, on a part
+ * of one tile.  SP2B_TIMEOUT when the call reports it. */
 int sp2b_selftest_solve_timeout(int wait);
 int sp2b_set_step_timing(int enable);
 int sp2b_step_timing(double* ms, long long* launches);

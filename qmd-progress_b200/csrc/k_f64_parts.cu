@@ -2,6 +2,7 @@
 // part, in any number of parts (the whole batch, or the few parts that a reduced-precision
 // solve flags for FP64).
 #include <algorithm>
+#include <cstring>
 
 #include "f64_tile.cuh"
 #include "kernels_subgraph.cuh"
@@ -27,6 +28,8 @@ struct F64PartsMaps {
 //
 // Tiles and k-blocks stop at the part's size (edge and 16), not at the 128-padded one, and
 // every element sums k in ascending order whatever the edge: results do not depend on it.
+// A consumer's own wait ends unless a copy never arrives: the loader issues every k-block of an
+// item that it announces, and the end mark last, whatever ended it.
 // Residual sums go out per tile and warp and are added in a fixed order afterwards.
 //
 // Bound by the DMMA pipe, and for a few parts by the chain of one step: operand latency,
@@ -71,13 +74,20 @@ __global__ void __launch_bounds__(F64Tile<BT>::NT + 32, BT == 32 ? 2 : 1)
           const int part = p.tpart[t];
           const unsigned need = (unsigned)p.pnt[part] * (unsigned)k;
           ok = false;
-          for (uint32_t it = 0; it < kSpinLimit; ++it) {
+          for (uint32_t it = 0; it < p.polls; ++it) {
             unsigned v;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p.done + part) : "memory");
             if (v >= need) { ok = true; break; }
             if ((it & 63) == 63 && *(volatile const int*)p.err) break;
           }
-          if (!ok) break;
+          if (!ok) {
+            // The call reports SP2B_TIMEOUT.  The consumers learn of it in the order of the
+            // items, by the end mark: all warps finish what was loaded and leave together (one
+            // that left by itself would keep the others at the barrier of its tile).
+            atomicExch(p.err, 1);
+            ok = true;
+            break;
+          }
           fence_proxy_async_global();   // the other CTAs' results, then the TMA reads
         }
         const CUtensorMap* mx = &maps.x[k & 1];
@@ -104,9 +114,15 @@ __global__ void __launch_bounds__(F64Tile<BT>::NT + 32, BT == 32 ? 2 : 1)
           s_item[st] = -1;
           mbar_arrive(smem_u32(&bar_full[st]));
         }
+        // every stage consumed: no consumer gave up (asked here and not by the consumers: code
+        // behind their loop makes the compiler reconverge inside it, 6 % at 16^3)
+        for (uint32_t u = g > (uint32_t)C::ST ? g - C::ST : 0; u < g; ++u)
+          if (!mbar_wait(smem_u32(&bar_empty[u % C::ST]), (u / C::ST) & 1, &s_abort)) {
+            atomicExch(p.err, 1);
+            break;
+          }
       } else {
-        // a wait ran out: the call reports SP2B_TIMEOUT; no copy stays in flight
-        s_abort = 1;
+        // no stage came free: the consumers gave up too (s_abort); no copy stays in flight
         atomicExch(p.err, 1);
         for (uint32_t u = g > (uint32_t)C::ST ? g - C::ST : 0; u < g; ++u)
           for (uint32_t i = 0; i < kSpinLimit; ++i)
@@ -231,8 +247,10 @@ size_t f64_parts_partials(int ntiles, int nsteps, int bt) {
   return (size_t)ntiles * nsteps * (bt == 32 ? F64Tile<32>::NW : F64Tile<64>::NW);
 }
 
-cudaError_t launch_f64_parts(const F64PartsArgs& a, int bt, long long rows, double* vv,
+cudaError_t launch_f64_parts(const F64PartsArgs& a0, int bt, long long rows, double* vv,
                              cudaStream_t st) {
+  F64PartsArgs a = a0;
+  if (a.polls == 0) a.polls = kSpinLimit;
   if (a.ntiles <= 0 || a.nsteps <= 0) return cudaSuccess;
   // item numbers are 32-bit
   if ((long long)a.ntiles * a.nsteps > 0x7fffffffLL - 4096) return cudaErrorInvalidValue;
@@ -242,6 +260,44 @@ cudaError_t launch_f64_parts(const F64PartsArgs& a, int bt, long long rows, doub
   k_f64_parts_sums<<<a.nsteps, 256, 0, st>>>(a.partials, per, vv);
   note_launch();
   return cudaGetLastError();
+}
+
+// One part of one tile, two steps.  With two tiles to wait for after the first step, the
+// second step's wait runs out after `polls` polls; with one, the launch ends without error.
+cudaError_t launch_f64_parts_selftest(double* x0, double* x1, void* scratch, int bt, int tiles_awaited,
+                                      uint32_t polls, int* err, cudaStream_t st) {
+  constexpr int ld = 128;
+  struct Lists {
+    int4 tile;
+    int tpart, pnt, pp[2];
+    unsigned done, ticket;
+  } h;
+  memset(&h, 0, sizeof(h));
+  h.tile = make_int4(0, 0, 32, 32);
+  h.pnt = tiles_awaited;
+  cudaError_t e = cudaMemsetAsync(x0, 0, (size_t)ld * ld * sizeof(double), st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(scratch, &h, sizeof(h), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(err, 0, sizeof(int), st);
+  if (e != cudaSuccess) return e;
+  Lists* d = static_cast<Lists*>(scratch);
+  F64PartsArgs a;
+  memset(&a, 0, sizeof(a));
+  a.x[0] = x0;
+  a.x[1] = x1;
+  a.tiles = &d->tile;
+  a.tpart = &d->tpart;
+  a.pnt = &d->pnt;
+  a.pp = d->pp;
+  a.done = &d->done;
+  a.ticket = &d->ticket;
+  a.err = err;
+  a.ntiles = 1;
+  a.nsteps = 2;
+  a.ld = ld;
+  a.polls = polls;
+  e = launch_f64_parts(a, bt, ld, nullptr, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);   // (h leaves scope)
+  return e;
 }
 
 }  // namespace sp2b

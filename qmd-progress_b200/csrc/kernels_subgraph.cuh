@@ -58,10 +58,14 @@ struct F64PartsArgs {
   double* partials;     // residual sums, f64_parts_partials() doubles (null: not formed)
   int* err;
   int ntiles, nsteps, ld;
+  uint32_t polls;       // bound of a tile's wait for its part (0: kSpinLimit)
 };
 size_t f64_parts_partials(int ntiles, int nsteps, int bt);
 cudaError_t launch_f64_parts(const F64PartsArgs& a, int bt, long long rows, double* vv,
                              cudaStream_t st);
+// Self-test of its bounded waits on 128 x 128 buffers and 64 bytes of scratch.
+cudaError_t launch_f64_parts_selftest(double* x0, double* x1, void* scratch, int bt, int tiles_awaited,
+                                      uint32_t polls, int* err, cudaStream_t st);
 
 // Batched INT8 digit-split form (exact INT8 precision of the sub-graph loop): the
 // iterate as four signed 8-bit planes of M = rint(2^31 (X - I/2)) in each packed buffer

@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "kernels.cuh"
+#include "kernels_subgraph.cuh"
 #include "sp2b_ctx.h"
 
 namespace sp2b {
@@ -1063,11 +1064,35 @@ int sp2b_selftest_wait_timeout(int spin_limit) {
   return SP2B_OK;
 }
 
+// A sub-graph launch whose waits end, then one whose second step waits for a tile too many.
+static int selftest_parts_timeout() {
+  int status = SP2B_OK;
+  Ctx* c = get_ctx(&status);
+  if (!c) return status;
+  std::lock_guard<std::mutex> lk(c->mu);
+  SP2B_CUDA_TRY(c->ensure_f64(128, 3));
+  for (int bt : {32, 64})
+    for (int awaited : {1, 2}) {
+      SP2B_CUDA_TRY(launch_f64_parts_selftest(c->x64[0], c->x64[1], c->x64[2], bt, awaited, 4096,
+                                              c->err, c->stream));
+      int herr = 0;
+      SP2B_CUDA_TRY(cudaMemcpy(&herr, c->err, sizeof(int), cudaMemcpyDeviceToHost));
+      if ((herr != 0) != (awaited == 2)) {
+        set_last_error("self-test: FP64 parts, edge %d, %d tiles awaited: error word %d", bt, awaited,
+                       herr);
+        return SP2B_CUDA_ERROR;
+      }
+    }
+  set_last_error("a device-side wait timed out");
+  return SP2B_TIMEOUT;
+}
+
 int sp2b_selftest_solve_timeout(int wait) {
-  if (wait != 1 && wait != 2) {
-    set_last_error("wait must be 1 or 2");
+  if (wait < 1 || wait > 3) {
+    set_last_error("wait must be 1, 2 or 3");
     return SP2B_BAD_ARG;
   }
+  if (wait == 3) return selftest_parts_timeout();
   // one step of an order whose tiles are cut between CTAs
   const int n = 449, pp = BR_X2;
   std::vector<double> h((size_t)n * n, 0.0), rho((size_t)n * n);

@@ -65,3 +65,13 @@ def test_parts_against_oracle_with_both_edges(cuda, sizes):
         sp2b.tune_set(key, ch)
     assert np.array_equal(core, core2)
     assert np.allclose(vv2, vv, rtol=TOL, atol=0)
+
+
+def test_a_wait_that_runs_out_is_reported(cuda):
+    """A part's second step waits for a tile that nothing finishes: every thread of the launch
+    leaves, the error is on record, and the next solve is sound."""
+    from sp2b import _lib
+    L = _lib.lib()
+    for _ in range(3):
+        assert L.sp2b_selftest_solve_timeout(3) == _lib.SP2B_TIMEOUT, _lib.last_error()
+    test_parts_against_oracle_with_both_edges(cuda, [63, 64, 65])
