@@ -203,6 +203,17 @@ static cudaStream_t pick_stream(const sp2b_opts* o, Ctx* c) {
 
 static thread_local int t_exact_switch = 0;   // the last solve restarted in the exact form
 
+// Waits for a stream when a call leaves, unless the call ends with its own wait.  The context's
+// buffers and done word go to the next call, on whatever stream that one runs: steps still in
+// flight would take its records and iterates for their own.
+struct WaitOnReturn {
+  cudaStream_t st;
+  bool armed = true;
+  ~WaitOnReturn() {
+    if (armed) cudaStreamSynchronize(st);
+  }
+};
+
 // One solve.  A mixed trace-driven solve with exact_switch > 0 sets *want_exact and
 // returns without writing its outputs when its loop shows a spectrum the split products
 // cannot resolve: still running after exact_switch steps, or stopped on the stagnation
@@ -242,6 +253,7 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
     set_last_error("bad argument: precision %d", j.prec);
     return SP2B_BAD_ARG;
   }
+  WaitOnReturn leave{st};
   int maxlaunch;
   if (j.ctl.algo == ALGO_SEQ) maxlaunch = j.ctl.icount;
   else if (j.ctl.algo == ALGO_BASIC) maxlaunch = j.ctl.maxit + 1;
@@ -619,6 +631,7 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
     }
     SP2B_CUDA_TRY(cudaStreamSynchronize(st));
   }
+  leave.armed = false;   // (at_once: the poll waited)
   if (oz) {
     int S = 0, herr = 0;
     double r2max = 0.0;

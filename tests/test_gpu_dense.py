@@ -359,3 +359,30 @@ def test_alg2_genseq_fp64_parity_config1_size(cuda):
     assert got.icount == ref.icount
     assert rel(got.rho, ref.rho) <= FP64_TOL
     assert np.allclose(got.vv, ref.vv, rtol=1e-9, atol=1e-12)
+
+
+@pytest.mark.parametrize("prec", [sp2b.PREC_MIXED_FP16, sp2b.PREC_EXACT_INT8, sp2b.PREC_FP64])
+def test_refused_input_leaves_nothing_in_flight(cuda, prec):
+    """A solve that ends with an error has no step left on its stream, where the next call on
+    another stream would share the context's buffers with it."""
+    torch = cuda
+    n = 2048
+    good = torch.from_numpy(M.two_band_1d(n, seed=1)).cuda()
+    bad = good.clone()
+    bad[3, 5] = bad[5, 3] = float("nan")
+    rho = torch.empty_like(good)
+    L = _lib.lib()
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+
+    def solve(h, stream):
+        o = _lib.make_opts(precision=prec, device_ptrs=True, stream=stream.cuda_stream)
+        return L.sp2b_sp2_alg2(h.data_ptr(), rho.data_ptr(), n, 0.0, 0.5, 0, 100, b"None", 1e-10, 0,
+                               C.byref(o), None)
+    assert solve(good, s2) == 0
+    want = rho.clone()
+    for _ in range(10):
+        assert solve(bad, s1) == _lib.SP2B_BAD_INPUT
+        assert s1.query()
+        assert solve(good, s2) == 0
+        assert torch.equal(rho, want)
