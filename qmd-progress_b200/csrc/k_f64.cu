@@ -3,6 +3,7 @@
 #include <algorithm>
 #include <cstring>
 #include <string>
+#include <vector>
 
 #include "f64_dmma.cuh"
 #include "reduce.cuh"
@@ -462,8 +463,9 @@ __global__ void __launch_bounds__(WM* WN * 32, 1) k_sym_gemm_f64(const StepArgs 
   publish_and_finalize(p, s, red, &s_flag);
 }
 
-// Tile edge of a single dense FP64 product of padded size np: the solve's measured choice
-// for this device and size (tune_f64_solve) when one was made, else 128 once its tiles fill the SMs twice, else 64.
+// Tile edge of a single dense FP64 product of padded size np: the measured choice for this
+// device and size (tune_f64_tile) when one was made, else 128 once its tiles fill the SMs
+// twice, else 64.
 int f64_tile(int np) {
   int c = 0;
   if (tune_lookup(f64_tune_key(np), &c) && (c == 64 || c == 128)) return c;
@@ -503,6 +505,42 @@ cudaError_t launch_sym_gemm_f64(const StepArgs& a0, cudaStream_t st) {
   const int t = a.np / bt;
   a.ntiles = t * (t + 1) / 2;   // the partial sums the last CTA reduces: one per launched tile
   return launch_f64_bt(a, bt, a.ntiles, st);
+}
+
+// Measures the edges 128 and 64 of a single product at np (x_in -> x_out, the same k order
+// per element in both, so the choice changes no result) and records the faster one for
+// f64_tile.  partials must hold 4 doubles per 64-edge tile.
+int tune_f64_tile(int np, const double* x_in, double* x_out, double* partials, unsigned* counter,
+                  double* sums_out, cudaStream_t st) {
+  int c = 0;
+  const std::string key = f64_tune_key(np);
+  if (!tune_enabled() || tune_lookup(key, &c)) return SP2B_OK;
+  const int edges[2] = {128, 64};
+  StepArgs q;
+  memset(&q, 0, sizeof(q));
+  q.np = np;
+  q.ld = np;
+  q.A = q.B = q.E = x_in;
+  q.out = x_out;
+  q.alpha = 1.0;
+  q.partials = partials;
+  q.counter = counter;
+  q.sums_out = sums_out;
+  // timed on zeros (the buffer may not hold data yet; DMMA time does not depend on values)
+  if (cudaMemsetAsync(const_cast<double*>(x_in), 0, (size_t)np * np * sizeof(double), st) !=
+      cudaSuccess)
+    return SP2B_CUDA_ERROR;
+  std::vector<float> ms;
+  int best = 0;
+  const int rc = tune_measure(2, 2, st, [&](int cand) -> int {
+    const int t = np / edges[cand];
+    return cudaMemsetAsync(counter, 0, 4 * sizeof(unsigned), st) == cudaSuccess &&
+                   launch_f64_bt(q, edges[cand], t * (t + 1) / 2, st) == cudaSuccess
+               ? SP2B_OK
+               : SP2B_CUDA_ERROR;
+  }, &ms, &best);
+  if (rc == SP2B_OK) tune_store(key, edges[best], ms);
+  return rc;
 }
 
 }  // namespace sp2b

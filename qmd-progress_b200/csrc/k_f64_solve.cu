@@ -445,11 +445,14 @@ cudaError_t launch_solve(const F64SolveArgs& a, int grid, cudaStream_t st) {
 // Tile edge of an order-n solve: 32 up to kF64SmallN, where 64-edge tiles are too few for the
 // SMs (n = 300: 235 us a solve with 32, 270 us with 64; n = 500: 296 and 284); above it the
 // measured choice for this device and padded size (tune_f64_solve), else 64.
+static std::string f64_solve_key(int np) {
+  return "f64-solve/sm" + std::to_string(device_sms()) + "/np" + std::to_string(np);
+}
 int f64_solve_tile(int n, int np, bool resp) {
   if (n <= kF64SmallN) return 32;
   int c = 0;
   if (resp) return 64;   // a 128-edge tile of sums does not fit beside the stages
-  return tune_lookup(f64_tune_key(np), &c) && (c == 64 || c == 128) ? c : 64;
+  return tune_lookup(f64_solve_key(np), &c) && (c == 64 || c == 128) ? c : 64;
 }
 
 // Steps per launch: a launch stays below a tenth of a second (30 TFLOP/s of symmetric
@@ -493,7 +496,7 @@ cudaError_t launch_f64_solve(const F64SolveArgs& a, int n, int np, double* work,
 int tune_f64_solve(int n, int np, const F64SolveArgs& a0, double* work, size_t cap,
                    cudaStream_t st) {
   int c = 0;
-  const std::string key = f64_tune_key(np);
+  const std::string key = f64_solve_key(np);
   if (n <= kF64SmallN || a0.d[0] || !tune_enabled() || tune_lookup(key, &c)) return SP2B_OK;
   F64SolveArgs a = a0;
   a.k0 = 0;

@@ -95,3 +95,30 @@ def test_a_wait_that_runs_out_is_reported(cuda, wait):
     ref = O.sp2_alg2(h, 0.5, 0, 100, "None", 1e-10)
     got = sp2b.sp2_alg2(h, 0.5, 0, 100, "None", 1e-10)
     assert np.linalg.norm(got.rho - ref.rho) <= TOL * np.linalg.norm(ref.rho)
+
+
+@pytest.mark.parametrize("n", [500, 1000, 1300])
+def test_single_product_edge_choice_changes_no_bit(cuda, n):
+    """The recorded edge of single FP64 products ("f64-step/...") is theirs alone, measured on
+    them, and either one gives the same bits: a solve, and a refinement by FP64 products."""
+    h = M.two_band_1d(n, seed=5)
+    sms = cuda.cuda.get_device_properties(0).multi_processor_count
+    key = f"f64-step/sm{sms}/np{(n + 127) // 128 * 128}"
+
+    def results():
+        r = sp2b.sp2_alg2(h, 0.5, 0, 100, "Rel", 1e-10)
+        m = sp2b.sp2_alg2(h, 0.5, 0, 100, "None", 1e-10, precision=sp2b.PREC_MIXED_FP16,
+                          mcweeny_products=sp2b.MCW_FP64)
+        return r.rho, m.rho
+    first = results()
+    choice, ms = sp2b.tune_get(key)
+    assert choice in (64, 128)
+    if len(ms) == 2:
+        assert ms[(128, 64).index(choice)] == min(ms)
+    try:
+        for c in (64, 128):
+            sp2b.tune_set(key, c)
+            for a, b in zip(results(), first):
+                assert np.array_equal(a, b)
+    finally:
+        sp2b.tune_set(key, choice)

@@ -128,7 +128,7 @@ def test_fermi_init_norecs_with_the_other_tile_edge(cuda):
     h = _lattice(8)
     n = h.shape[0]
     sms = cuda.cuda.get_device_properties(0).multi_processor_count
-    key = f"f64-step/sm{sms}/np{(n + 127) // 128 * 128}"
+    key = f"f64-solve/sm{sms}/np{(n + 127) // 128 * 128}"
     was = sp2b.tune_get(key)
     xr, kr, mur, _, _, _, sgnr = O.sp2_fermi_init_norecs(h, 24, 0.5 * n, 1.0, 1e-9, 1e-12, 40.0)
     try:
