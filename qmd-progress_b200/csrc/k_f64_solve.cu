@@ -3,12 +3,9 @@
 // forward-mode response the anticommutator {X, Delta} beside X^2.
 #include <algorithm>
 #include <cstring>
-#include <string>
-#include <vector>
 
 #include "f64_tile.cuh"
 #include "reduce.cuh"
-#include "sp2b_tune.h"
 #include "work_lists.h"
 
 namespace sp2b {
@@ -442,19 +439,6 @@ cudaError_t launch_solve(const F64SolveArgs& a, int grid, cudaStream_t st) {
 
 }  // namespace
 
-// Tile edge of an order-n solve: 32 up to kF64SmallN, where 64-edge tiles are too few for the
-// SMs (n = 300: 235 us a solve with 32, 270 us with 64; n = 500: 296 and 284); above it the
-// measured choice for this device and padded size (tune_f64_solve), else 64.
-static std::string f64_solve_key(int np) {
-  return "f64-solve/sm" + std::to_string(device_sms()) + "/np" + std::to_string(np);
-}
-int f64_solve_tile(int n, int np, bool resp) {
-  if (n <= kF64SmallN) return 32;
-  int c = 0;
-  if (resp) return 64;   // a 128-edge tile of sums does not fit beside the stages
-  return tune_lookup(f64_solve_key(np), &c) && (c == 64 || c == 128) ? c : 64;
-}
-
 // Steps per launch: a launch stays below a tenth of a second (30 TFLOP/s of symmetric
 // products), so that a long solve leaves the GPU to others in between.
 int f64_solve_chunk(int n, bool resp) {
@@ -464,10 +448,11 @@ int f64_solve_chunk(int n, bool resp) {
 
 size_t f64_solve_ws_doubles(int n, bool resp) { return f64_solve_doubles(n, resp, device_sms()); }
 
-static cudaError_t launch_f64_solve_bt(const F64SolveArgs& a0, int n, int np, int bt, double* work,
-                                       size_t cap, cudaStream_t st) {
+cudaError_t launch_f64_solve(const F64SolveArgs& a0, int n, int np, double* work, size_t cap,
+                             cudaStream_t st) {
   F64SolveArgs a = a0;
-  const F64Plan pl = f64_plan(n, bt, a.d[0] != nullptr, device_sms());
+  const bool resp = a.d[0] != nullptr;
+  const F64Plan pl = f64_plan(n, f64_edge(n, resp), resp, device_sms());
   if (!work || f64_plan_doubles(pl) > cap) return cudaErrorInvalidValue;
   a.ld = np;
   a.kb = (n + 15) / 16;
@@ -484,44 +469,6 @@ static cudaError_t launch_f64_solve_bt(const F64SolveArgs& a0, int n, int np, in
   else e = launch_solve<128>(a, pl.grid, st);
   note_launch();
   return e == cudaSuccess ? cudaGetLastError() : e;
-}
-
-cudaError_t launch_f64_solve(const F64SolveArgs& a, int n, int np, double* work, size_t cap,
-                             cudaStream_t st) {
-  return launch_f64_solve_bt(a, n, np, f64_solve_tile(n, np, a.d[0] != nullptr), work, cap, st);
-}
-
-// Measures the tile edges 128 and 64 at np (one SP2 step each) and records the faster one
-// for f64_solve_tile.  `a` as for a solve; its records, sums and iterates are overwritten.
-int tune_f64_solve(int n, int np, const F64SolveArgs& a0, double* work, size_t cap,
-                   cudaStream_t st) {
-  int c = 0;
-  const std::string key = f64_solve_key(np);
-  if (n <= kF64SmallN || a0.d[0] || !tune_enabled() || tune_lookup(key, &c)) return SP2B_OK;
-  F64SolveArgs a = a0;
-  a.k0 = 0;
-  a.k1 = 1;
-  a.ctl.algo = ALGO_SEQ;
-  a.ctl.icount = 1;
-  a.pp_out = nullptr;
-  a.vv_out = nullptr;
-  a.trd_out = nullptr;
-  // timed on zeros (the buffers may not hold data yet; DMMA time does not depend on values)
-  const size_t bytes = (size_t)np * np * sizeof(double);
-  if (cudaMemsetAsync(a.x[0], 0, bytes, st) != cudaSuccess ||
-      cudaMemsetAsync(const_cast<int*>(a.pp_in), 0, sizeof(int), st) != cudaSuccess ||
-      cudaMemsetAsync(a.rec, 0, sizeof(SP2Rec), st) != cudaSuccess ||
-      cudaMemsetAsync(a.err, 0, sizeof(int), st) != cudaSuccess)
-    return SP2B_CUDA_ERROR;
-  const int edges[2] = {128, 64};
-  std::vector<float> ms;
-  int best = 0;
-  const int rc = tune_measure(2, 2, st, [&](int cand) -> int {
-    return launch_f64_solve_bt(a, n, np, edges[cand], work, cap, st) == cudaSuccess ? SP2B_OK
-                                                                                  : SP2B_CUDA_ERROR;
-  }, &ms, &best);
-  if (rc == SP2B_OK) tune_store(key, edges[best], ms);
-  return rc;
 }
 
 }  // namespace sp2b

@@ -121,8 +121,6 @@ struct F64SolveArgs {
   unsigned* flags;      // per CTA: its piece of step k is complete (k + 1 - k0)
   unsigned* bar;        // grid barrier counter
 };
-int f64_solve_tile(int n, int np, bool resp);
-int tune_f64_solve(int n, int np, const F64SolveArgs& a, double* work, size_t cap, cudaStream_t st);
 // Workspace of an order-n solve: with a response also of solves of that order without one.
 size_t f64_solve_ws_doubles(int n, bool resp);
 int f64_solve_chunk(int n, bool resp);

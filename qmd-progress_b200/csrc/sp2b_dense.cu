@@ -283,10 +283,8 @@ static int dense_solve_once(const DenseJob& j, bool* want_exact) {
     fa.sout = c->sout;
     fa.err = c->err;
     SP2B_CUDA_TRY(c->ensure_f64_solve(n, resp));
-    // the measured tile edges for this size, of a single product and of the solve (first solve
-    // at np on this device)
-    int trc = tune_f64_tile(np, c->x64[0], c->x64[1], c->partials, c->counter, c->small + 16, st);
-    if (trc == SP2B_OK) trc = tune_f64_solve(n, np, fa, c->f64w, c->f64w_cap, st);
+    // the measured tile edge of single products at this size (first solve at np on this device)
+    const int trc = tune_f64_tile(np, c->x64[0], c->x64[1], c->partials, c->counter, c->small + 16, st);
     if (trc != SP2B_OK) {
       set_last_error("FP64 tile tuning failed");
       return trc;

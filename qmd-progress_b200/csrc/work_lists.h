@@ -65,8 +65,14 @@ inline F64Plan f64_plan(int n, int bt, bool resp, int sms) {
   return pl;
 }
 
-// Edge 32 up to here, larger ones above (f64_solve_tile).
-constexpr int kF64SmallN = 416;
+// Tile edge of an order-n solve, a rule on n alone: the pieces of cut tiles depend on it, and
+// so the last bits of a result, which are to be the same in every process.  32 up to 416, where
+// 64-edge tiles are too few for the SMs (n = 300: 235 us a solve with 32, 270 us with 64;
+// n = 500: 296 and 284).  128 from 4096 on, without a response (its tile of sums does not fit
+// beside the stages): eight steps at n = 3000 take 7.49 ms with 128 and 7.12 with 64, at 4096
+// 17.40 and 17.55, at 8192 134.3 and 137.7, at 12288 447 and 477.
+inline int f64_edge(int n, bool resp) { return n <= 416 ? 32 : n < 4096 || resp ? 64 : 128; }
+
 constexpr int kF64Sums = 5;   // ||X'||^2, Tr X', ||X - X^2||^2 (core rows), Tr X^2, Tr Delta'
 
 // Workspace of a launch, in doubles: one piece per CTA, the partial sums of two steps, then
@@ -75,24 +81,12 @@ inline size_t f64_plan_doubles(const F64Plan& pl) {
   return (size_t)pl.grid * pl.bt * pl.bt + 2 * (size_t)pl.grid * kF64Sums + pl.grid / 2 + 2;
 }
 
-// The tile edges that a launch of order n may take (returns how many).
-inline int f64_edges(int n, bool resp, int (&bt)[2]) {
-  bt[0] = n <= kF64SmallN ? 32 : 64;
-  bt[1] = 128;
-  return n <= kF64SmallN || resp ? 1 : 2;
-}
-
 // Workspace that covers every launch of order n.  With a response also the launches without
 // one: a set-up for X and Delta serves passes over X alone too (SP2-Fermi generates its
 // sequence that way).
 inline size_t f64_solve_doubles(int n, bool resp, int sms) {
-  size_t w = 0;
-  for (int r = 0; r <= (resp ? 1 : 0); ++r) {
-    int bt[2];
-    const int m = f64_edges(n, r != 0, bt);
-    for (int i = 0; i < m; ++i) w = std::max(w, f64_plan_doubles(f64_plan(n, bt[i], r != 0, sms)));
-  }
-  return w;
+  const size_t w = f64_plan_doubles(f64_plan(n, f64_edge(n, false), false, sms));
+  return resp ? std::max(w, f64_plan_doubles(f64_plan(n, f64_edge(n, true), true, sms))) : w;
 }
 
 // ---- INT8 residue products (k_oz_gemm) ----

@@ -98,9 +98,11 @@ def test_a_wait_that_runs_out_is_reported(cuda, wait):
 
 
 @pytest.mark.parametrize("n", [500, 1000, 1300])
-def test_single_product_edge_choice_changes_no_bit(cuda, n):
-    """The recorded edge of single FP64 products ("f64-step/...") is theirs alone, measured on
-    them, and either one gives the same bits: a solve, and a refinement by FP64 products."""
+def test_recorded_choices_change_no_bit(cuda, n):
+    """No recorded decision changes a result: the edge of single FP64 products ("f64-step/...")
+    is theirs alone, measured on them, and either one gives the same bits, in a solve and in a
+    refinement by FP64 products; the solve's own edge is a rule on n, whatever a decision file
+    holds for it."""
     h = M.two_band_1d(n, seed=5)
     sms = cuda.cuda.get_device_properties(0).multi_processor_count
     key = f"f64-step/sm{sms}/np{(n + 127) // 128 * 128}"
@@ -118,6 +120,7 @@ def test_single_product_edge_choice_changes_no_bit(cuda, n):
     try:
         for c in (64, 128):
             sp2b.tune_set(key, c)
+            sp2b.tune_set(key.replace("step", "solve"), c)
             for a, b in zip(results(), first):
                 assert np.array_equal(a, b)
     finally:

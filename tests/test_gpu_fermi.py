@@ -121,21 +121,17 @@ def test_fermi_init_norecs_matches_oracle(cuda, beta0):
     assert abs(np.trace(x) - nocc) <= 1e-8
 
 
-def test_fermi_init_norecs_with_the_other_tile_edge(cuda):
-    """The generating pass carries X alone in the workspace set up for X and dX/dmu; with the
-    wider tile edge recorded for this size it needs the larger of the two (sizes on the CPU:
-    tests/test_work_lists.py)."""
-    h = _lattice(8)
+def test_fermi_init_norecs_where_the_passes_take_two_tile_edges(cuda):
+    """From n = 4096 on the generating pass over X alone takes wider tiles, and more workspace,
+    than the passes with dX/dmu (sizes on the CPU: tests/test_work_lists.py).  With a target
+    the probe never reaches, norecs is the plain init: the same sequence, mu, beta and X."""
+    h = _lattice(16)
     n = h.shape[0]
-    sms = cuda.cuda.get_device_properties(0).multi_processor_count
-    key = f"f64-solve/sm{sms}/np{(n + 127) // 128 * 128}"
-    was = sp2b.tune_get(key)
-    xr, kr, mur, _, _, _, sgnr = O.sp2_fermi_init_norecs(h, 24, 0.5 * n, 1.0, 1e-9, 1e-12, 40.0)
-    try:
-        sp2b.tune_set(key, 128)
-        x, k, mu, _, _, _, sgn = sp2b.sp2_fermi_init_norecs(h, 24, 0.5 * n, 40.0, 1.0, 1e-9, 1e-12)
-    finally:
-        sp2b.tune_set(key, was[0] if was else 64)
-    assert k == kr and sgn == sgnr
-    assert abs(mu - mur) <= 1e-9 * max(1.0, abs(mur))
-    assert np.linalg.norm(x - xr) <= 1e-10 * np.linalg.norm(xr)
+    nocc, nsteps = 0.5 * n, 12
+    x, k, mu, beta, _, _, sgn = sp2b.sp2_fermi_init_norecs(h, nsteps, nocc, 1e12, 1.0, 1e-9, 1e-12)
+    xi, mui, betai, _, _, sgni = sp2b.sp2_fermi_init(h, nsteps, nocc, 1.0, 1e-9, 1e-12)
+    assert k == nsteps and sgn == sgni
+    assert abs(mu - mui) <= 1e-9 * max(1.0, abs(mui))
+    assert abs(beta - betai) <= 1e-9 * abs(betai)
+    assert np.linalg.norm(x - xi) <= 1e-10 * np.linalg.norm(xi)
+    assert abs(np.trace(x) - nocc) <= 1e-8

@@ -27,8 +27,7 @@ def lists(tmp_path_factory):
 @pytest.mark.parametrize("sms", [148, 132, 7])
 @pytest.mark.parametrize("resp", [0, 1])
 def test_fp64_shares(lists, sms, resp):
-    # every size up to 1300 with the edge its rule gives and the tuner's candidates, then a
-    # few large ones
+    # every size up to 1300 with the edge of its rule and the next one up, then a few large ones
     for n in list(range(1, 1300)) + [2000, 3500, 4097, 8192, 20011, 32768, 65536]:
         for bt in ((32,) if n <= 416 else (64, 128)):
             assert lists.check_f64(n, bt, resp, sms) == 0, (n, bt)

@@ -49,17 +49,16 @@ extern "C" int check_f64(int n, int bt, int resp, int sms) {
 }
 
 // The workspace of an order-n set-up holds every launch that may use it: with a response both
-// the launches with it and those without, at every edge.
+// the launches with it and those without, at the edge each of them takes.
 extern "C" int check_f64_workspace(int n, int resp, int sms) {
   const size_t have = f64_solve_doubles(n, resp != 0, sms);
-  for (int r = 0; r <= resp; ++r)
-    for (int bt : {32, 64, 128}) {
-      if ((bt == 32) != (n <= 416) || (r && bt == 128)) continue;
-      const F64Plan pl = f64_plan(n, bt, r != 0, sms);
-      // pieces, sums of two steps, flags and the barrier counter
-      const size_t words = (size_t)pl.grid + 1;
-      if ((size_t)pl.grid * bt * bt + 10 * (size_t)pl.grid + (words + 1) / 2 > have) return 1 + bt + r;
-    }
+  for (int r = 0; r <= resp; ++r) {
+    const int bt = f64_edge(n, r != 0);
+    const F64Plan pl = f64_plan(n, bt, r != 0, sms);
+    // pieces, sums of two steps, flags and the barrier counter
+    const size_t words = (size_t)pl.grid + 1;
+    if ((size_t)pl.grid * bt * bt + 10 * (size_t)pl.grid + (words + 1) / 2 > have) return 1 + r;
+  }
   return 0;
 }
 
