@@ -439,12 +439,7 @@ cudaError_t launch_solve(const F64SolveArgs& a, int grid, cudaStream_t st) {
 
 }  // namespace
 
-// Steps per launch: a launch stays below a tenth of a second (30 TFLOP/s of symmetric
-// products), so that a long solve leaves the GPU to others in between.
-int f64_solve_chunk(int n, bool resp) {
-  const double flops = (double)n * n * n * (resp ? 3.0 : 1.0);
-  return (int)std::max(1.0, std::min(1e6, 2e12 / flops));
-}
+int f64_solve_chunk(int n, bool resp) { return f64_steps_per_launch(n, resp); }
 
 size_t f64_solve_ws_doubles(int n, bool resp) { return f64_solve_doubles(n, resp, device_sms()); }
 

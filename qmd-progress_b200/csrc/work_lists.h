@@ -73,6 +73,14 @@ inline F64Plan f64_plan(int n, int bt, bool resp, int sms) {
 // 17.40 and 17.55, at 8192 134.3 and 137.7, at 12288 447 and 477.
 inline int f64_edge(int n, bool resp) { return n <= 416 ? 32 : n < 4096 || resp ? 64 : 128; }
 
+// Steps per launch, so that a long solve leaves the GPU to others in between: a launch of more
+// than one step takes about a tenth of a second at most.  Large steps cost their products (30
+// TFLOP/s of symmetric ones), the smallest their fixed 6 us, up to 25 at n = 740.
+inline int f64_steps_per_launch(int n, bool resp) {
+  const double flops = (double)n * n * n * (resp ? 3.0 : 1.0);
+  return (int)std::max(1.0, std::min(5e3, 2e12 / flops));
+}
+
 constexpr int kF64Sums = 5;   // ||X'||^2, Tr X', ||X - X^2||^2 (core rows), Tr X^2, Tr Delta'
 
 // Workspace of a launch, in doubles: one piece per CTA, the partial sums of two steps, then

@@ -40,6 +40,13 @@ def test_fp64_workspace_covers_every_launch(lists, sms):
             assert lists.check_f64_workspace(n, resp, sms) == 0, (n, resp)
 
 
+def test_fp64_launches_stay_short(lists):
+    lists.f64_launch_ms.restype = C.c_double
+    for n in list(range(1, 1300)) + [2000, 4097, 8192, 12000]:
+        for resp in (0, 1):
+            assert lists.f64_launch_ms(n, resp) <= 110.0, (n, resp)
+
+
 @pytest.mark.parametrize("sms", [148, 20])
 def test_int8_product_lists(lists, sms):
     for nb in list(range(1, 40)) + [64, 65, 97]:

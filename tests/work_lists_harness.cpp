@@ -62,6 +62,14 @@ extern "C" int check_f64_workspace(int n, int resp, int sms) {
   return 0;
 }
 
+// Milliseconds of the longest launch of order n: 6 us a step and its products at 30 TFLOP/s
+// (0 when a launch is one step).
+extern "C" double f64_launch_ms(int n, int resp) {
+  const int steps = f64_steps_per_launch(n, resp != 0);
+  const double flops = (double)n * n * n * (resp ? 3.0 : 1.0);
+  return steps <= 1 ? 0.0 : 1e3 * steps * (6e-6 + flops / 30e12);
+}
+
 // Every upper 128-block of every plane once, lists without holes, tiles inside the matrix.
 extern "C" int check_oz(int nb, int planes, int sms) {
   std::vector<int4> w;
