@@ -235,10 +235,12 @@ static cudaError_t launch_parts(const F64PartsArgs& a, long long rows, cudaStrea
   cudaError_t e = cudaFuncSetAttribute(k_f64_parts<BT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)C::SMEM);
   if (e != cudaSuccess) return e;
-  const int grid = std::min(a.ntiles, device_sms() * (BT == 32 ? 2 : 1));
   void* args[] = {(void*)&m, (void*)&a};
-  e = cudaLaunchCooperativeKernel((const void*)k_f64_parts<BT>, dim3(grid), dim3(C::NT + 32), args,
-                                  C::SMEM, st);
+  e = launch_cooperative(st, [&](int sms) {
+    const int grid = std::min(a.ntiles, sms * (BT == 32 ? 2 : 1));
+    return cudaLaunchCooperativeKernel((const void*)k_f64_parts<BT>, dim3(grid), dim3(C::NT + 32),
+                                       args, C::SMEM, st);
+  });
   note_launch();
   return e;
 }

@@ -447,23 +447,25 @@ cudaError_t launch_f64_solve(const F64SolveArgs& a0, int n, int np, double* work
                              cudaStream_t st) {
   F64SolveArgs a = a0;
   const bool resp = a.d[0] != nullptr;
-  const F64Plan pl = f64_plan(n, f64_edge(n, resp), resp, device_sms());
-  if (!work || f64_plan_doubles(pl) > cap) return cudaErrorInvalidValue;
-  a.ld = np;
-  a.kb = (n + 15) / 16;
-  a.ntiles = pl.tiles * (pl.tiles + 1) / 2;
-  a.snap = pl.snap;
-  a.ws = work;
-  a.partials = work + (size_t)pl.grid * pl.bt * pl.bt;
-  a.flags = reinterpret_cast<unsigned*>(a.partials + 2 * (size_t)pl.grid * kSums);
-  a.bar = a.flags + pl.grid;
-  cudaError_t e = cudaMemsetAsync(a.flags, 0, (pl.grid + 1) * sizeof(unsigned), st);
-  if (e != cudaSuccess) return e;
-  if (pl.bt == 32) e = launch_solve<32>(a, pl.grid, st);
-  else if (pl.bt == 64) e = launch_solve<64>(a, pl.grid, st);
-  else e = launch_solve<128>(a, pl.grid, st);
+  const cudaError_t le = launch_cooperative(st, [&](int sms) {
+    const F64Plan pl = f64_plan(n, f64_edge(n, resp), resp, sms);
+    if (!work || f64_plan_doubles(pl) > cap) return cudaErrorInvalidValue;
+    a.ld = np;
+    a.kb = (n + 15) / 16;
+    a.ntiles = pl.tiles * (pl.tiles + 1) / 2;
+    a.snap = pl.snap;
+    a.ws = work;
+    a.partials = work + (size_t)pl.grid * pl.bt * pl.bt;
+    a.flags = reinterpret_cast<unsigned*>(a.partials + 2 * (size_t)pl.grid * kSums);
+    a.bar = a.flags + pl.grid;
+    cudaError_t e = cudaMemsetAsync(a.flags, 0, (pl.grid + 1) * sizeof(unsigned), st);
+    if (e != cudaSuccess) return e;
+    if (pl.bt == 32) return launch_solve<32>(a, pl.grid, st);
+    if (pl.bt == 64) return launch_solve<64>(a, pl.grid, st);
+    return launch_solve<128>(a, pl.grid, st);
+  });
   note_launch();
-  return e == cudaSuccess ? cudaGetLastError() : e;
+  return le == cudaSuccess ? cudaGetLastError() : le;
 }
 
 }  // namespace sp2b

@@ -87,6 +87,19 @@ std::string f64_tune_key(int np);
 int tune_f64_tile(int np, const double* x_in, double* x_out, double* partials, unsigned* counter,
                   double* sums_out, cudaStream_t st);
 int device_sms();       // SM count of the current device
+int stream_sms(cudaStream_t st);   // SMs that launches on st may use (fewer in a green context)
+
+// A cooperative launch whose grid run(sms) sizes for so many SMs: those of the stream, and
+// fewer while the driver refuses the grid as too large to be resident (a share of the SMs that
+// the stream does not show).
+template <typename F>
+inline cudaError_t launch_cooperative(cudaStream_t st, F&& run) {
+  for (int sms = stream_sms(st);; sms = (sms + 1) / 2) {
+    const cudaError_t e = run(sms);
+    if (e != cudaErrorCooperativeLaunchTooLarge || sms <= 1) return e;
+    (void)cudaGetLastError();
+  }
+}
 int f64_ntiles(int np);
 cudaError_t launch_gersh(const double* h, int n, int ld, double* rowsum, int nsplit,
                          double* bounds, double* partials, unsigned* counter, cudaStream_t st);

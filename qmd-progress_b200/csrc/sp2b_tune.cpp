@@ -1,6 +1,8 @@
 // Launch-configuration autotuner: the decision table, its file, and the timing loop.
 #include "sp2b_tune.h"
 
+#include <cudaTypedefs.h>
+
 #include <algorithm>
 #include <atomic>
 #include <cstdio>
@@ -10,6 +12,7 @@
 #include <mutex>
 #include <sstream>
 
+#include "kernels.cuh"
 #include "sp2b.h"
 
 namespace sp2b {
@@ -69,6 +72,32 @@ int device_sms() {
     return 148;
   if (dev >= 0 && dev < 64) sms[dev].store(v, std::memory_order_relaxed);
   return v;
+}
+
+int stream_sms(cudaStream_t st) {
+  typedef PFN_cuStreamGetGreenCtx_v12040 GreenOf;
+  typedef PFN_cuGreenCtxGetDevResource_v12040 ResourceOf;
+  static GreenOf green_of = nullptr;
+  static ResourceOf resource_of = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    cudaDriverEntryPointQueryResult q;
+    void *a = nullptr, *b = nullptr;
+    if (cudaGetDriverEntryPoint("cuStreamGetGreenCtx", &a, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess &&
+        cudaGetDriverEntryPoint("cuGreenCtxGetDevResource", &b, cudaEnableDefault, &q) ==
+            cudaSuccess &&
+        q == cudaDriverEntryPointSuccess) {
+      green_of = reinterpret_cast<GreenOf>(a);
+      resource_of = reinterpret_cast<ResourceOf>(b);
+    }
+  });
+  CUgreenCtx g = nullptr;
+  CUdevResource r;
+  if (green_of && resource_of && green_of(st, &g) == CUDA_SUCCESS && g &&
+      resource_of(g, &r, CU_DEV_RESOURCE_TYPE_SM) == CUDA_SUCCESS && r.sm.smCount > 0)
+    return std::min((int)r.sm.smCount, device_sms());
+  return device_sms();
 }
 
 bool tune_enabled() {

@@ -24,7 +24,7 @@ def lists(tmp_path_factory):
     return C.CDLL(out)
 
 
-@pytest.mark.parametrize("sms", [148, 132, 7])
+@pytest.mark.parametrize("sms", [148, 132, 7, 1])
 @pytest.mark.parametrize("resp", [0, 1])
 def test_fp64_shares(lists, sms, resp):
     # every size up to 1300 with the edge of its rule and the next one up, then a few large ones
