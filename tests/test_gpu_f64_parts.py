@@ -1,7 +1,7 @@
 """The persistent FP64 sub-graph solve (k_f64_parts) at the edges of its tiles: parts of one
-16-row k-block, one 32- and one 64-edge tile and either side of them, a part above 512 (the
-extraction path of large parts) and parts without core rows, against the oracle's
-prg_sp2_submatrix per part, with both tile edges giving the same rows.
+16-row k-block, one 32- and one 64-edge tile and either side of them, a part above 512 and
+parts without core rows, against the oracle's prg_sp2_submatrix per part, with both tile edges
+giving the same rows.  (Parts about the extraction's limit: tests/test_gpu_extraction.py.)
 
 Sums of n <= 600 terms over 12 steps: 12 * 600 * 1.1e-16 = 8e-13 between two orders."""
 import numpy as np

@@ -137,8 +137,8 @@ def test_int8_lattice_within_1e6_of_fp64_batch(cuda):
 
 
 def test_int8_subgraph_parts_above_512(cuda):
-    """Parts larger than 512 (core+halo ~610): the digit planes come from the FP64
-    extraction (k_norm_digits) instead of straight from CSR; within 1e-7 of the oracle."""
+    """Parts larger than 512 (core+halo ~610), straight from CSR as all up to 2048 (larger
+    ones: tests/test_gpu_extraction.py); within 1e-7 of the oracle."""
     n = 1400
     h, g, parts, emin, emax, pp, maxiter = _setup(n, 600)
     rho_ref, vv_ref, _ = O.subgraph_sp2_loop(h, g, parts, pp, maxiter, emin, emax)
