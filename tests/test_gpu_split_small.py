@@ -60,3 +60,54 @@ def test_split_step_and_reverse_step(cuda, n):
         got = full(o)
         assert float((got - ref).norm()) <= 2.0 * tol * float(ref.norm())
         assert torch.equal(got, got.T)
+
+
+@pytest.mark.parametrize("n", [2300, 2560, 3072, 3328, 3840, 4352])
+def test_dense_solve_where_the_last_wave_is_cut(cuda, n):
+    """The dense solve at the sizes whose last wave's tiles are cut in two: the sums that a step
+    leaves for the next one's branch (its record) against the iterate it wrote, and the
+    McWeeny combine product on the same tiles."""
+    import ctypes as C
+
+    torch = cuda
+    from sp2b import _lib
+    L = _lib.lib()
+    npad = int(L.sp2b_split_dim(n))
+    h = torch.from_numpy(M.two_band_1d(n, seed=n)).cuda()
+    rho = torch.empty_like(h)
+    st = torch.cuda.current_stream().cuda_stream
+    o = _lib.make_opts(precision=_lib.PREC_MIXED_FP16, mcweeny=0, device_ptrs=True, stream=st)
+    off = h.abs().sum(0) - h.diagonal().abs()
+    emin, emax = float((h.diagonal() - off).min()), float((h.diagonal() + off).max())
+    x0 = (emax * torch.eye(n, dtype=h.dtype, device="cuda") - h) / (emax - emin)
+    tol = 2.0 * (npad / 16 + 8) * 2.0 ** -23
+    for branch in (1, 0):
+        pp, vv = np.array([branch], dtype=np.int32), np.zeros(1)
+        _lib.check(L.sp2b_sp2_alg2_seq(h.data_ptr(), rho.data_ptr(), n, 0.0, pp.ctypes.data, 1,
+                                       vv.ctypes.data, 0, C.byref(o)), "seq")
+        recs = np.zeros((2, 9))
+        it = C.c_int(0)
+        _lib.check(L.sp2b_last_solve_info(C.byref(it), C.byref(it), C.byref(it), C.byref(it),
+                                          recs.ctypes.data, 2), "info")
+        x = 0.5 * rho
+        p = x0 @ x0
+        want = p if branch else 2.0 * x0 - p
+        assert float((x - want).norm()) <= tol * float(want.norm())
+        assert torch.equal(x, x.T)
+        # {trx, trx_data, fro2, ..., trp}: sums of what was stored, but for its rounding to hi + lo
+        _, trx, fro2, *_, trp = recs[1]
+        assert abs(trx - float(x.trace())) <= 2.0 ** -20 * float(x.diagonal().abs().sum())
+        assert abs(fro2 - float(x.norm()) ** 2) <= 2.0 ** -20 * float(x.norm()) ** 2
+        assert abs(trp - float(p.trace())) <= tol * float(p.trace())
+        res = float((x0 - p).norm())
+        assert abs(vv[0] - res) <= tol * float(p.norm()) + 2.0 ** -21 * float(x0.norm())
+    # a whole solve: the refined density of a gapped system, as tests/test_gpu_dense.py bounds it
+    o = _lib.make_opts(precision=_lib.PREC_MIXED_FP16, device_ptrs=True, stream=st)
+    o64 = _lib.make_opts(precision=_lib.PREC_FP64, device_ptrs=True, stream=st)
+    ref = torch.empty_like(h)
+    for out, opts in ((rho, o), (ref, o64)):
+        _lib.check(L.sp2b_sp2_alg2(h.data_ptr(), out.data_ptr(), n, 0.0, 0.5, 0, 100, b"Rel", 1e-10, 0,
+                                   C.byref(opts), None), "alg2")
+    assert float((rho - ref).norm()) / n <= 1e-6
+    assert float((rho - ref).abs().max()) <= 1e-6      # in no tile more than elsewhere
+    assert torch.equal(rho, rho.T)
