@@ -10,6 +10,7 @@ Hamiltonians: output produced by the reference itself on this machine.
 * The race (printed; not asserted): the reference's own loop time and whole call against
   this library's device-resident mixed solve, N = 8192 two-band.
 """
+import os
 import time
 
 import numpy as np
@@ -21,6 +22,12 @@ import sp2b
 from sp2b import modelham as M
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def reference_build():
+    if not os.path.exists(PA.LIB):
+        pytest.skip("oracle/_ref/libprg_sp2_tc.so is built where a PROGRESS tree is present")
 
 
 @pytest.mark.parametrize("n", [1024, 2048])
