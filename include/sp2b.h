@@ -247,9 +247,10 @@ int sp2b_sp2_entropy_function(double mu, double h1, double hN, int nsteps, const
                               double* gg, double* ee, int npoints);
 
 /* ---- Launch-configuration autotuner ---------------------------------------------------
- * The first solve of a new shape on a device times the equivalent launch configurations of
- * its step kernel with CUDA events and keeps the fastest:
- *   "f64-step/sm<S>/np<np>"          dense FP64 step tile edge, 128 or 64;
+ * The first solve of a new shape on a device times equivalent launch configurations with CUDA
+ * events and keeps the fastest:
+ *   "f64-step/sm<S>/np<np>"          tile edge of single FP64 products (FP64 McWeeny, idempotency,
+ *                                     SP2-Fermi's correction, allocation-free steps), 128 or 64;
  *   "subgraph/f64/sm<S>/<np>x<k>,..." batched FP64 sub-graph tile edge, 64 or 32;
  *   "subgraph/split/sm<S>/<np>x<k>,..." batched split tile order, 0 (largest parts first) or
  *                                     1 (every other wave reversed: balanced over the CTAs).

@@ -21,7 +21,7 @@ namespace sp2b {
 // fragment are taken in pairs, 0 1, 8 9, 2 3, 10 11 of a group of sixteen (the odd fragment
 // 4 5, 12 13, 6 7, 14 15): under that swizzle the sixteen 8-byte words that a half-warp
 // loads (four k rows, four columns) then lie in distinct banks, and k stays ascending.
-// Full / empty mbarriers instead of a block barrier per k-block let the eight warps drift:
+// Full / empty mbarriers instead of a block barrier per k-block let the warps drift:
 // with __syncthreads they waited there a fifth of the time.
 template <int BT>
 struct F64Tile {

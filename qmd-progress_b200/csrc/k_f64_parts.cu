@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(F64Tile<BT>::NT + 32, BT == 32 ? 2 : 1)
   }
 }
 
-// vv[k] += the residual sums of step k, one block per step, in a fixed order.
+// vv[k] = the residual sums of step k, one block per step, in a fixed order.
 __global__ void __launch_bounds__(256)
     k_f64_parts_sums(const double* __restrict__ partials, int per_step, double* __restrict__ vv) {
   __shared__ double red[32];

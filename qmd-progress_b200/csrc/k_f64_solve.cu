@@ -43,14 +43,13 @@ struct F64SolveMaps {
 
 }  // namespace
 
-// Bound by the DMMA pipe (37 TFLOP/s measured with registers only).  The per-step launches
-// this replaces spent ~10 us of each step on launch, record reads, mirrored stores and the
-// last CTA's sums, computed whole padded 128-blocks, left SMs idle in the last wave of
-// tiles and, for the response, formed {X, Delta} as two products with a stored middle.  Here
-// a step costs its k-blocks (92 % of the DMMA rate at n = 3500), ~4 us per tile epilogue and
-// ~3 us of barrier and decision.  Per solve on B200, before -> now: n = 100 365 -> 169 us,
-// n = 1000 985 -> 640 us, n = 2000 (14 steps) 4.0 ms, n = 3500 23.0 -> 19.3 ms, response
-// n = 777 2.40 -> 0.91 ms.
+// Bound by the DMMA pipe (37 TFLOP/s measured with registers only) and for small orders by the
+// chain of one step: its k-blocks, ~4 us per tile epilogue, ~3 us of barrier and decision.  One
+// launch per step would add ~10 us of launch, record reads and a last CTA's sums to each,
+// padded 128-blocks, idle SMs in the last wave of tiles and, for the response, {X, Delta} as
+// two products with a stored middle.  Whole calls on B200, that form -> this one: n = 100 365
+// -> 112 us, n = 1000 985 -> 604 us, n = 3500 22.0 -> 18.3 ms (0.88 of the DMMA rate over the
+// call), response n = 777 2.40 -> 0.85 ms.
 //
 // One CTA walks its share of each step's units (F64Split), then all CTAs meet at a grid
 // barrier (a counter, bounded wait) and every CTA sums the partials in CTA order and takes

@@ -633,9 +633,9 @@ __global__ void __launch_bounds__(256)
 //    k_oz_residues_f64 form them again (planes by a pass over X cost 27 us a step at
 //    n = 2744).  The row norms that the scale needs are integer sums on the way; the last
 //    CTA takes their maximum (stored per block and summed by a launch of its own: 6 us a step
-//    more).  50 us at n = 2744, where the bytes take 30 at the measured copy rate.  One resident wave of CTAs walks the upper 32 x 32 block pairs (diagonal blocks
-//    hold both triangles, whose squares are equal bit for bit: the integer products are
-//    symmetric).
+//    more).  50 us at n = 2744, where the bytes take 30 at the measured copy rate.  One
+//    resident wave of CTAs walks the upper 32 x 32 block pairs (diagonal blocks hold both
+//    triangles, whose squares are equal bit for bit: the integer products are symmetric).
 // ---------------------------------------------------------------------------------
 // ||row||^2 shares in units of 2^-44, rounded up: integer sums do not depend on their order,
 // and the scale's bound only needs the norm from above (at most np/32 units too much, 1e-10).
